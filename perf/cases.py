@@ -8,7 +8,8 @@ verified or a few sequences decode together, some tens in a busy server, and hun
 while prompts are read.
 
 `listed()` holds the cases, `draw()` makes more of the same ranges, `prepare()` builds what a program
-has in hand before the call, `run()` is one pass through the public entry points.
+has in hand before the call, `run()` is one pass through the public entry points, `exact()` what that
+pass returns, in 64 bits.
 """
 from __future__ import annotations
 
@@ -126,12 +127,17 @@ def _backend():
     return _BACKEND
 
 
-def _weight(be, rng, t, n, k):
+def _rows(rng, t, n, k):
     """N(0, 0.02) rows through the library's reference quantizer.  A few hundred distinct rows are drawn and every
     row of the matrix is one of them, so that a large matrix is made quickly; the library treats all rows alike."""
     base = rng.standard_normal((min(n, 307), k), dtype=np.float32) * np.float32(0.02)
     packed = mb.quantize(_TYPES[t], base)
-    return be.upload(_TYPES[t], packed[rng.integers(0, len(base), n)], n, k)
+    return packed, rng.integers(0, len(base), n)
+
+
+def _weight(be, rng, t, n, k):
+    packed, index = _rows(rng, t, n, k)
+    return be.upload(_TYPES[t], packed[index], n, k)
 
 
 def _acts(gen, m, k, dtype):
@@ -142,11 +148,14 @@ def _acts(gen, m, k, dtype):
     return x.to(_DTYPES[dtype])
 
 
-def _layer_weights(be, rng, c):
+def _layer_shapes(c):
     h, i, t, td = c["hidden"], c["inter"], c["type"], c["type_down"]
-    shapes = {"q": (t, c["q_rows"], h), "k": (t, c["kv_rows"], h), "v": (td, c["kv_rows"], h), "o": (t, h, c["q_rows"]),
-              "gate": (t, i, h), "up": (t, i, h), "down": (td, h, i)}
-    first = {name: _weight(be, rng, *s) for name, s in shapes.items()}
+    return {"q": (t, c["q_rows"], h), "k": (t, c["kv_rows"], h), "v": (td, c["kv_rows"], h), "o": (t, h, c["q_rows"]),
+            "gate": (t, i, h), "up": (t, i, h), "down": (td, h, i)}
+
+
+def _layer_weights(be, rng, c):
+    first = {name: _weight(be, rng, *s) for name, s in _layer_shapes(c).items()}
     # further layers hold the same values in memory of their own: every layer is read from HBM
     return [first] + [{name: w.clone() for name, w in first.items()} for _ in range(c["layers"] - 1)]
 
@@ -241,6 +250,94 @@ def run(s):
         be.project_multi([w["gate"], w["up"]], x["hidden"], [y["gate"], y["up"]])
         be.project(w["down"], x["act"], out=y["down"])
     return s["y"]
+
+
+# ---- the same results in 64 bits ---------------------------------------------------------------------
+
+_E2M1 = [0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0]
+
+
+def _values(t, packed, k):
+    """The weights that rows of GGUF blocks stand for, [rows][k] in 64 bits."""
+    elems, size = _BLOCK[t]
+    b = torch.from_numpy(np.ascontiguousarray(packed).view(np.uint8).reshape(-1, size)).cuda()
+    half = lambda at: b[:, at:at + 2].contiguous().view(torch.float16).double()  # noqa: E731
+    nibbles = lambda q: torch.cat([q & 15, q >> 4], dim=-1)                       # noqa: E731
+    if t == "Q8_0":
+        v = half(0) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif t == "Q4_0":
+        v = half(0) * (nibbles(b[:, 2:]).double() - 8)
+    elif t == "MXFP4":
+        v = torch.exp2(b[:, :1].double() - 127) * torch.tensor(_E2M1, device="cuda", dtype=torch.float64)[nibbles(b[:, 1:]).long()]
+    elif t in ("Q4_K", "Q5_K"):
+        s = b[:, 4:16]
+        scale = torch.cat([s[:, :4] & 63, (s[:, 8:] & 15) | (s[:, :4] >> 6 << 4)], dim=1).double()
+        least = torch.cat([s[:, 4:8] & 63, (s[:, 8:] >> 4) | (s[:, 4:8] >> 6 << 4)], dim=1).double()
+        q = nibbles(b[:, size - 128:].reshape(-1, 4, 32)).reshape(-1, 8, 32)
+        if t == "Q5_K":
+            q = q | ((b[:, None, 16:48] >> torch.arange(8, device="cuda", dtype=torch.uint8)[None, :, None]) & 1) << 4
+        v = (half(0) * scale)[:, :, None] * q.double() - (half(2) * least)[:, :, None]
+    else:  # Q6_K: two halves of 128 weights, each four runs of 32
+        low = nibbles(b[:, :128].reshape(-1, 2, 64)).reshape(-1, 2, 4, 32)
+        high = (b[:, 128:192].reshape(-1, 2, 1, 32) >> torch.tensor([0, 2, 4, 6], device="cuda", dtype=torch.uint8)[None, None, :, None]) & 3
+        scale = half(208) * b[:, 192:208].contiguous().view(torch.int8).double()
+        v = scale[:, :, None] * ((low | high << 4).reshape(-1, 16, 16).double() - 32)
+    return v.reshape(-1, k)
+
+
+class _Weight64:
+    def __init__(self, rng, t, n, k):
+        packed, index = _rows(rng, t, n, k)
+        self.v, self.index, self.n = _values(t, packed, k), torch.from_numpy(index).cuda(), n
+
+    def __call__(self, x):
+        return (x.double() @ self.v.T)[:, self.index]
+
+
+def exact(case, seed):
+    """What `run` returns on the state of `prepare(case, seed)`, from the same draws, in 64 bits."""
+    rng = np.random.default_rng(seed)
+    gen = torch.Generator(device="cuda").manual_seed(int(seed))
+    c = dict(case)
+    kind, m = c["kind"], c["m"]
+    if kind in ("call", "plan"):
+        w = _Weight64(rng, c["type"], c["n"], c["k"])
+        return [w(_acts(gen, m, c["k"], c["x"])) for _ in range(c["copies"])]
+    if kind == "host":
+        w = _Weight64(rng, c["type"], c["n"], c["k"])
+        return w(_acts(gen, m, c["k"], c["x"])).cpu().numpy()
+    if kind == "mlp_plan":
+        h, i = c["hidden"], c["inter"]
+        gate, up, down = _Weight64(rng, c["type"], i, h), _Weight64(rng, c["type"], i, h), _Weight64(rng, c["type"], h, i)
+        y = ([], [], [])
+        for _ in range(c["layers"]):
+            x = _acts(gen, m, h, c["x"])
+            y[0].append(gate(x))
+            y[1].append(up(x))
+            y[2].append(down(_acts(gen, m, i, c["x"])))
+        return [torch.stack(v) for v in y]
+    if kind == "chain":
+        h = c["hidden"]
+        stream = torch.randn((m, h), generator=gen, device="cuda").double()
+        w = {name: _Weight64(rng, *s) for name, s in _layer_shapes(c).items()}
+        normed = lambda x, g: x * torch.rsqrt((x * x).mean(dim=1, keepdim=True) + 1e-5) * g.double()  # noqa: E731
+        parts = []
+        for _ in range(c["layers"]):
+            norm1, norm2 = (1.0 + 0.1 * torch.randn(h, generator=gen, device="cuda") for _ in range(2))
+            attn = _acts(gen, m, c["q_rows"], "f32") * 0.1
+            x = normed(stream, norm1)
+            parts += [w["q"](x), w["k"](x), w["v"](x)]
+            stream = stream + w["o"](attn)
+            x = normed(stream, norm2)
+            act = torch.nn.functional.silu(w["gate"](x)) * w["up"](x)
+            parts.append(act)
+            stream = stream + w["down"](act)
+        return {"stream": stream, "parts": parts}
+    w = {name: _Weight64(rng, *s) for name, s in _layer_shapes(c).items()}
+    x = {"hidden": _acts(gen, m, c["hidden"], c["x"]), "attn": _acts(gen, m, c["q_rows"], c["x"]), "act": _acts(gen, m, c["inter"], c["x"])}
+    source = {"o": "attn", "down": "act"}
+    y = {name: p(x[source.get(name, "hidden")]) for name, p in w.items()}
+    return [y] * c["layers"]
 
 
 # ---- what a pass cannot do without ------------------------------------------------------------------
