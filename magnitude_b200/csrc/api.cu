@@ -92,6 +92,8 @@ struct b200q_ctx {
     // prefill path: bf16 copy of fp32 activations
     void *gemm_scratch = nullptr;
     size_t gemm_scratch_bytes = 0;
+    void *dense_w = nullptr;          // fp16 weights of the two-launch GEMM, one panel at a time
+    size_t dense_w_bytes = 0;
     float *gemm_part = nullptr;       // K-split partial products of skinny batches (allocated on first use)
     // skinny route (2..16 rows): chunk sums, row-block counters, job table
     uint8_t *sk_ws = nullptr;
@@ -100,7 +102,7 @@ struct b200q_ctx {
     bool peer_stale = false;          // a peer exchange timed out: the ranks' call counters no longer agree
     bool peer_ipc = true;             // peer buffers were mapped through CUDA IPC (else given as pointers)
     int skinny_min_m = 3;             // smallest M that takes the skinny route (smaller batches: the dp4a kernel)
-    int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1;
+    int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1, gemm_dense = -1;
     // tunables (environment overrides for experiments)
     int gemv_warps = 0, gemv_depth = 0, gemv_grid = 0, gemv_smem = 0, gemv_rows = 0, gemv_debug = 0, gemv_pdl = 1, gemv_teams = 2, gemv_xprep = 1, gemv_nap = 0;
     // tensor parallel
@@ -286,23 +288,87 @@ b200q_status run_gemv(b200q_ctx *ctx, const b200q_weight *const *w, int nw, cons
     return run_stream(ctx, &J, nullptr, 1, M, st);
 }
 
+// scratch for the fp16 copy of M activation rows
+b200q_status ensure_gemm_scratch(b200q_ctx *ctx, int64_t M, int64_t K, cudaStream_t st) {
+    const size_t need = gemm_x_scratch_bytes((int)M, (int)K);
+    if (need <= ctx->gemm_scratch_bytes) return B200Q_OK;
+    if (ctx->gemm_scratch) {
+        CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still read the old buffer
+        cudaFree(ctx->gemm_scratch);
+        ctx->gemm_scratch = nullptr;
+        ctx->gemm_scratch_bytes = 0;
+    }
+    CU_TRY(ctx, cudaMalloc(&ctx->gemm_scratch, need));
+    ctx->gemm_scratch_bytes = need;
+    return B200Q_OK;
+}
+
+// Workspace for the fp16 weights of the two-launch GEMM: a fixed size from the first use on (only a K above
+// 262144 asks for more), so that a later call with larger weights allocates nothing.  False where it
+// cannot be had (no memory, or the stream is being captured): the one-launch kernels take the call.
+bool ensure_dense_scratch(b200q_ctx *ctx, int64_t Kpad, cudaStream_t st) {
+    const size_t need = std::max(kDenseScratchBytes, (size_t)Kpad * 2 * 256);
+    if (need <= ctx->dense_w_bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    void *ptr = nullptr;
+    if (cudaMalloc(&ptr, need) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (ctx->dense_w) cudaFree(ctx->dense_w);      // waits for the device: earlier launches may still read it
+    ctx->dense_w = ptr;
+    ctx->dense_w_bytes = need;
+    return true;
+}
+
+// Larger batches: fp16 copies of the activations and of all the call's weights, then one dense GEMM over them.
+// False: the one-launch kernels are the faster ones here, or there is no workspace.
+bool run_dense(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int64_t M, int64_t ldx,
+               void *const *y, int y_dtype, const int64_t *ldy, cudaStream_t st, b200q_status *status) {
+    if (ctx->gemm_pair != 1 || ctx->gemm_dense == 0 || M < (ctx->gemm_dense > 0 ? ctx->gemm_dense : 128)) return false;
+    DenseLaunch a{};
+    a.qt = w[0]->type;
+    a.K = (int)w[0]->K;
+    a.Kpad = (int)w[0]->Kpad;
+    for (int i = 0; i < nw; ++i) {
+        if (w[i]->N == 0) continue;
+        a.w[a.nw] = w[i]->dev;
+        a.n[a.nw] = (int)w[i]->N;
+        a.y[a.nw] = y[i];
+        a.ldy[a.nw] = ldy[i];
+        ++a.nw;
+    }
+    a.y_is_bf16 = y_dtype == B200Q_TYPE_BF16;
+    a.x = x;
+    a.ldx = ldx;
+    a.x_is_bf16 = x_dtype == B200Q_TYPE_BF16;
+    a.M = (int)M;
+    a.status = ctx->status_dev;
+    a.sm_count = ctx->sm_count;
+    a.bn_override = ctx->gemm_bn;
+    if (ctx->gemm_dense < 0 && !dense_pays(a)) return false;
+    if (!ensure_dense_scratch(ctx, a.Kpad, st)) return false;
+    a.scratch = ctx->dense_w;
+    a.scratch_bytes = ctx->dense_w_bytes;
+    if ((*status = ensure_gemm_scratch(ctx, M, a.K, st)) != B200Q_OK) return true;
+    a.x16 = ctx->gemm_scratch;
+    cudaError_t e = dense_gemm_run(a, st, &ctx->last_launches);
+    if (e != cudaSuccess) *status = cuda_fail(ctx, e, "dense GEMM launch");
+    return true;
+}
+
 // prefill route: one activation conversion per weight set and one tensor-core launch per weight
 b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int x_dtype, int64_t M, int64_t ldx,
                       void *y, int y_dtype, int64_t ldy, cudaStream_t st, int *launches, bool x_already_converted) {
     // Both tensor-core operands are fp16: the activations are converted into context-owned scratch
     // memory first (once for all the weights of a set, which share them).
     if (!x_already_converted) {
-        const size_t need = gemm_x_scratch_bytes((int)M, (int)w->K);
-        if (need > ctx->gemm_scratch_bytes) {
-            if (ctx->gemm_scratch) {
-                CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still read the old buffer
-                cudaFree(ctx->gemm_scratch);
-                ctx->gemm_scratch = nullptr;
-                ctx->gemm_scratch_bytes = 0;
-            }
-            CU_TRY(ctx, cudaMalloc(&ctx->gemm_scratch, need));
-            ctx->gemm_scratch_bytes = need;
-        }
+        b200q_status s = ensure_gemm_scratch(ctx, M, w->K, st);
+        if (s != B200Q_OK) return s;
         cudaError_t e = gemm_convert_x(x, x_dtype == B200Q_TYPE_BF16, ldx, ctx->gemm_scratch, (int)M, (int)w->K, st);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "activation conversion launch");
         ++*launches;
@@ -435,6 +501,8 @@ b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
     }
     if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
         ctx->last_route = B200Q_ROUTE_GEMM;
+        b200q_status ds = B200Q_OK;
+        if (run_dense(ctx, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;
         bool converted = false;
         for (int i = 0; i < nw; ++i) {
             if (w[i]->N == 0) continue;
@@ -608,6 +676,7 @@ b200q_status b200q_ctx_create(int32_t device, b200q_ctx **out) {
     ctx->gemv_nap = env_int("B200Q_GEMV_NAP", 0);
     ctx->gemm_bn = env_int("B200Q_GEMM_BN", 0);
     ctx->gemm_pair = env_int("B200Q_GEMM_PAIR", 1);
+    ctx->gemm_dense = env_int("B200Q_GEMM_DENSE", -1);
     ctx->gemm_ksplit = env_int("B200Q_GEMM_KSPLIT", 1);
     *out = ctx;
     return B200Q_OK;
@@ -626,6 +695,7 @@ void b200q_ctx_destroy(b200q_ctx *ctx) {
     if (ctx->hx_dev) cudaFree(ctx->hx_dev);
     if (ctx->hy_dev) cudaFree(ctx->hy_dev);
     if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
+    if (ctx->dense_w) cudaFree(ctx->dense_w);
     if (ctx->gemm_part) cudaFree(ctx->gemm_part);
     if (ctx->sk_ws) cudaFree(ctx->sk_ws);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
@@ -647,6 +717,7 @@ b200q_status b200q_ctx_set_option(b200q_ctx *ctx, int32_t option, int64_t value)
         CU_TRY(ctx, gemv_set_wait_limit_ns(ns));
         CU_TRY(ctx, skinny_set_wait_limit_ns(ns));
         CU_TRY(ctx, gemm_set_wait_limit_ns(ns));
+        CU_TRY(ctx, dense_set_wait_limit_ns(ns));
         CU_TRY(ctx, peer_set_wait_limit_ns(ns));
         return B200Q_OK;
     }

@@ -11,6 +11,7 @@ namespace b200q {
 cudaError_t gemv_set_wait_limit_ns(unsigned long long ns);
 cudaError_t skinny_set_wait_limit_ns(unsigned long long ns);
 cudaError_t gemm_set_wait_limit_ns(unsigned long long ns);
+cudaError_t dense_set_wait_limit_ns(unsigned long long ns);
 cudaError_t peer_set_wait_limit_ns(unsigned long long ns);
 
 // ---- layout.cu ------------------------------------------------------------------------------
@@ -156,6 +157,32 @@ cudaError_t gemm_launch(const GemmLaunch &a, cudaStream_t st);
 // describe the caller's activations (bf16 or fp32), nothing is allocated
 size_t gemm_static_scratch_elems();
 cudaError_t gemm_launch_static(GemmLaunch a, int x_is_bf16, cudaStream_t st);
+
+// ---- gemm_dense.cu --------------------------------------------------------------------------
+// One activation, up to four weights of one type and K: fp16 copies of both in workspaces, then a dense GEMM.
+constexpr int kDenseMaxWeights = 4;
+struct DenseLaunch {
+    int qt, nw, K, Kpad;
+    const uint8_t *w[kDenseMaxWeights];   // streaming-layout weights
+    int n[kDenseMaxWeights];              // their rows (> 0)
+    void *y[kDenseMaxWeights];
+    long long ldy[kDenseMaxWeights];
+    int y_is_bf16;
+    const void *x;                        // activations [M][K], bf16 or fp32
+    long long ldx;
+    int x_is_bf16, M;
+    void *x16;                            // workspace of gemm_x_scratch_bytes(M, K)
+    void *scratch;                        // workspace for the fp16 weights; at least 256 rows of Kpad elements
+    size_t scratch_bytes;
+    int *status;
+    int sm_count;
+    int bn_override;                      // 0 = choose the token tile
+};
+// 256 MB: all projections of an 8B-class model in one panel; with 128 MB the gate and up matrices of such a
+// layer took two, each with a partial last round (28672 x 4096, 512 rows: 165 us against 143)
+constexpr size_t kDenseScratchBytes = size_t(256) << 20;
+bool dense_pays(const DenseLaunch &a);    // worth two launches? (sizes only; scratch and pointers not needed)
+cudaError_t dense_gemm_run(const DenseLaunch &a, cudaStream_t st, int *launches);
 
 // ---- peer.cu --------------------------------------------------------------------------------
 // Exchange buffer of one GPU.  Every element travels as an 8-byte (value, call number) pair written
