@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(kPrepThreads) dense_prep_kernel(const PrepPara
     __shared__ __align__(16) uint8_t out[kRowGroup * 4096];
     pdl_launch_dependents();
     if ((int)blockIdx.x < p.x_blocks) {
+        pdl_wait();              // X may come from the launch before, which may also still read the copies
         const unsigned total = (unsigned)p.M * (unsigned)p.K8;
         for (unsigned i = blockIdx.x * kPrepThreads + threadIdx.x; i < total; i += (unsigned)p.x_blocks * kPrepThreads) {
             const unsigned m = i / (unsigned)p.K8, c = i - m * (unsigned)p.K8;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kPrepThreads) dense_prep_kernel(const PrepPara
     for (int i = threadIdx.x; i < kRowGroup * row_b / 16; i += kPrepThreads)
         reinterpret_cast<uint4 *>(in)[i] = __ldg(reinterpret_cast<const uint4 *>(src) + i);
     __syncthreads();
+    pdl_wait();                  // the weights depend on no launch, the workspace on the GEMM that last read it
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rec = lane >> 2;
     const int nrec = min(kChunkRecs, p.nsb - c * kChunkRecs);
     const uint32_t row_s = smem_u32(in) + warp * row_b, out_s = smem_u32(out) + warp * 4096;
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const DensePara
     cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&sm->tmem_base);
+    pdl_launch_dependents();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -370,10 +373,17 @@ bool encode_2d(CUtensorMap *map, const void *base, long long cols, long long row
 }
 
 template <int QT>
-void launch_prep(const PrepParams &p, bool bf16, cudaStream_t st) {
-    if (p.x_blocks + p.tiles == 0) return;
-    if (bf16) dense_prep_kernel<QT, true><<<p.x_blocks + p.tiles, kPrepThreads, 0, st>>>(p);
-    else dense_prep_kernel<QT, false><<<p.x_blocks + p.tiles, kPrepThreads, 0, st>>>(p);
+cudaError_t launch_prep(const PrepParams &p, bool bf16, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(p.x_blocks + p.tiles));
+    cfg.blockDim = dim3(kPrepThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return bf16 ? cudaLaunchKernelEx(&cfg, dense_prep_kernel<QT, true>, p) : cudaLaunchKernelEx(&cfg, dense_prep_kernel<QT, false>, p);
 }
 
 }  // namespace
@@ -477,16 +487,16 @@ cudaError_t dense_gemm_run(const DenseLaunch &a, cudaStream_t st, int *launches)
                 ++*launches;
             }
         }
+        cudaError_t e;
         switch (a.qt) {
-        case QT_Q4_K: launch_prep<QT_Q4_K>(pp, a.x_is_bf16, st); break;
-        case QT_Q5_K: launch_prep<QT_Q5_K>(pp, a.x_is_bf16, st); break;
-        case QT_Q4_0: launch_prep<QT_Q4_0>(pp, a.x_is_bf16, st); break;
-        case QT_MXFP4: launch_prep<QT_MXFP4>(pp, a.x_is_bf16, st); break;
-        case QT_Q6_K: launch_prep<QT_Q6_K>(pp, a.x_is_bf16, st); break;
-        case QT_Q8_0: launch_prep<QT_Q8_0>(pp, a.x_is_bf16, st); break;
+        case QT_Q4_K: e = launch_prep<QT_Q4_K>(pp, a.x_is_bf16, st); break;
+        case QT_Q5_K: e = launch_prep<QT_Q5_K>(pp, a.x_is_bf16, st); break;
+        case QT_Q4_0: e = launch_prep<QT_Q4_0>(pp, a.x_is_bf16, st); break;
+        case QT_MXFP4: e = launch_prep<QT_MXFP4>(pp, a.x_is_bf16, st); break;
+        case QT_Q6_K: e = launch_prep<QT_Q6_K>(pp, a.x_is_bf16, st); break;
+        case QT_Q8_0: e = launch_prep<QT_Q8_0>(pp, a.x_is_bf16, st); break;
         default: return cudaErrorInvalidValue;
         }
-        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ++*launches;
 
