@@ -95,13 +95,15 @@ struct b200q_ctx {
     void *dense_w = nullptr;          // fp16 weights of the two-launch GEMM, one panel at a time
     size_t dense_w_bytes = 0;
     float *gemm_part = nullptr;       // K-split partial products of skinny batches (allocated on first use)
-    // skinny route (2..16 rows): chunk sums, row-block counters, job table
+    // small batches (2..32 rows): sums of tiles shared by several blocks
     uint8_t *sk_ws = nullptr;
-    size_t sk_ws_bytes = 0;
+    uint8_t *sk_img = nullptr;        // activation images
+    size_t sk_img_bytes = 0;
     uint64_t tp_timeout_ms = 60000;   // host deadline of b200q_tp_init
     bool peer_stale = false;          // a peer exchange timed out: the ranks' call counters no longer agree
     bool peer_ipc = true;             // peer buffers were mapped through CUDA IPC (else given as pointers)
     int skinny_min_m = 3;             // smallest M that takes the skinny route (smaller batches: the dp4a kernel)
+    int mid_max_m = 32;               // largest M that runs on the small-batch kernels (17 and more rows)
     int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1, gemm_dense = -1;
     // tunables (environment overrides for experiments)
     int gemv_warps = 0, gemv_depth = 0, gemv_grid = 0, gemv_smem = 0, gemv_rows = 0, gemv_debug = 0, gemv_pdl = 1, gemv_teams = 2, gemv_xprep = 1, gemv_nap = 0;
@@ -125,6 +127,7 @@ struct b200q_plan {
     // plans on the skinny route (3..16 rows by default): groups of products run by the skinny kernel, one launch pair per group
     std::vector<SkinnySet *> sets;
     uint8_t *sk_ws = nullptr;
+    uint8_t *sk_img = nullptr;
     uint8_t *sk_jobs = nullptr;
 };
 
@@ -405,13 +408,12 @@ b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int 
     return B200Q_OK;
 }
 
-// skinny route: 2..16 activation rows, mma.sync on exact integer weights (skinny.cu); all weights of
+// small batches: 2..32 activation rows, mma.sync on weights unpacked in registers (skinny.cu); all weights of
 // the call share x, type and K
 b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int M,
                         int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy, cudaStream_t st) {
     SkinnyProduct prods[4];
     int n = 0;
-    size_t need = 0;
     for (int i = 0; i < nw; ++i) {
         if (w[i]->N == 0) continue;
         SkinnyProduct &a = prods[n++];
@@ -427,27 +429,38 @@ b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
         a.ldy = ldy[i];
         a.y_is_bf16 = y_dtype == B200Q_TYPE_BF16;
         a.M = M;
-        need += skinny_part_bytes(a);
     }
     if (n == 0) return B200Q_OK;
-    if (need > ctx->sk_ws_bytes) {
-        if (ctx->sk_ws) {
-            CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still use the old buffer
-            cudaFree(ctx->sk_ws);
-            ctx->sk_ws = nullptr;
-            ctx->sk_ws_bytes = 0;
+    if (!ctx->sk_ws) {           // one size serves every call
+        uint8_t *ws = nullptr;
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), skinny_ws_bytes()));
+        cudaError_t e = skinny_ws_init(ws, true);
+        if (e != cudaSuccess) {
+            cudaFree(ws);
+            return cuda_fail(ctx, e, "small-batch workspace");
         }
-        const size_t grow = std::max(need, size_t(4) << 20);
-        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ctx->sk_ws), grow));
-        ctx->sk_ws_bytes = grow;
+        ctx->sk_ws = ws;
+    }
+    const size_t need = skinny_image_bytes(prods[0]);      // the call's weights share x
+    if (need > ctx->sk_img_bytes) {
+        if (ctx->sk_img) {
+            CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still use the old buffer
+            cudaFree(ctx->sk_img);
+            ctx->sk_img = nullptr;
+            ctx->sk_img_bytes = 0;
+        }
+        const size_t grow = std::max(need, size_t(8) << 20);
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ctx->sk_img), grow));
+        ctx->sk_img_bytes = grow;
     }
     SkinnyBuffers buf{};
     buf.ws = ctx->sk_ws;
-    buf.ws_bytes = ctx->sk_ws_bytes;
+    buf.ws_bytes = skinny_ws_bytes();
+    buf.img = ctx->sk_img;
+    buf.img_bytes = ctx->sk_img_bytes;
     buf.jobs_dev = nullptr;      // at most four products: their descriptions travel in the kernel parameters
     buf.status = ctx->status_dev;
     buf.sm_count = ctx->sm_count;
-    buf.smem_limit = ctx->smem_optin;
     cudaError_t e = skinny_run(prods, n, buf, st, &ctx->last_launches);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "skinny kernel launch");
     return B200Q_OK;
@@ -487,20 +500,12 @@ b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
     if (M >= ctx->skinny_min_m && M <= skinny_max_m()) {
         // verify / small continuous batches: one pass over the packed weights, exact bf16 activations
         ctx->last_route = B200Q_ROUTE_SKINNY;
-        const bool f32 = x_dtype != B200Q_TYPE_BF16;
-        const int step = f32 ? 8 : 16;     // fp32 rows take two token slots each (high and low halves)
-        for (int64_t m0 = 0; m0 < M; m0 += step) {
-            const int mc = (int)std::min<int64_t>(step, M - m0);
-            void *yy[4];
-            for (int i = 0; i < nw; ++i) yy[i] = (char *)y[i] + m0 * ldy[i] * act_size(y_dtype);
-            const void *xx = (const char *)x + m0 * ldx * act_size(x_dtype);
-            b200q_status s = run_skinny(ctx, w, nw, xx, x_dtype, mc, ldx, yy, y_dtype, ldy, st);
-            if (s != B200Q_OK) return s;
-        }
-        return B200Q_OK;
+        return run_skinny(ctx, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
     }
     if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
         ctx->last_route = B200Q_ROUTE_GEMM;
+        if (M > skinny_max_m() && M <= ctx->mid_max_m)
+            return run_skinny(ctx, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
         b200q_status ds = B200Q_OK;
         if (run_dense(ctx, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;
         bool converted = false;
@@ -588,29 +593,32 @@ b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job 
             groups.back().prods.push_back(a);
         }
     }
-    size_t ws = 0;
-    for (const Group &g : groups)
-        for (const SkinnyProduct &a : g.prods) ws += skinny_part_bytes(a);
     if (groups.empty()) return B200Q_OK;
-    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_ws), std::max<size_t>(ws, 256)));
+    // the groups run one after another and share the workspaces
+    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_ws), skinny_ws_bytes()));
+    CU_TRY(ctx, skinny_ws_init(pl->sk_ws, false));
+    size_t img = 0;
+    for (const Group &g : groups) {
+        size_t sum = 0;
+        for (const SkinnyProduct &a : g.prods) sum += skinny_image_bytes(a);
+        img = std::max(img, sum);
+    }
+    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_img), img));
     CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_jobs), groups.size() * skinny_job_table_bytes()));
-    size_t ws_off = 0;
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group &g = groups[gi];
-        size_t gws = 0;
-        for (const SkinnyProduct &a : g.prods) gws += skinny_part_bytes(a);
         SkinnyBuffers buf{};
-        buf.ws = pl->sk_ws + ws_off;
-        buf.ws_bytes = gws;
+        buf.ws = pl->sk_ws;
+        buf.ws_bytes = skinny_ws_bytes();
+        buf.img = pl->sk_img;
+        buf.img_bytes = img;
         buf.jobs_dev = pl->sk_jobs + gi * skinny_job_table_bytes();
         buf.status = ctx->status_dev;
         buf.sm_count = ctx->sm_count;
-        buf.smem_limit = ctx->smem_optin;
         SkinnySet *set = nullptr;
         cudaError_t e = skinny_set_create(g.prods.data(), (int)g.prods.size(), buf, &set);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "skinny plan group");
         pl->sets.push_back(set);
-        ws_off += gws;
     }
     return B200Q_OK;
 }
@@ -676,6 +684,7 @@ b200q_status b200q_ctx_create(int32_t device, b200q_ctx **out) {
     ctx->gemv_nap = env_int("B200Q_GEMV_NAP", 0);
     ctx->gemm_bn = env_int("B200Q_GEMM_BN", 0);
     ctx->gemm_pair = env_int("B200Q_GEMM_PAIR", 1);
+    ctx->mid_max_m = std::min(env_int("B200Q_MID_MAX", skinny_max_mid_m()), skinny_max_mid_m());
     ctx->gemm_dense = env_int("B200Q_GEMM_DENSE", -1);
     ctx->gemm_ksplit = env_int("B200Q_GEMM_KSPLIT", 1);
     *out = ctx;
@@ -698,6 +707,7 @@ void b200q_ctx_destroy(b200q_ctx *ctx) {
     if (ctx->dense_w) cudaFree(ctx->dense_w);
     if (ctx->gemm_part) cudaFree(ctx->gemm_part);
     if (ctx->sk_ws) cudaFree(ctx->sk_ws);
+    if (ctx->sk_img) cudaFree(ctx->sk_img);
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     delete ctx;
 }
@@ -1176,6 +1186,7 @@ void b200q_plan_destroy(b200q_plan *plan) {
     if (plan->xq_dev) cudaFree(plan->xq_dev);
     for (SkinnySet *set : plan->sets) skinny_set_destroy(set);
     if (plan->sk_ws) cudaFree(plan->sk_ws);
+    if (plan->sk_img) cudaFree(plan->sk_img);
     if (plan->sk_jobs) cudaFree(plan->sk_jobs);
     delete plan;
 }

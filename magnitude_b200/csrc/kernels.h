@@ -91,14 +91,13 @@ cudaError_t stream_xprep_launch(const StreamJob *jobs_dev, int njobs, int M, cud
 cudaError_t stream_launch(const StreamLaunch &a, cudaStream_t st);
 
 // ---- skinny.cu ------------------------------------------------------------------------------
-// 2..16 activation rows against one or more weights of one block type: the packed weights stream
-// through shared memory once and meet the exact bf16 activations in mma.sync with fp32 accumulation;
-// products whose K spans several 2048-weight chunks end with a small chunk-sum launch.
+// 2..32 activation rows against one or more weights of one block type: the packed weights stream
+// through shared memory once and meet fp16 activations in mma.sync with fp32 accumulation.
 struct SkinnyProduct {
     int qt;
     const uint8_t *w;        // streaming-layout weights
     int N, K, Kpad;
-    const void *x;           // activations [M][K], bf16 (M <= 16) or fp32 (M <= 8: hi/lo halves take two token slots)
+    const void *x;           // activations [M][K], bf16 or fp32 (M <= 16: as high and low halves; above: rounded to fp16)
     long long ldx;
     int x_is_bf16;
     void *y;
@@ -107,16 +106,20 @@ struct SkinnyProduct {
     int M;
 };
 struct SkinnyBuffers {
-    uint8_t *ws;             // chunk sums of the call (skinny_part_bytes per product)
+    uint8_t *ws;             // sums of shared tiles (skinny_ws_bytes, once through skinny_ws_init)
     size_t ws_bytes;
+    uint8_t *img;            // activation images: skinny_image_bytes of every product of its own x.  Launches that follow
+    size_t img_bytes;        // each other in a stream may share both
     void *jobs_dev;          // skinny_job_table_bytes() of device memory for calls with more than one product
     int *status;
     int sm_count;
-    size_t smem_limit;
 };
-int skinny_max_m();
+int skinny_max_m();          // the largest M of the exact route
+int skinny_max_mid_m();      // the largest M the kernels take
 int skinny_max_products();
-size_t skinny_part_bytes(const SkinnyProduct &a);
+size_t skinny_ws_bytes();
+cudaError_t skinny_ws_init(uint8_t *ws, bool own_stream);
+size_t skinny_image_bytes(const SkinnyProduct &a);
 size_t skinny_job_table_bytes();
 // at most four products (their descriptions travel in the kernel parameters): prepare, launch, forget
 cudaError_t skinny_run(const SkinnyProduct *prods, int n, const SkinnyBuffers &buf, cudaStream_t st, int *launches);
@@ -181,6 +184,8 @@ struct DenseLaunch {
 // 256 MB: all projections of an 8B-class model in one panel; with 128 MB the gate and up matrices of such a
 // layer took two, each with a partial last round (28672 x 4096, 512 rows: 165 us against 143)
 constexpr size_t kDenseScratchBytes = size_t(256) << 20;
+// 256 MB: all projections of an 8B-class model in one panel; with 128 MB the gate and up matrices of such a
+// layer took two, each with a partial last round (28672 x 4096, 512 rows: 165 us against 143)
 bool dense_pays(const DenseLaunch &a);    // worth two launches? (sizes only; scratch and pointers not needed)
 cudaError_t dense_gemm_run(const DenseLaunch &a, cudaStream_t st, int *launches);
 

@@ -1,0 +1,98 @@
+"""Edges of the small-batch kernels that the shapes of test_gpu_skinny.py do not reach.
+
+Tolerance, relative to max(|ref|, rms of the token's results): up to 16 tokens weights and activations enter exactly
+(activations to 2^-22 of their record's largest for fp32), so what remains is fp32 accumulation inside a
+record, at most 256 roundings of 2^-24 on sums a few times the result's rms: 1e-4.  Above 16 tokens fp32 activations
+and Q6_K weights are rounded to fp16, 2^-11 each, and errors of K independent terms add up to about 2^-11 of the rms;
+the largest of some thousand results is within a few times that: 2e-3.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+import magnitude_b200 as mb  # noqa: E402
+
+TYPES = [mb.TYPE_Q4_K, mb.TYPE_Q6_K, mb.TYPE_Q8_0, mb.TYPE_Q5_K, mb.TYPE_Q4_0, mb.TYPE_MXFP4]
+
+
+def _weights(orc, backend, qt, n, k, seed):
+    """Few distinct rows, so that a tall matrix is cheap to check: (handle, distinct rows dequantized, row of each)."""
+    rng = np.random.default_rng(seed)
+    base = orc.quantize(qt, rng.standard_normal((min(n, 96), k), dtype=np.float32) * np.float32(0.02))
+    index = rng.integers(0, len(base), n)
+    return backend.upload(qt, base[index], n, k), torch.from_numpy(orc.dequantize(qt, base, k)).cuda().double(), torch.from_numpy(index).cuda()
+
+
+def _check(y, x, rows, index, rel):
+    ref = (x.double() @ rows.T)[:, index]
+    rms = ref.pow(2).mean(dim=1, keepdim=True).sqrt()
+    worst = ((y.double() - ref).abs() / torch.maximum(ref.abs(), rms).clamp_min(1e-300)).max().item()
+    assert worst <= rel, f"worst error {worst:.2e}"
+
+
+# token tiles of 8, 16 and 32; tiles of 192 and 256 rows and one row more; whole, short and several chunks
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("m", [3, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("n,k", [(192, 256), (193, 2304), (257, 2048), (1025, 4352)])
+def test_tile_edges(backend, orc, qt, m, n, k):
+    w, rows, index = _weights(orc, backend, qt, n, k, n + m)
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32)).cuda()
+    for xx in (x.to(torch.bfloat16), x):
+        y = backend.project(w, xx)
+        backend.sync()
+        _check(y, xx, rows, index, 1e-4 if m <= 16 else 2e-3)
+
+
+# more slots per block than stages: prepared images, the ring goes round several times, tiles begin and end mid-block
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("m", [7, 16, 31])
+def test_many_slots_per_block(backend, orc, qt, m):
+    w, rows, index = _weights(orc, backend, qt, 12289, 8448, m)
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, 8448), dtype=np.float32)).cuda().to(torch.bfloat16)
+    for _ in range(2):                       # the second run finds the shared tiles' sums and counts as the first left them
+        y = backend.project(w, x)
+        backend.sync()
+        _check(y, x, rows, index, 1e-4 if m <= 16 else 2e-3)
+
+
+# every record has a scale of its own: tokens of very different size, records of zeros, one channel far above the rest
+@pytest.mark.parametrize("m", [8, 24])
+def test_activation_range(backend, orc, m):
+    k = 2048
+    w, rows, index = _weights(orc, backend, mb.TYPE_Q4_K, 300, k, 1)
+    x = torch.from_numpy(np.random.default_rng(2).standard_normal((m, k), dtype=np.float32)).cuda()
+    x *= torch.exp2(torch.linspace(-60, 60, m, device="cuda"))[:, None]
+    x[:, 256:512] = 0
+    x[:, 700] *= 4096
+    x[1] = 0
+    x = x.to(torch.bfloat16)
+    y = backend.project(w, x)
+    backend.sync()
+    _check(y, x, rows, index, 1e-4)          # bf16 tokens and Q4_K weights enter exactly at every batch size
+    assert torch.all(y[1] == 0)
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_non_finite_activations_stay_in_their_token(backend, orc, value):
+    w, rows, index = _weights(orc, backend, mb.TYPE_Q4_K, 300, 1024, 3)
+    x = torch.from_numpy(np.random.default_rng(4).standard_normal((8, 1024), dtype=np.float32)).cuda().to(torch.bfloat16)
+    x[5, 77] = value
+    y = backend.project(w, x)
+    backend.sync()
+    assert not torch.isfinite(y[5]).any()
+    keep = [0, 1, 2, 3, 4, 6, 7]
+    _check(y[keep], x[keep], rows, index, 1e-4)
+
+
+def test_a_product_has_the_same_bits_in_every_company(backend, orc):
+    shapes = [(700, 4096), (2048, 4096), (513, 4096)]
+    x = torch.from_numpy(np.random.default_rng(5).standard_normal((12, 4096), dtype=np.float32)).cuda().to(torch.bfloat16)
+    ws = [_weights(orc, backend, mb.TYPE_Q5_K, n, k, i)[0] for i, (n, k) in enumerate(shapes)]
+    alone = [backend.project(w, x) for w in ws]
+    for _ in range(3):
+        together = backend.project_multi(ws, x)
+        backend.sync()
+        for a, b in zip(alone, together):
+            assert torch.equal(a, b)
