@@ -83,7 +83,7 @@ enum {
     B200Q_ROUTE_SKINNY = 2, /* 3 <= M <= 16: streaming kernel, exact integer weights x exact bf16 activations in
                                mma.sync with fp32 accumulation */
     B200Q_ROUTE_GEMM = 3    /* larger M: activations converted to fp16, weights to fp16 or fp16-exact integers, fp32
-                               accumulation; mma.sync up to 32 rows, then tcgen05 / TMEM */
+                               accumulation; mma.sync up to 48 rows, then tcgen05 / TMEM */
 };
 
 /* Per-context settings (b200q_ctx_set_option). */

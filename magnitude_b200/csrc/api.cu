@@ -95,7 +95,7 @@ struct b200q_ctx {
     void *dense_w = nullptr;          // fp16 weights of the two-launch GEMM, one panel at a time
     size_t dense_w_bytes = 0;
     float *gemm_part = nullptr;       // K-split partial products of skinny batches (allocated on first use)
-    // small batches (2..32 rows): sums of tiles shared by several blocks
+    // small batches (2..48 rows): sums of tiles shared by several blocks
     uint8_t *sk_ws = nullptr;
     uint8_t *sk_img = nullptr;        // activation images
     size_t sk_img_bytes = 0;
@@ -103,7 +103,7 @@ struct b200q_ctx {
     bool peer_stale = false;          // a peer exchange timed out: the ranks' call counters no longer agree
     bool peer_ipc = true;             // peer buffers were mapped through CUDA IPC (else given as pointers)
     int skinny_min_m = 3;             // smallest M that takes the skinny route (smaller batches: the dp4a kernel)
-    int mid_max_m = 32;               // largest M that runs on the small-batch kernels (17 and more rows)
+    int mid_max_m = 48;               // largest M that runs on the small-batch kernels (17 and more rows)
     int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1, gemm_dense = -1;
     // tunables (environment overrides for experiments)
     int gemv_warps = 0, gemv_depth = 0, gemv_grid = 0, gemv_smem = 0, gemv_rows = 0, gemv_debug = 0, gemv_pdl = 1, gemv_teams = 2, gemv_xprep = 1, gemv_nap = 0;
@@ -408,7 +408,7 @@ b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int 
     return B200Q_OK;
 }
 
-// small batches: 2..32 activation rows, mma.sync on weights unpacked in registers (skinny.cu); all weights of
+// small batches: 2..48 activation rows, mma.sync on weights unpacked in registers (skinny.cu); all weights of
 // the call share x, type and K
 b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int M,
                         int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy, cudaStream_t st) {
@@ -479,6 +479,20 @@ b200q_status validate_mm(b200q_ctx *ctx, const b200q_weight *w, const void *x, i
     return B200Q_OK;
 }
 
+// 17..48 rows: the small-batch kernel runs all weights of a call in one launch, the one-CTA GEMM one after another, each
+// with few K ranges per SM.  us, small-batch / GEMM: Q4_K 4096 + 1024 rows of K = 4096, 17 tokens 18 / 27, 48 tokens 28 / 29;
+// 2 x 14336, 48 tokens 55 / 71; 2 x 25600 rows of K = 5120, 48 tokens 100 / 149.  A single weight: 14336 x 4096, 32 tokens
+// 30 / 35, 48 tokens 40 / 37; 4096 x 4096, 17 tokens 15.7 / 16.5, 32 tokens 18.5 / 16.5.
+bool mid_pays(const b200q_ctx *ctx, const b200q_weight *const *w, int nw, int M) {
+    int weights = 0;
+    int64_t slots = 0;
+    for (int i = 0; i < nw; ++i) {
+        weights += w[i]->N > 0;
+        slots += (w[i]->N + 191) / 192 * (w[i]->Kpad / 256);
+    }
+    return weights >= 2 || M <= 20 || (M <= 32 && slots >= 4 * (int64_t)ctx->sm_count);
+}
+
 // One weight set (1..4 weights sharing x), any M: picks the route and launches.
 b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype,
                         int64_t M, int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy,
@@ -504,7 +518,7 @@ b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
     }
     if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
         ctx->last_route = B200Q_ROUTE_GEMM;
-        if (M > skinny_max_m() && M <= ctx->mid_max_m)
+        if (M > skinny_max_m() && M <= ctx->mid_max_m && mid_pays(ctx, w, nw, (int)M))
             return run_skinny(ctx, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
         b200q_status ds = B200Q_OK;
         if (run_dense(ctx, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;

@@ -91,7 +91,7 @@ cudaError_t stream_xprep_launch(const StreamJob *jobs_dev, int njobs, int M, cud
 cudaError_t stream_launch(const StreamLaunch &a, cudaStream_t st);
 
 // ---- skinny.cu ------------------------------------------------------------------------------
-// 2..32 activation rows against one or more weights of one block type: the packed weights stream
+// 2..48 activation rows against one or more weights of one block type: the packed weights stream
 // through shared memory once and meet fp16 activations in mma.sync with fp32 accumulation.
 struct SkinnyProduct {
     int qt;

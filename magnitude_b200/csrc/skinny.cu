@@ -45,16 +45,16 @@ bool sk_encode(EncodeTiledFn enc, CUtensorMap *map, const uint8_t *w, int qt, in
 }
 
 int token_tiles(int M) {
-    return M <= 8 ? 1 : M <= 16 ? 2 : 4;
+    return M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 6;
 }
 
 }  // namespace
 
 int skinny_max_m() { return 16; }
-int skinny_max_mid_m() { return 32; }
+int skinny_max_mid_m() { return 48; }
 
-// sums of one shared tile per block (192 rows x 32 tokens is the largest, 256 x 16 the next), and their counts
-static constexpr size_t kSkSumBytes = size_t(kSkMaxGrid) * 192 * 32 * sizeof(double);
+// sums of one shared tile per block (192 rows x 48 tokens is the largest), and their counts
+static constexpr size_t kSkSumBytes = size_t(kSkMaxGrid) * 192 * 48 * sizeof(double);
 static constexpr size_t kSkCountBytes = size_t(kSkMaxGrid) * sk_warps(1) * sizeof(unsigned);
 size_t skinny_ws_bytes() { return kSkSumBytes + kSkCountBytes; }
 // Zeroes before it returns.  With a stream of its own it may be called while another stream is being captured.

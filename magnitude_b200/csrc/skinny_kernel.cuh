@@ -1,4 +1,4 @@
-// Small batches (2..32 activation rows; speculative-decode verify, sequences decoding together):
+// Small batches (2..48 activation rows; speculative-decode verify, sequences decoding together):
 // Y[m][n] = sum_k X[m][k] * W[n][k] with the packed weights read from HBM once.
 //
 // Two launches, or one where every block has few slots and makes what it needs of the first itself.
@@ -637,6 +637,7 @@ template <int QT> cudaError_t sk_launch_type(const SkParams &p, int NT, int P, i
     case 2 * 4 + 1: return sk_launch_t<QT, 2, 1>(p, grid, st);
     case 2 * 4 + 2: return sk_launch_t<QT, 2, 2>(p, grid, st);
     case 4 * 4 + 1: return sk_launch_t<QT, 4, 1>(p, grid, st);
+    case 6 * 4 + 1: return sk_launch_t<QT, 6, 1>(p, grid, st);
     default: return cudaErrorInvalidValue;
     }
 }

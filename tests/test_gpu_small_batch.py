@@ -57,8 +57,23 @@ def test_many_slots_per_block(backend, orc, qt, m):
         _check(y, x, rows, index, 1e-4 if m <= 16 else 2e-3)
 
 
+# several weights of up to 48 rows run on these kernels, too; a single one only where it is large enough
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("m", [20, 21, 33, 48, 49])
+def test_sets_of_weights_up_to_48_rows(backend, orc, qt, m):
+    shapes, k = [400, 193], 2304
+    ws = [_weights(orc, backend, qt, n, k, n) for n in shapes]
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32)).cuda()
+    for xx in (x.to(torch.bfloat16), x):
+        ys = backend.project_multi([w for w, _, _ in ws], xx)
+        one = backend.project(ws[0][0], xx)
+        backend.sync()
+        for y, (_, rows, index) in zip(ys + [one], ws + [ws[0]]):
+            _check(y, xx, rows, index, 2e-3)
+
+
 # every record has a scale of its own: tokens of very different size, records of zeros, one channel far above the rest
-@pytest.mark.parametrize("m", [8, 24])
+@pytest.mark.parametrize("m", [8, 20])
 def test_activation_range(backend, orc, m):
     k = 2048
     w, rows, index = _weights(orc, backend, mb.TYPE_Q4_K, 300, k, 1)
