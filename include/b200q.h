@@ -24,7 +24,8 @@
  *     threads (the library's one-time set-up is thread-safe);
  *   - calls are stream-ordered: each enqueues on the stream it is given and returns.  The scratch a
  *     context owns (fp16 activation copy, partial sums, dependency counters) is shared by all its
- *     b200q_matmul* calls, so keep one context's calls on one stream or order them with events;
+ *     b200q_matmul* calls, so keep one context's calls on one stream or order them with events (the
+ *     *_host calls have scratch of their own: they may run while device calls are in flight);
  *     a plan owns its scratch, but two runs of one plan must not overlap.  The first call with a
  *     larger M x K may allocate: make it before any stream capture;
  *   - weights are W[N][K] in GGUF order: N output rows, each K/blk consecutive packed blocks;

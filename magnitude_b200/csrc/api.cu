@@ -73,6 +73,28 @@ int env_int(const char *name, int dflt) {
 
 }  // namespace
 
+namespace {
+
+// What a call leaves in device memory between its launches.  Calls that share a set must be ordered by one stream.
+struct Scratch {
+    void *gemm_x = nullptr;           // fp16 copy of the activations
+    size_t gemm_x_bytes = 0;
+    void *dense_w = nullptr;          // fp16 weights of the two-launch GEMM, one panel at a time
+    size_t dense_w_bytes = 0;
+    float *gemm_part = nullptr;       // K-split partial products (allocated on first use)
+    // small batches (2..48 rows): sums of tiles shared by several blocks, zero between launches
+    uint8_t *sk_ws = nullptr;
+    uint8_t *sk_img = nullptr;        // activation images
+    size_t sk_img_bytes = 0;
+    void free_all() {
+        for (void *p : {gemm_x, dense_w, (void *)gemm_part, (void *)sk_ws, (void *)sk_img})
+            if (p) cudaFree(p);
+        *this = Scratch{};
+    }
+};
+
+}  // namespace
+
 struct b200q_ctx {
     int device = 0;
     int sm_count = 0;
@@ -89,16 +111,8 @@ struct b200q_ctx {
     size_t hx_bytes = 0;
     void *hy_dev = nullptr;
     size_t hy_bytes = 0;
-    // prefill path: bf16 copy of fp32 activations
-    void *gemm_scratch = nullptr;
-    size_t gemm_scratch_bytes = 0;
-    void *dense_w = nullptr;          // fp16 weights of the two-launch GEMM, one panel at a time
-    size_t dense_w_bytes = 0;
-    float *gemm_part = nullptr;       // K-split partial products of skinny batches (allocated on first use)
-    // small batches (2..48 rows): sums of tiles shared by several blocks
-    uint8_t *sk_ws = nullptr;
-    uint8_t *sk_img = nullptr;        // activation images
-    size_t sk_img_bytes = 0;
+    Scratch scratch;                  // calls on the caller's stream
+    Scratch hscratch;                 // host-buffer calls: the caller cannot order hstream after calls in flight on its own stream
     uint64_t tp_timeout_ms = 60000;   // host deadline of b200q_tp_init
     bool peer_stale = false;          // a peer exchange timed out: the ranks' call counters no longer agree
     bool peer_ipc = true;             // peer buffers were mapped through CUDA IPC (else given as pointers)
@@ -292,26 +306,26 @@ b200q_status run_gemv(b200q_ctx *ctx, const b200q_weight *const *w, int nw, cons
 }
 
 // scratch for the fp16 copy of M activation rows
-b200q_status ensure_gemm_scratch(b200q_ctx *ctx, int64_t M, int64_t K, cudaStream_t st) {
+b200q_status ensure_gemm_scratch(b200q_ctx *ctx, Scratch &sc, int64_t M, int64_t K, cudaStream_t st) {
     const size_t need = gemm_x_scratch_bytes((int)M, (int)K);
-    if (need <= ctx->gemm_scratch_bytes) return B200Q_OK;
-    if (ctx->gemm_scratch) {
+    if (need <= sc.gemm_x_bytes) return B200Q_OK;
+    if (sc.gemm_x) {
         CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still read the old buffer
-        cudaFree(ctx->gemm_scratch);
-        ctx->gemm_scratch = nullptr;
-        ctx->gemm_scratch_bytes = 0;
+        cudaFree(sc.gemm_x);
+        sc.gemm_x = nullptr;
+        sc.gemm_x_bytes = 0;
     }
-    CU_TRY(ctx, cudaMalloc(&ctx->gemm_scratch, need));
-    ctx->gemm_scratch_bytes = need;
+    CU_TRY(ctx, cudaMalloc(&sc.gemm_x, need));
+    sc.gemm_x_bytes = need;
     return B200Q_OK;
 }
 
 // Workspace for the fp16 weights of the two-launch GEMM: a fixed size from the first use on (only a K above
 // 262144 asks for more), so that a later call with larger weights allocates nothing.  False where it
 // cannot be had (no memory, or the stream is being captured): the one-launch kernels take the call.
-bool ensure_dense_scratch(b200q_ctx *ctx, int64_t Kpad, cudaStream_t st) {
+bool ensure_dense_scratch(Scratch &sc, int64_t Kpad, cudaStream_t st) {
     const size_t need = std::max(kDenseScratchBytes, (size_t)Kpad * 2 * 256);
-    if (need <= ctx->dense_w_bytes) return true;
+    if (need <= sc.dense_w_bytes) return true;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
@@ -322,15 +336,15 @@ bool ensure_dense_scratch(b200q_ctx *ctx, int64_t Kpad, cudaStream_t st) {
         cudaGetLastError();
         return false;
     }
-    if (ctx->dense_w) cudaFree(ctx->dense_w);      // waits for the device: earlier launches may still read it
-    ctx->dense_w = ptr;
-    ctx->dense_w_bytes = need;
+    if (sc.dense_w) cudaFree(sc.dense_w);      // waits for the device: earlier launches may still read it
+    sc.dense_w = ptr;
+    sc.dense_w_bytes = need;
     return true;
 }
 
 // Larger batches: fp16 copies of the activations and of all the call's weights, then one dense GEMM over them.
 // False: the one-launch kernels are the faster ones here, or there is no workspace.
-bool run_dense(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int64_t M, int64_t ldx,
+bool run_dense(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int64_t M, int64_t ldx,
                void *const *y, int y_dtype, const int64_t *ldy, cudaStream_t st, b200q_status *status) {
     if (ctx->gemm_pair != 1 || ctx->gemm_dense == 0 || M < (ctx->gemm_dense > 0 ? ctx->gemm_dense : 128)) return false;
     DenseLaunch a{};
@@ -354,29 +368,29 @@ bool run_dense(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void 
     a.sm_count = ctx->sm_count;
     a.bn_override = ctx->gemm_bn;
     if (ctx->gemm_dense < 0 && !dense_pays(a)) return false;
-    if (!ensure_dense_scratch(ctx, a.Kpad, st)) return false;
-    a.scratch = ctx->dense_w;
-    a.scratch_bytes = ctx->dense_w_bytes;
-    if ((*status = ensure_gemm_scratch(ctx, M, a.K, st)) != B200Q_OK) return true;
-    a.x16 = ctx->gemm_scratch;
+    if (!ensure_dense_scratch(sc, a.Kpad, st)) return false;
+    a.scratch = sc.dense_w;
+    a.scratch_bytes = sc.dense_w_bytes;
+    if ((*status = ensure_gemm_scratch(ctx, sc, M, a.K, st)) != B200Q_OK) return true;
+    a.x16 = sc.gemm_x;
     cudaError_t e = dense_gemm_run(a, st, &ctx->last_launches);
     if (e != cudaSuccess) *status = cuda_fail(ctx, e, "dense GEMM launch");
     return true;
 }
 
 // prefill route: one activation conversion per weight set and one tensor-core launch per weight
-b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int x_dtype, int64_t M, int64_t ldx,
+b200q_status run_gemm(b200q_ctx *ctx, Scratch &sc, const b200q_weight *w, const void *x, int x_dtype, int64_t M, int64_t ldx,
                       void *y, int y_dtype, int64_t ldy, cudaStream_t st, int *launches, bool x_already_converted) {
     // Both tensor-core operands are fp16: the activations are converted into context-owned scratch
     // memory first (once for all the weights of a set, which share them).
     if (!x_already_converted) {
-        b200q_status s = ensure_gemm_scratch(ctx, M, w->K, st);
+        b200q_status s = ensure_gemm_scratch(ctx, sc, M, w->K, st);
         if (s != B200Q_OK) return s;
-        cudaError_t e = gemm_convert_x(x, x_dtype == B200Q_TYPE_BF16, ldx, ctx->gemm_scratch, (int)M, (int)w->K, st);
+        cudaError_t e = gemm_convert_x(x, x_dtype == B200Q_TYPE_BF16, ldx, sc.gemm_x, (int)M, (int)w->K, st);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "activation conversion launch");
         ++*launches;
     }
-    const void *xb = ctx->gemm_scratch;
+    const void *xb = sc.gemm_x;
     const long long ldb = (w->K + 7) & ~int64_t(7);
     GemmLaunch a{};
     a.qt = w->type;
@@ -395,12 +409,12 @@ b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int 
     a.bn_override = ctx->gemm_bn;
     a.debug = ctx->gemm_debug;
     a.pair = ctx->gemm_pair;
-    if (M < 128 && !ctx->gemm_part && ctx->gemm_ksplit) {
+    if (M < 128 && !sc.gemm_part && ctx->gemm_ksplit) {
         void *ptr = nullptr;
-        if (cudaMalloc(&ptr, kGemmPartBytes) == cudaSuccess) ctx->gemm_part = reinterpret_cast<float *>(ptr);
+        if (cudaMalloc(&ptr, kGemmPartBytes) == cudaSuccess) sc.gemm_part = reinterpret_cast<float *>(ptr);
         else cudaGetLastError();      // no workspace: the product runs unsplit
     }
-    a.part = ctx->gemm_ksplit ? ctx->gemm_part : nullptr;
+    a.part = ctx->gemm_ksplit ? sc.gemm_part : nullptr;
     a.part_bytes = kGemmPartBytes;
     cudaError_t e = gemm_launch(a, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "tensor-core GEMM launch");
@@ -410,7 +424,7 @@ b200q_status run_gemm(b200q_ctx *ctx, const b200q_weight *w, const void *x, int 
 
 // small batches: 2..48 activation rows, mma.sync on weights unpacked in registers (skinny.cu); all weights of
 // the call share x, type and K
-b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int M,
+b200q_status run_skinny(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int M,
                         int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy, cudaStream_t st) {
     SkinnyProduct prods[4];
     int n = 0;
@@ -431,7 +445,7 @@ b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
         a.M = M;
     }
     if (n == 0) return B200Q_OK;
-    if (!ctx->sk_ws) {           // one size serves every call
+    if (!sc.sk_ws) {           // one size serves every call
         uint8_t *ws = nullptr;
         CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), skinny_ws_bytes()));
         cudaError_t e = skinny_ws_init(ws, true);
@@ -439,25 +453,25 @@ b200q_status run_skinny(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
             cudaFree(ws);
             return cuda_fail(ctx, e, "small-batch workspace");
         }
-        ctx->sk_ws = ws;
+        sc.sk_ws = ws;
     }
     const size_t need = skinny_image_bytes(prods[0]);      // the call's weights share x
-    if (need > ctx->sk_img_bytes) {
-        if (ctx->sk_img) {
+    if (need > sc.sk_img_bytes) {
+        if (sc.sk_img) {
             CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still use the old buffer
-            cudaFree(ctx->sk_img);
-            ctx->sk_img = nullptr;
-            ctx->sk_img_bytes = 0;
+            cudaFree(sc.sk_img);
+            sc.sk_img = nullptr;
+            sc.sk_img_bytes = 0;
         }
         const size_t grow = std::max(need, size_t(8) << 20);
-        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ctx->sk_img), grow));
-        ctx->sk_img_bytes = grow;
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&sc.sk_img), grow));
+        sc.sk_img_bytes = grow;
     }
     SkinnyBuffers buf{};
-    buf.ws = ctx->sk_ws;
+    buf.ws = sc.sk_ws;
     buf.ws_bytes = skinny_ws_bytes();
-    buf.img = ctx->sk_img;
-    buf.img_bytes = ctx->sk_img_bytes;
+    buf.img = sc.sk_img;
+    buf.img_bytes = sc.sk_img_bytes;
     buf.jobs_dev = nullptr;      // at most four products: their descriptions travel in the kernel parameters
     buf.status = ctx->status_dev;
     buf.sm_count = ctx->sm_count;
@@ -494,7 +508,7 @@ bool mid_pays(const b200q_ctx *ctx, const b200q_weight *const *w, int nw, int M)
 }
 
 // One weight set (1..4 weights sharing x), any M: picks the route and launches.
-b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, const void *x, int x_dtype,
+b200q_status matmul_any(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *w, int nw, const void *x, int x_dtype,
                         int64_t M, int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy,
                         cudaStream_t st) {
     ctx->last_route = B200Q_ROUTE_NONE;
@@ -514,18 +528,18 @@ b200q_status matmul_any(b200q_ctx *ctx, const b200q_weight *const *w, int nw, co
     if (M >= ctx->skinny_min_m && M <= skinny_max_m()) {
         // verify / small continuous batches: one pass over the packed weights, exact bf16 activations
         ctx->last_route = B200Q_ROUTE_SKINNY;
-        return run_skinny(ctx, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
+        return run_skinny(ctx, sc, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
     }
     if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
         ctx->last_route = B200Q_ROUTE_GEMM;
         if (M > skinny_max_m() && M <= ctx->mid_max_m && mid_pays(ctx, w, nw, (int)M))
-            return run_skinny(ctx, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
+            return run_skinny(ctx, sc, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
         b200q_status ds = B200Q_OK;
-        if (run_dense(ctx, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;
+        if (run_dense(ctx, sc, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;
         bool converted = false;
         for (int i = 0; i < nw; ++i) {
             if (w[i]->N == 0) continue;
-            b200q_status s = run_gemm(ctx, w[i], x, x_dtype, M, ldx, y[i], y_dtype, ldy[i], st, &ctx->last_launches, converted);
+            b200q_status s = run_gemm(ctx, sc, w[i], x, x_dtype, M, ldx, y[i], y_dtype, ldy[i], st, &ctx->last_launches, converted);
             if (s != B200Q_OK) return s;
             converted = true;
         }
@@ -717,11 +731,8 @@ void b200q_ctx_destroy(b200q_ctx *ctx) {
     if (ctx->hstream) cudaStreamDestroy(ctx->hstream);
     if (ctx->hx_dev) cudaFree(ctx->hx_dev);
     if (ctx->hy_dev) cudaFree(ctx->hy_dev);
-    if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
-    if (ctx->dense_w) cudaFree(ctx->dense_w);
-    if (ctx->gemm_part) cudaFree(ctx->gemm_part);
-    if (ctx->sk_ws) cudaFree(ctx->sk_ws);
-    if (ctx->sk_img) cudaFree(ctx->sk_img);
+    ctx->scratch.free_all();
+    ctx->hscratch.free_all();
     if (ctx->status_dev) cudaFree(ctx->status_dev);
     delete ctx;
 }
@@ -806,6 +817,8 @@ b200q_status b200q_sync(b200q_ctx *ctx, void *stream, uint64_t timeout_ms) {
     CU_TRY(ctx, cudaMemcpy(&status, ctx->status_dev, sizeof(int), cudaMemcpyDeviceToHost));
     if (status != DEV_OK) {
         cudaMemset(ctx->status_dev, 0, sizeof(int));
+        for (Scratch *sc : {&ctx->scratch, &ctx->hscratch})      // a later call must find the shared tiles' sums at zero
+            if (sc->sk_ws) CU_TRY(ctx, skinny_ws_init(sc->sk_ws, true));
         if (ctx->peer_world > 1) ctx->peer_stale = true;     // some rank may have skipped an exchange: counters disagree
         return fail(ctx, B200Q_ERR_TIMEOUT, "a kernel gave up a bounded wait (device status %d); results are invalid", status);
     }
@@ -944,7 +957,7 @@ b200q_status b200q_matmul(b200q_ctx *ctx, const b200q_weight *w, const void *x_d
     b200q_status s = check_ctx(ctx);
     if (s != B200Q_OK) return s;
     if ((s = validate_mm(ctx, w, x_dev, x_dtype, M, ldx, y_dev, y_dtype, ldy)) != B200Q_OK) return s;
-    return matmul_any(ctx, &w, 1, x_dev, x_dtype, M, ldx, &y_dev, y_dtype, &ldy, (cudaStream_t)stream);
+    return matmul_any(ctx, ctx->scratch, &w, 1, x_dev, x_dtype, M, ldx, &y_dev, y_dtype, &ldy, (cudaStream_t)stream);
 }
 
 b200q_status b200q_matmul_multi(b200q_ctx *ctx, const b200q_weight *const *w, int32_t n_weights,
@@ -959,7 +972,7 @@ b200q_status b200q_matmul_multi(b200q_ctx *ctx, const b200q_weight *const *w, in
         if (w[i]->type != w[0]->type || w[i]->K != w[0]->K)
             return fail(ctx, B200Q_ERR_INVALID_CONFIG, "weights of one launch must share type and K");
     }
-    return matmul_any(ctx, w, n_weights, x_dev, x_dtype, M, ldx, y_dev, y_dtype, ldy, (cudaStream_t)stream);
+    return matmul_any(ctx, ctx->scratch, w, n_weights, x_dev, x_dtype, M, ldx, y_dev, y_dtype, ldy, (cudaStream_t)stream);
 }
 
 b200q_status b200q_matmul_multi_host(b200q_ctx *ctx, const b200q_weight *const *w, int32_t n_weights,
@@ -987,7 +1000,7 @@ b200q_status b200q_matmul_multi_host(b200q_ctx *ctx, const b200q_weight *const *
     CU_TRY(ctx, cudaMemcpyAsync(ctx->hx_dev, x_host, xb, cudaMemcpyHostToDevice, st));
     void *yd[4];
     for (int i = 0; i < n_weights; ++i) yd[i] = (char *)ctx->hy_dev + yoff[i];
-    if ((s = matmul_any(ctx, w, n_weights, ctx->hx_dev, x_dtype, M, ldx, yd, y_dtype, ldy, st)) != B200Q_OK) return s;
+    if ((s = matmul_any(ctx, ctx->hscratch, w, n_weights, ctx->hx_dev, x_dtype, M, ldx, yd, y_dtype, ldy, st)) != B200Q_OK) return s;
     for (int i = 0; i < n_weights; ++i)
         if (w[i]->N > 0)
             CU_TRY(ctx, cudaMemcpyAsync(y_host[i], yd[i], (size_t)((M - 1) * ldy[i] + w[i]->N) * ys, cudaMemcpyDeviceToHost, st));

@@ -111,3 +111,27 @@ def test_a_product_has_the_same_bits_in_every_company(backend, orc):
         backend.sync()
         for a, b in zip(alone, together):
             assert torch.equal(a, b)
+
+
+# Host-buffer calls run on a stream of the library's own, which nothing orders after the calls in flight on the caller's:
+# the two must not meet in a workspace.  Tiles shared by several blocks are the state that an overlap would spoil for good.
+@pytest.mark.parametrize("m,m_host", [(8, 8), (16, 5), (20, 40), (300, 200)])
+def test_host_calls_beside_device_calls(backend, orc, m, m_host):
+    rel = 1e-4 if max(m, m_host) <= 16 else 2e-3
+    w, rows, index = _weights(orc, backend, mb.TYPE_Q4_K, 1200, 8192, 6)
+    h, hrows, hindex = _weights(orc, backend, mb.TYPE_Q6_K, 2100, 2304, 7)
+    x = torch.from_numpy(np.random.default_rng(8).standard_normal((m, 8192), dtype=np.float32)).cuda()
+    xh = np.random.default_rng(9).standard_normal((m_host, 2304), dtype=np.float32)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    out = [torch.empty((m, 1200), device="cuda") for _ in range(200)]
+    for y in out:
+        backend.project(w, x, out=y, stream=stream)
+    hosts = [backend.project_host(h, xh) for _ in range(10)]
+    backend.sync(stream)
+    last = backend.project(w, x)
+    backend.sync()
+    for y in out + [last]:
+        _check(y, x, rows, index, rel)
+    for y in hosts:
+        _check(torch.from_numpy(y).cuda(), torch.from_numpy(xh).cuda(), hrows, hindex, rel)
