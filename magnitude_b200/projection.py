@@ -164,8 +164,10 @@ class Backend:
             torch = _torch()
             if torch.cuda.is_initialized():
                 # the current device's current stream, without the Stream object torch.cuda.current_stream() makes:
-                # with it (and is_available(), which asks the driver) a call's host time was several microseconds longer
-                return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+                # with it (and is_available(), which asks the driver) a call's host time was several microseconds longer.
+                # The names are torch's own business, so a torch without them takes the public way.
+                raw, dev = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+                return c_void_p(raw(dev()) if raw and dev else torch.cuda.current_stream().cuda_stream)
             return c_void_p(0)
         if isinstance(stream, int):
             return c_void_p(stream)

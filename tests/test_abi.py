@@ -183,3 +183,15 @@ def test_no_cpu_fallback_without_a_device():
 def test_missing_library_fails_loudly(tmp_path):
     with pytest.raises(ImportError):
         B.load_library(tmp_path / "libb200q.so")
+
+
+def test_current_stream_without_private_torch_names(monkeypatch):
+    from types import SimpleNamespace as NS
+
+    from magnitude_b200 import projection
+
+    cuda = NS(is_initialized=lambda: True, current_stream=lambda: NS(cuda_stream=4242))
+    private = NS(_cuda_getCurrentRawStream=lambda device: 100 + device, _cuda_getDevice=lambda: 3)
+    for names, want in ((private, 103), (NS(), 4242)):
+        monkeypatch.setattr(projection, "_torch", lambda names=names: NS(cuda=cuda, _C=names))
+        assert projection.Backend._stream_ptr(None).value == want
