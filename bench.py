@@ -43,9 +43,10 @@ FALLBACK_TFLOPS = 1400.0
 # DRAM traffic of the dominant kernels from one ncu capture each (dram__bytes_read.sum +
 # dram__bytes_write.sum per launch; summaries under profiles/).  The decode figure was captured on a
 # 4-layer launch and is proportional to the layers a launch streams, so it is kept as a ratio to
-# the algorithmic bytes; a prefill launch is one whole product whatever the number of copies.
+# the algorithmic bytes; the two launches of a prefill product (fp16 copies, then the GEMM on them: 123.7 + 177.7 MB) are
+# one whole product whatever the number of copies.
 NCU_DECODE_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.014
-NCU_PREFILL_TRAFFIC_BYTES_PER_LAUNCH = 73.9e6
+NCU_PREFILL_TRAFFIC_BYTES_PER_PRODUCT = 301.4e6
 
 
 def peaks():
@@ -847,12 +848,12 @@ def run_prefill(args, emit=True):
         "warmup": max(args.warmup, 3), "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
         "dtype": "fp16 x fp16 tcgen05.mma, fp32 accumulate in TMEM (weights dequantized exactly to fp16, activations bf16 -> fp16)",
         "data": "synthetic", "config": cfg,
-        "roofline": {"bound": "tensor", "kernel": "gemm_tc_pair_kernel<Q4_K> (+ convert_x_vec8_kernel per product)", "achieved": value,
+        "roofline": {"bound": "tensor", "kernel": "dense_gemm_kernel (+ dense_prep_kernel<Q4_K> per product)", "achieved": value,
                      "peak": burst or peak, "unit": "TFLOP/s", "frac": value / (burst or peak),
                      "peak_source": f"of {'measured (burst: the timed region lasts tens of milliseconds)' if burst else src}",
-                     "peak_sustained": peak, "frac_of_sustained": value / peak, "traffic": NCU_PREFILL_TRAFFIC_BYTES_PER_LAUNCH,
+                     "peak_sustained": peak, "frac_of_sustained": value / peak, "traffic": NCU_PREFILL_TRAFFIC_BYTES_PER_PRODUCT,
                      "us_per_launch": ms_step * 1e3 / copies,
-                     "note": "2*M*N*K per product / device time per product, activation conversion launch included"},
+                     "note": "2*M*N*K per product / device time per product, the launch that makes the fp16 copies included"},
         "cpu_baseline": None,
         "e2e": {"value": flops_one * copies / e2e_s / 1e12, "unit": "TFLOP/s", "h2d_bytes_per_step": M * K * 2,
                 "d2h_bytes_per_step": M * N * 2, "ms_per_step": e2e_s * 1e3,
