@@ -224,6 +224,7 @@ b200q_status make_weight(b200q_ctx *ctx, int type, int64_t N, int64_t Kfull, con
         cudaError_t e = cudaMalloc(&w->dev, w->device_bytes + 256);
         if (e == cudaSuccess) e = cudaMemcpy(w->dev, staged.data(), w->device_bytes, cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemset(w->dev + w->device_bytes, 0, 256);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);      // in place before a call on any stream reads it
         if (e != cudaSuccess) {
             if (w->dev) cudaFree(w->dev);
             delete w;
@@ -908,6 +909,7 @@ b200q_status b200q_weight_clone(b200q_ctx *ctx, const b200q_weight *w, b200q_wei
     if (w->dev) {
         cudaError_t e = cudaMalloc(&c->dev, w->device_bytes + 256);
         if (e == cudaSuccess) e = cudaMemcpy(c->dev, w->dev, w->device_bytes + 256, cudaMemcpyDeviceToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) {
             if (c->dev) cudaFree(c->dev);
             delete c;
@@ -1164,6 +1166,7 @@ b200q_status b200q_plan_create(b200q_ctx *ctx, const b200q_job *jobs, int32_t n_
         const size_t bytes = pl->jobs.size() * sizeof(StreamJob);
         cudaError_t e = cudaMalloc(&pl->jobs_dev, bytes);
         if (e == cudaSuccess) e = cudaMemcpy(pl->jobs_dev, pl->jobs.data(), bytes, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) {
             if (pl->jobs_dev) cudaFree(pl->jobs_dev);
             delete pl;

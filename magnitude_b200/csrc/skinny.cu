@@ -140,6 +140,7 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
     if (n > kSkInline) {
         if (!buf.jobs_dev) return cudaErrorInvalidValue;
         cudaError_t e = cudaMemcpy(buf.jobs_dev, jobs, sizeof(SkJob) * (size_t)n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);     // a copy from pageable memory may return before it has arrived
         if (e != cudaSuccess) return e;
         p.jobs = reinterpret_cast<const SkJob *>(buf.jobs_dev);
     }

@@ -135,3 +135,24 @@ def test_host_calls_beside_device_calls(backend, orc, m, m_host):
         _check(y, x, rows, index, rel)
     for y in hosts:
         _check(torch.from_numpy(y).cuda(), torch.from_numpy(xh).cuda(), hrows, hindex, rel)
+
+
+# Plans of more than four products keep the tensor maps of their weights in device memory.  A plan made after another one was
+# destroyed may get the same address for other weights; run on a stream that is not ordered after the upload by itself.
+@pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K])
+def test_plans_made_and_destroyed_in_turn(backend, orc, qt):
+    stream = torch.cuda.Stream()
+    sets = []
+    for k in (512, 2304, 4096):
+        sets.append((k, [_weights(orc, backend, qt, 300 + 64 * i, k, k + i) for i in range(6)]))
+    for turn in range(12):
+        k, ws = sets[turn % 3]
+        x = torch.from_numpy(np.random.default_rng(turn).standard_normal((6, k), dtype=np.float32)).cuda().to(torch.bfloat16)
+        ys = [torch.empty((6, w.n), device="cuda") for w, _, _ in ws]
+        torch.cuda.synchronize()
+        plan = backend.plan([([w], x, [y]) for (w, _, _), y in zip(ws, ys)])
+        plan.run(stream=stream)
+        backend.sync(stream)
+        for y, (_, rows, index) in zip(ys, ws):
+            _check(y, x, rows, index, 1e-4)
+        plan.close()
