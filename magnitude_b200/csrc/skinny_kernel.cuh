@@ -598,6 +598,7 @@ __global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel
                                  : "l"(p.count + b0 * kSkConsumers + warp), "r"((unsigned)(b1 - b0))
                                  : "memory");
                 if (__shfl_sync(0xFFFFFFFFu, old, 0) != (unsigned)(b1 - b0)) continue;
+                __syncwarp();        // what lane 0 acquired is ordered before the other lanes' reads, too (a shuffle orders no memory)
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
