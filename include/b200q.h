@@ -26,8 +26,8 @@
  *     context owns (fp16 activation copy, partial sums, dependency counters) is shared by all its
  *     b200q_matmul* calls, so keep one context's calls on one stream or order them with events (the
  *     *_host calls have scratch of their own: they may run while device calls are in flight);
- *     a plan owns its scratch, but two runs of one plan must not overlap.  The first call with a
- *     larger M x K may allocate: make it before any stream capture;
+ *     a plan owns its scratch, but two runs of one plan must not overlap.  The first call of
+ *     a route, or with a larger M x K, may allocate: make it before any stream capture;
  *   - weights are W[N][K] in GGUF order: N output rows, each K/blk consecutive packed blocks;
  *   - activations X[M][K] and outputs Y[M][N] are row-major with leading dimensions in elements.
  *   - there is no CPU fallback: without a CUDA device every compute call fails with

@@ -423,6 +423,32 @@ b200q_status run_gemm(b200q_ctx *ctx, Scratch &sc, const b200q_weight *w, const 
     return B200Q_OK;
 }
 
+// workspaces of the small-batch kernels: shared tiles' sums (one size serves every call) and `need` bytes of activation images
+b200q_status ensure_skinny_scratch(b200q_ctx *ctx, Scratch &sc, size_t need, cudaStream_t st) {
+    if (!sc.sk_ws) {
+        uint8_t *ws = nullptr;
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), skinny_ws_bytes()));
+        cudaError_t e = skinny_ws_init(ws, true);
+        if (e != cudaSuccess) {
+            cudaFree(ws);
+            return cuda_fail(ctx, e, "small-batch workspace");
+        }
+        sc.sk_ws = ws;
+    }
+    if (need > sc.sk_img_bytes) {
+        if (sc.sk_img) {
+            CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still use the old buffer
+            cudaFree(sc.sk_img);
+            sc.sk_img = nullptr;
+            sc.sk_img_bytes = 0;
+        }
+        const size_t grow = std::max(need, size_t(8) << 20);
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&sc.sk_img), grow));
+        sc.sk_img_bytes = grow;
+    }
+    return B200Q_OK;
+}
+
 // small batches: 2..48 activation rows, mma.sync on weights unpacked in registers (skinny.cu); all weights of
 // the call share x, type and K
 b200q_status run_skinny(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int M,
@@ -446,28 +472,8 @@ b200q_status run_skinny(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *
         a.M = M;
     }
     if (n == 0) return B200Q_OK;
-    if (!sc.sk_ws) {           // one size serves every call
-        uint8_t *ws = nullptr;
-        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), skinny_ws_bytes()));
-        cudaError_t e = skinny_ws_init(ws, true);
-        if (e != cudaSuccess) {
-            cudaFree(ws);
-            return cuda_fail(ctx, e, "small-batch workspace");
-        }
-        sc.sk_ws = ws;
-    }
-    const size_t need = skinny_image_bytes(prods[0]);      // the call's weights share x
-    if (need > sc.sk_img_bytes) {
-        if (sc.sk_img) {
-            CU_TRY(ctx, cudaStreamSynchronize(st));   // earlier launches may still use the old buffer
-            cudaFree(sc.sk_img);
-            sc.sk_img = nullptr;
-            sc.sk_img_bytes = 0;
-        }
-        const size_t grow = std::max(need, size_t(8) << 20);
-        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&sc.sk_img), grow));
-        sc.sk_img_bytes = grow;
-    }
+    b200q_status s = ensure_skinny_scratch(ctx, sc, skinny_image_bytes(prods[0]), st);      // the call's weights share x
+    if (s != B200Q_OK) return s;
     SkinnyBuffers buf{};
     buf.ws = sc.sk_ws;
     buf.ws_bytes = skinny_ws_bytes();
@@ -508,6 +514,23 @@ bool mid_pays(const b200q_ctx *ctx, const b200q_weight *const *w, int nw, int M)
     return weights >= 2 || M <= 20 || (M <= 32 && slots >= 4 * (int64_t)ctx->sm_count);
 }
 
+// The tensor-core kernels take 17 and more rows as well: where the small-batch kernels' workspaces are missing and cannot be
+// had (no memory, or the stream is being captured), they do.
+bool mid_scratch(b200q_ctx *ctx, Scratch &sc, const b200q_weight *w, int x_dtype, int M, cudaStream_t st) {
+    SkinnyProduct a{};
+    a.K = (int)w->K;
+    a.Kpad = (int)w->Kpad;
+    a.x_is_bf16 = x_dtype == B200Q_TYPE_BF16;
+    a.M = M;
+    const size_t need = skinny_image_bytes(a);
+    if (sc.sk_ws && need <= sc.sk_img_bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool ok = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+                    ensure_skinny_scratch(ctx, sc, need, st) == B200Q_OK;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
 // One weight set (1..4 weights sharing x), any M: picks the route and launches.
 b200q_status matmul_any(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *w, int nw, const void *x, int x_dtype,
                         int64_t M, int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy,
@@ -533,7 +556,7 @@ b200q_status matmul_any(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *
     }
     if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
         ctx->last_route = B200Q_ROUTE_GEMM;
-        if (M > skinny_max_m() && M <= ctx->mid_max_m && mid_pays(ctx, w, nw, (int)M))
+        if (M > skinny_max_m() && M <= ctx->mid_max_m && mid_pays(ctx, w, nw, (int)M) && mid_scratch(ctx, sc, w[0], x_dtype, (int)M, st))
             return run_skinny(ctx, sc, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
         b200q_status ds = B200Q_OK;
         if (run_dense(ctx, sc, w, nw, x, x_dtype, M, ldx, y, y_dtype, ldy, st, &ds)) return ds;

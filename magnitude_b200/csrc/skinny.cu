@@ -57,7 +57,7 @@ int skinny_max_mid_m() { return 48; }
 static constexpr size_t kSkSumBytes = size_t(kSkMaxGrid) * 192 * 48 * sizeof(double);
 static constexpr size_t kSkCountBytes = size_t(kSkMaxGrid) * sk_warps(1) * sizeof(unsigned);
 size_t skinny_ws_bytes() { return kSkSumBytes + kSkCountBytes; }
-// Zeroes before it returns.  With a stream of its own it may be called while another stream is being captured.
+// Zeroes before it returns, on the legacy stream or on one of its own, which waits for no other.
 cudaError_t skinny_ws_init(uint8_t *ws, bool own_stream) {
     cudaStream_t st = nullptr;
     cudaError_t e = own_stream ? cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) : cudaSuccess;

@@ -156,3 +156,47 @@ def test_plans_made_and_destroyed_in_turn(backend, orc, qt):
         for y, (_, rows, index) in zip(ys, ws):
             _check(y, x, rows, index, 1e-4)
         plan.close()
+
+
+def _captured(call, warm):
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        warm()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    return graph
+
+
+@pytest.mark.parametrize("m,n", [(8, [640]), (16, [300, 1025]), (32, [640, 640])])
+def test_replay_from_a_graph(backend, orc, m, n):
+    k = 4352
+    ws = [_weights(orc, backend, mb.TYPE_Q5_K, i, k, i) for i in n]
+    x = torch.zeros((m, k), dtype=torch.bfloat16, device="cuda")
+    ys = [torch.empty((m, i), device="cuda") for i in n]
+    call = lambda: backend.project_multi([w for w, _, _ in ws], x, ys)      # noqa: E731
+    graph = _captured(call, call)
+    for turn in range(3):
+        x.copy_(torch.from_numpy(np.random.default_rng(turn).standard_normal((m, k), dtype=np.float32)))
+        graph.replay()
+        backend.sync()
+        for y, (_, rows, index) in zip(ys, ws):
+            _check(y, x, rows, index, 1e-4 if m <= 16 else 2e-3)
+
+
+# A set of 32 rows captured before the small-batch kernels' workspaces exist: a larger call has made what the GEMM needs
+def test_capture_without_the_workspaces(orc):
+    be = mb.Backend(0)
+    k = 2048
+    ws = [_weights(orc, be, mb.TYPE_Q4_K, n, k, n) for n in (400, 300)]
+    x = torch.from_numpy(np.random.default_rng(1).standard_normal((100, k), dtype=np.float32)).cuda().to(torch.bfloat16)
+    ys = [torch.zeros((32, n), device="cuda") for n in (400, 300)]
+    graph = _captured(lambda: be.project_multi([w for w, _, _ in ws], x[:32], ys), lambda: be.project(ws[0][0], x))
+    graph.replay()
+    be.sync()
+    for y, (_, rows, index) in zip(ys, ws):
+        _check(y, x[:32], rows, index, 2e-3)
+    del graph
+    be.close()
