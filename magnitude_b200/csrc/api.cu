@@ -423,12 +423,14 @@ b200q_status run_gemm(b200q_ctx *ctx, Scratch &sc, const b200q_weight *w, const 
     return B200Q_OK;
 }
 
+size_t ctx_ws_bytes(const b200q_ctx *ctx) { return skinny_ws_bytes(skinny_max_mid_m(), ctx->sm_count); }
+
 // workspaces of the small-batch kernels: shared tiles' sums (one size serves every call) and `need` bytes of activation images
 b200q_status ensure_skinny_scratch(b200q_ctx *ctx, Scratch &sc, size_t need, cudaStream_t st) {
     if (!sc.sk_ws) {
         uint8_t *ws = nullptr;
-        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), skinny_ws_bytes()));
-        cudaError_t e = skinny_ws_init(ws, true);
+        CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&ws), ctx_ws_bytes(ctx)));
+        cudaError_t e = skinny_ws_init(ws, ctx_ws_bytes(ctx), true);
         if (e != cudaSuccess) {
             cudaFree(ws);
             return cuda_fail(ctx, e, "small-batch workspace");
@@ -476,7 +478,7 @@ b200q_status run_skinny(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *
     if (s != B200Q_OK) return s;
     SkinnyBuffers buf{};
     buf.ws = sc.sk_ws;
-    buf.ws_bytes = skinny_ws_bytes();
+    buf.ws_bytes = ctx_ws_bytes(ctx);
     buf.img = sc.sk_img;
     buf.img_bytes = sc.sk_img_bytes;
     buf.jobs_dev = nullptr;      // at most four products: their descriptions travel in the kernel parameters
@@ -647,8 +649,9 @@ b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job 
     }
     if (groups.empty()) return B200Q_OK;
     // the groups run one after another and share the workspaces
-    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_ws), skinny_ws_bytes()));
-    CU_TRY(ctx, skinny_ws_init(pl->sk_ws, false));
+    const size_t ws_bytes = skinny_ws_bytes(M, ctx->sm_count);
+    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_ws), ws_bytes));
+    CU_TRY(ctx, skinny_ws_init(pl->sk_ws, ws_bytes, false));
     size_t img = 0;
     for (const Group &g : groups) {
         size_t sum = 0;
@@ -661,7 +664,7 @@ b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job 
         const Group &g = groups[gi];
         SkinnyBuffers buf{};
         buf.ws = pl->sk_ws;
-        buf.ws_bytes = skinny_ws_bytes();
+        buf.ws_bytes = ws_bytes;
         buf.img = pl->sk_img;
         buf.img_bytes = img;
         buf.jobs_dev = pl->sk_jobs + gi * skinny_job_table_bytes();
@@ -842,7 +845,7 @@ b200q_status b200q_sync(b200q_ctx *ctx, void *stream, uint64_t timeout_ms) {
     if (status != DEV_OK) {
         cudaMemset(ctx->status_dev, 0, sizeof(int));
         for (Scratch *sc : {&ctx->scratch, &ctx->hscratch})      // a later call must find the shared tiles' sums at zero
-            if (sc->sk_ws) CU_TRY(ctx, skinny_ws_init(sc->sk_ws, true));
+            if (sc->sk_ws) CU_TRY(ctx, skinny_ws_init(sc->sk_ws, ctx_ws_bytes(ctx), true));
         if (ctx->peer_world > 1) ctx->peer_stale = true;     // some rank may have skipped an exchange: counters disagree
         return fail(ctx, B200Q_ERR_TIMEOUT, "a kernel gave up a bounded wait (device status %d); results are invalid", status);
     }

@@ -117,8 +117,8 @@ struct SkinnyBuffers {
 int skinny_max_m();          // the largest M of the exact route
 int skinny_max_mid_m();      // the largest M the kernels take
 int skinny_max_products();
-size_t skinny_ws_bytes();
-cudaError_t skinny_ws_init(uint8_t *ws, bool own_stream);
+size_t skinny_ws_bytes(int M, int sm_count);      // grows with M: what serves 48 rows serves fewer, too
+cudaError_t skinny_ws_init(uint8_t *ws, size_t bytes, bool own_stream);
 size_t skinny_image_bytes(const SkinnyProduct &a);
 size_t skinny_job_table_bytes();
 // at most four products (their descriptions travel in the kernel parameters): prepare, launch, forget

@@ -53,16 +53,18 @@ int token_tiles(int M) {
 int skinny_max_m() { return 16; }
 int skinny_max_mid_m() { return 48; }
 
-// sums of one shared tile per block (192 rows x 48 tokens is the largest), and their counts
-static constexpr size_t kSkSumBytes = size_t(kSkMaxGrid) * 192 * 48 * sizeof(double);
+// Counts of the shared tiles, then their sums: one tile per block, as wide as M asks for (2.4 MB per eight tokens)
 static constexpr size_t kSkCountBytes = size_t(kSkMaxGrid) * sk_warps(1) * sizeof(unsigned);
-size_t skinny_ws_bytes() { return kSkSumBytes + kSkCountBytes; }
+size_t skinny_ws_bytes(int M, int sm_count) {
+    const int nt = token_tiles(M);
+    return kSkCountBytes + (size_t)std::min(sm_count, kSkMaxGrid) * sk_tile_rows(nt) * 8 * nt * sizeof(double);
+}
 // Zeroes before it returns, on the legacy stream or on one of its own, which waits for no other.
-cudaError_t skinny_ws_init(uint8_t *ws, bool own_stream) {
+cudaError_t skinny_ws_init(uint8_t *ws, size_t bytes, bool own_stream) {
     cudaStream_t st = nullptr;
     cudaError_t e = own_stream ? cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) : cudaSuccess;
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(ws, 0, skinny_ws_bytes(), st);
+    e = cudaMemsetAsync(ws, 0, bytes, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (own_stream) cudaStreamDestroy(st);
     return e;
@@ -82,7 +84,7 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
     if (n < 1 || n > kSkMaxJobs || !prods) return cudaErrorInvalidValue;
     const int M = prods[0].M, qt = prods[0].qt;
     const bool f32 = !prods[0].x_is_bf16;
-    if (M < 1 || M > skinny_max_mid_m() || buf.ws_bytes < skinny_ws_bytes()) return cudaErrorInvalidValue;
+    if (M < 1 || M > skinny_max_mid_m() || buf.ws_bytes < skinny_ws_bytes(M, buf.sm_count)) return cudaErrorInvalidValue;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
     set->qt = qt;
@@ -144,8 +146,8 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
         if (e != cudaSuccess) return e;
         p.jobs = reinterpret_cast<const SkJob *>(buf.jobs_dev);
     }
-    p.sums = reinterpret_cast<double *>(buf.ws);
-    p.count = reinterpret_cast<unsigned *>(buf.ws + kSkSumBytes);
+    p.count = reinterpret_cast<unsigned *>(buf.ws);
+    p.sums = reinterpret_cast<double *>(buf.ws + kSkCountBytes);
     p.status = buf.status;
     p.njobs = n;
     p.slots = slots;

@@ -200,3 +200,37 @@ def test_capture_without_the_workspaces(orc):
         _check(y, x[:32], rows, index, 2e-3)
     del graph
     be.close()
+
+
+# A plan owns its workspaces, 2.4 MB of sums per eight tokens (the driver hands out steps of 2 MB): they stay small beside a model's weights, also for an engine with two plans per layer
+@pytest.mark.parametrize("m,limit_mb", [(4, 5), (16, 8)])
+def test_memory_of_a_plan(backend, orc, m, limit_mb):
+    w, _, _ = _weights(orc, backend, mb.TYPE_Q4_K, 512, 4096, 1)
+    x = torch.zeros((m, 4096), dtype=torch.bfloat16, device="cuda")
+    y = torch.empty((m, 512), device="cuda")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    plans = [backend.plan([([w], x, [y])]) for _ in range(32)]
+    used = (before - torch.cuda.mem_get_info()[0]) / 32 / 2**20
+    for p in plans:
+        p.close()
+    assert used < limit_mb, f"{used:.1f} MB a plan"
+
+
+# Plans share no state, so two of them may run at the same time
+def test_two_plans_on_two_streams(backend, orc):
+    made = []
+    for seed, (qt, n, k, m) in enumerate([(mb.TYPE_Q4_K, 1300, 4096, 5), (mb.TYPE_Q6_K, 700, 8192, 12)]):
+        ws = [_weights(orc, backend, qt, n + i, k, seed + i) for i in range(5)]
+        x = torch.from_numpy(np.random.default_rng(seed).standard_normal((m, k), dtype=np.float32)).cuda().to(torch.bfloat16)
+        ys = [torch.empty((m, w.n), device="cuda") for w, _, _ in ws]
+        made.append((backend.plan([([w], x, [y]) for (w, _, _), y in zip(ws, ys)]), torch.cuda.Stream(), ws, x, ys))
+    torch.cuda.synchronize()
+    for _ in range(30):
+        for plan, stream, _, _, _ in made:
+            plan.run(stream=stream)
+    for plan, stream, ws, x, ys in made:
+        backend.sync(stream)
+        for y, (_, rows, index) in zip(ys, ws):
+            _check(y, x, rows, index, 1e-4)
+        plan.close()
