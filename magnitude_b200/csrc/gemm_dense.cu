@@ -117,13 +117,14 @@ struct DenseParams {
     int stages, stage_bytes; // operand ring: 128 weight rows and bn / 2 tokens per stage and CTA
     int m_tiles, tiles;
     // The last round would leave pairs idle: the tiles from `whole` on (of bn tokens) are cut into `split`
-    // tiles of `bn2` tokens each.
+    // tiles of `bn2` tokens each, the last of them what is left of bn.
     int whole, split, bn2;
     int *status;
 };
 
 struct DenseTile {
     int stripe, t0, width;   // 256-row stripe, first token, tokens
+    int box;                 // tokens that the two activation loads bring: width or more
 };
 __device__ __forceinline__ DenseTile dense_tile(const DenseParams &p, int tile) {
     int sub = 0, w = p.bn;
@@ -136,7 +137,8 @@ __device__ __forceinline__ DenseTile dense_tile(const DenseParams &p, int tile) 
     DenseTile t;
     t.stripe = tile / p.m_tiles;
     t.t0 = (tile - t.stripe * p.m_tiles) * p.bn + sub * w;
-    t.width = w;
+    t.width = min(w, p.bn - sub * w);
+    t.box = w;
     return t;
 }
 
@@ -215,9 +217,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const DensePara
             bool ok = true;
             for (int tile = pair; tile < p.tiles && ok; tile += n_pairs) {
                 const DenseTile t = dense_tile(p, tile);
-                const int half = t.width >> 1;
-                const int arow = t.stripe * kStripe + (int)rank * kRows, brow = t.t0 + (int)rank * half;
-                const uint32_t bytes_pair = 2u * (kABytes + (uint32_t)half * kBK * 2);
+                const int arow = t.stripe * kStripe + (int)rank * kRows, brow = t.t0 + (int)rank * (t.width >> 1);
+                const uint32_t bytes_pair = 2u * (kABytes + (uint32_t)(t.box >> 1) * kBK * 2);
                 const CUtensorMap *bm = tile < p.whole ? &bmap : &bmap2;
                 for (int ks = 0; ks < p.ksteps; ++ks) {
                     ok = dense_wait(empty_s + 8 * stage, phase, sm, p.status);

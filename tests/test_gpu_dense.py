@@ -52,9 +52,10 @@ def _all(pair, qt, shapes, k, x, dtype):
         assert torch.equal(a, b) and torch.equal(a, c)
 
 
-# edges of the 256-row stripes, the 32-token widths and the 8-record chunks
+# edges of the 256-row stripes, the 32-token widths and the 8-record chunks; 512 tokens of 2560 rows: a last round of 20
+# tiles of 256 tokens, cut into three of 96, 96 and 64
 @pytest.mark.parametrize("qt", TYPES)
-@pytest.mark.parametrize("m,shapes,k", [(128, [256], 256), (129, [257], 2304), (255, [511, 4, 130], 2048), (513, [1000], 4352), (333, [2051, 260], 1280)])
+@pytest.mark.parametrize("m,shapes,k", [(128, [256], 256), (129, [257], 2304), (255, [511, 4, 130], 2048), (513, [1000], 4352), (512, [2560], 1024), (333, [2051, 260], 1280)])
 def test_same_bits(pair, qt, m, shapes, k):
     x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32)).cuda()
     _all(pair, qt, shapes, k, x.to(torch.bfloat16), torch.float32)
