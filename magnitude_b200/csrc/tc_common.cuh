@@ -406,12 +406,16 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 // Activations -> fp16, the format the weights are dequantized to (both tensor-core operands must
 // share one format), rounding to nearest even.  fp16 has three more mantissa bits than bf16 but a
 // narrower exponent: bf16 values between 2^-14 and 65504 in magnitude convert exactly, larger ones
-// saturate to +-65504, smaller ones lose bits as fp16 subnormals or flush to zero (below 2^-25).
+// (infinities too) saturate to +-65504, smaller ones lose bits as fp16 subnormals or flush to zero (below 2^-25).
+// NaN stays NaN (fminf and fmaxf would return the bound).
 __device__ __forceinline__ uint32_t to_h2_sat(float lo, float hi) {
-    lo = fminf(fmaxf(lo, -65504.f), 65504.f);   // NaN passes through both
-    hi = fminf(fmaxf(hi, -65504.f), 65504.f);
     uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    asm("{\n\t.reg .f32 a, b;\n\t"
+        "max.NaN.f32 a, %1, %3;\n\tmin.NaN.f32 a, a, %4;\n\t"
+        "max.NaN.f32 b, %2, %3;\n\tmin.NaN.f32 b, b, %4;\n\t"
+        "cvt.rn.f16x2.f32 %0, a, b;\n\t}"
+        : "=r"(r)
+        : "f"(hi), "f"(lo), "f"(-65504.f), "f"(65504.f));
     return r;
 }
 

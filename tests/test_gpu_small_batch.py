@@ -234,3 +234,19 @@ def test_two_plans_on_two_streams(backend, orc):
         for y, (_, rows, index) in zip(ys, ws):
             _check(y, x, rows, index, 1e-4)
         plan.close()
+
+
+# A NaN must not come out as a number, whichever kernel takes the call: single weights and sets, 17 rows and more
+@pytest.mark.parametrize("m,n", [(20, [300]), (32, [300]), (32, [300, 200]), (64, [300]), (150, [300]), (150, [40000])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_nan_stays_nan_in_larger_batches(backend, orc, m, n, dtype):
+    k = 1024
+    ws = [_weights(orc, backend, mb.TYPE_Q4_K, i, k, i) for i in n]
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32)).cuda().to(dtype)
+    x[5, 77] = float("nan")
+    ys = backend.project_multi([w for w, _, _ in ws], x)
+    backend.sync()
+    keep = [i for i in range(m) if i != 5]
+    for y, (_, rows, index) in zip(ys, ws):
+        assert torch.isnan(y[5]).all()
+        _check(y[keep], x[keep], rows, index, 2e-3)
