@@ -152,14 +152,18 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
     p.njobs = n;
     p.slots = slots;
     int grid = std::min(std::min(buf.sm_count, kSkMaxGrid), slots);
-    // A whole number of blocks per tile where that leaves no block with more slots: then no block has two tiles to share
+    // A whole number of blocks per tile where that leaves no block with more slots: then no block has two tiles to share.  As
+    // few of them as the longest run allows (us a call, 4096 x 14336 Q6_K, 8 rows: 9 blocks of 6 or 7 slots a tile 23.1, 8 of 7 22.5)
     int tiles = 0, nsb = jobs[0].nsb;
     for (int i = 0; i < n; ++i) {
         tiles += jobs[i].tiles;
         if (jobs[i].nsb != nsb) nsb = 0;
     }
     const int each = std::min(grid / tiles, nsb);
-    if (each > 0 && (nsb + each - 1) / each <= (slots + grid - 1) / grid) grid = tiles * each;
+    if (each > 0 && (nsb + each - 1) / each <= (slots + grid - 1) / grid) {
+        const int most = (nsb + each - 1) / each;
+        grid = tiles * ((nsb + most - 1) / most);
+    }
     set->grid = grid;
     // Few slots per block: each block makes the images of its own slots, in place, and the first launch falls away
     // (us a call, one launch / two: Q4_K 1024 x 4096, 8 rows 7.3 / 8.4, 16 rows 8.9 / 9.8).  With more slots, warps that

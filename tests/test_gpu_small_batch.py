@@ -250,3 +250,15 @@ def test_nan_stays_nan_in_larger_batches(backend, orc, m, n, dtype):
     for y, (_, rows, index) in zip(ys, ws):
         assert torch.isnan(y[5]).all()
         _check(y[keep], x[keep], rows, index, 2e-3)
+
+
+# 16 tiles of 56 records: 144 blocks could share them, 128 with seven records each are as quick
+@pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K])
+@pytest.mark.parametrize("m", [8, 16, 20])
+def test_equal_runs_of_records(backend, orc, qt, m):
+    w, rows, index = _weights(orc, backend, qt, 3841, 14336, m)
+    x = torch.from_numpy(np.random.default_rng(m).standard_normal((m, 14336), dtype=np.float32)).cuda().to(torch.bfloat16)
+    for _ in range(2):
+        y = backend.project(w, x)
+        backend.sync()
+        _check(y, x, rows, index, 1e-4 if m <= 16 else 2e-3)
