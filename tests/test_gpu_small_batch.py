@@ -252,6 +252,20 @@ def test_nan_stays_nan_in_larger_batches(backend, orc, m, n, dtype):
         _check(y[keep], x[keep], rows, index, 2e-3)
 
 
+# Jobs of one plan may read one activation buffer with different K (and so need images of their own)
+def test_plan_jobs_of_different_k_share_a_buffer(backend, orc):
+    x = torch.from_numpy(np.random.default_rng(1).standard_normal((9, 4096), dtype=np.float32)).cuda().to(torch.bfloat16)
+    ws = [_weights(orc, backend, mb.TYPE_Q8_0, n, k, n) for n, k in [(300, 4096), (257, 2048), (500, 4096), (193, 2304), (64, 2048)]]
+    ys = [torch.empty((9, w.n), device="cuda") for w, _, _ in ws]
+    plan = backend.plan([([w], x[:, :w.k], [y]) for (w, _, _), y in zip(ws, ys)])
+    for _ in range(2):
+        plan.run()
+    backend.sync()
+    for y, (w, rows, index) in zip(ys, ws):
+        _check(y, x[:, :w.k], rows, index, 1e-4)
+    plan.close()
+
+
 # 16 tiles of 56 records: 144 blocks could share them, 128 with seven records each are as quick
 @pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K])
 @pytest.mark.parametrize("m", [8, 16, 20])
