@@ -84,7 +84,8 @@ enum {
     B200Q_ROUTE_SKINNY = 2, /* 3 <= M <= 16: streaming kernel, exact integer weights x exact bf16 activations in
                                mma.sync with fp32 accumulation */
     B200Q_ROUTE_GEMM = 3    /* larger M: activations converted to fp16, weights to fp16 or fp16-exact integers, fp32
-                               accumulation; mma.sync up to 48 rows, then tcgen05 / TMEM */
+                               accumulation; tcgen05 / TMEM, or mma.sync for sets of weights up to 48 rows and single
+                               ones up to 20 (tall ones up to 32).  |x| > 65504 may saturate */
 };
 
 /* Per-context settings (b200q_ctx_set_option). */
@@ -260,8 +261,9 @@ b200q_status b200q_matmul(b200q_ctx *ctx, const b200q_weight *w, const void *x_d
                           void *stream);
 
 /* Several weights of the same type and K applied to one activation in a single launch
- * (gate+up, or Q+K sharing x): Y_i[M][N_i] = X . W_i^T.  n_weights <= 4.  Falls back to one
- * launch per weight for M > 4. */
+ * (gate+up, or Q+K sharing x): Y_i[M][N_i] = X . W_i^T.  n_weights <= 4.  Up to 48
+ * rows, and from 128 on where the weights are copied to fp16 first, one launch covers all weights (a
+ * second one prepares operands); else there is one per weight. */
 b200q_status b200q_matmul_multi(b200q_ctx *ctx, const b200q_weight *const *w, int32_t n_weights,
                                 const void *x_dev, int32_t x_dtype, int64_t M, int64_t ldx,
                                 void *const *y_dev, int32_t y_dtype, const int64_t *ldy, void *stream);

@@ -322,7 +322,7 @@ b200q_status ensure_gemm_scratch(b200q_ctx *ctx, Scratch &sc, int64_t M, int64_t
 }
 
 // Workspace for the fp16 weights of the two-launch GEMM: a fixed size from the first use on (only a K above
-// 262144 asks for more), so that a later call with larger weights allocates nothing.  False where it
+// 524288 asks for more), so that a later call with larger weights allocates nothing.  False where it
 // cannot be had (no memory, or the stream is being captured): the one-launch kernels take the call.
 bool ensure_dense_scratch(Scratch &sc, int64_t Kpad, cudaStream_t st) {
     const size_t need = std::max(kDenseScratchBytes, (size_t)Kpad * 2 * 256);
@@ -503,9 +503,13 @@ b200q_status validate_mm(b200q_ctx *ctx, const b200q_weight *w, const void *x, i
 }
 
 // 17..48 rows: the small-batch kernel runs all weights of a call in one launch, the one-CTA GEMM one after another, each
-// with few K ranges per SM.  us, small-batch / GEMM: Q4_K 4096 + 1024 rows of K = 4096, 17 tokens 18 / 27, 48 tokens 28 / 29;
-// 2 x 14336, 48 tokens 55 / 71; 2 x 25600 rows of K = 5120, 48 tokens 100 / 149.  A single weight: 14336 x 4096, 32 tokens
-// 30 / 35, 48 tokens 40 / 37; 4096 x 4096, 17 tokens 15.7 / 16.5, 32 tokens 18.5 / 16.5.
+// with few K ranges per SM, a conversion before them and a sum of K ranges after each.  Sets of weights, us a call in a loop
+// of calls (launches included), small-batch / GEMM, at 17 and 48 rows (2 x 14336 x 4096; the smallest lead there is at 48 rows:
+// 2 x 8192 x 8192):
+//   Q4_K 42 / 72, 55 / 76; 60 / 86     Q5_K 46 / 79, 61 / 83; 68 / 90      Q6_K 47 / 79, 58 / 83; 63 / 91
+//   Q8_0 46 / 75, 59 / 79; 63 / 88     Q4_0 44 / 74, 63 / 78; 68 / 86      MXFP4 50 / 74, 64 / 79; 72 / 86
+// and 2 x 512 rows of K = 4096, any type: 11 / 31, 16 / 33.  A single weight, Q4_K, device time: 14336 x 4096, 32 rows 30 / 35,
+// 48 rows 40 / 37; 4096 x 4096, 17 rows 15.7 / 16.5, 32 rows 18.5 / 16.5.
 bool mid_pays(const b200q_ctx *ctx, const b200q_weight *const *w, int nw, int M) {
     int weights = 0;
     int64_t slots = 0;
@@ -556,7 +560,7 @@ b200q_status matmul_any(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *
         ctx->last_route = B200Q_ROUTE_SKINNY;
         return run_skinny(ctx, sc, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
     }
-    if (M > mt) {   // prefill / verify batches: tensor cores, one launch per weight
+    if (M > mt) {   // prefill / verify batches: tensor cores
         ctx->last_route = B200Q_ROUTE_GEMM;
         if (M > skinny_max_m() && M <= ctx->mid_max_m && mid_pays(ctx, w, nw, (int)M) && mid_scratch(ctx, sc, w[0], x_dtype, (int)M, st))
             return run_skinny(ctx, sc, w, nw, x, x_dtype, (int)M, ldx, y, y_dtype, ldy, st);
@@ -605,7 +609,7 @@ b200q_status ensure_host_path(b200q_ctx *ctx, size_t xb, size_t yb) {
 
 // A plan on the skinny route (3..16 activation rows by default): consecutive products of one block type form a group that one
 // skinny launch runs (a job that reads what earlier jobs wrote starts a new group, so stream order
-// provides the dependency); the plan owns the groups' images, chunk sums, counters and job tables.
+// provides the dependency); the plan owns their images, the sums and counts of shared tiles and the job tables.
 b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job *jobs, int n_jobs, int M) {
     struct Group { std::vector<SkinnyProduct> prods; };
     std::vector<Group> groups;

@@ -181,11 +181,9 @@ struct DenseLaunch {
     int sm_count;
     int bn_override;                      // 0 = choose the token tile
 };
-// 256 MB: all projections of an 8B-class model in one panel; with 128 MB the gate and up matrices of such a
+// 256 MB: every projection of an 8B-class layer in one panel; with 128 MB the gate and up matrices of such a
 // layer took two, each with a partial last round (28672 x 4096, 512 rows: 165 us against 143)
 constexpr size_t kDenseScratchBytes = size_t(256) << 20;
-// 256 MB: all projections of an 8B-class model in one panel; with 128 MB the gate and up matrices of such a
-// layer took two, each with a partial last round (28672 x 4096, 512 rows: 165 us against 143)
 bool dense_pays(const DenseLaunch &a);    // worth two launches? (sizes only; scratch and pointers not needed)
 cudaError_t dense_gemm_run(const DenseLaunch &a, cudaStream_t st, int *launches);
 
