@@ -142,7 +142,6 @@ struct b200q_plan {
     std::vector<SkinnySet *> sets;
     uint8_t *sk_ws = nullptr;
     uint8_t *sk_img = nullptr;
-    uint8_t *sk_jobs = nullptr;
 };
 
 struct b200q_weight {
@@ -481,7 +480,6 @@ b200q_status run_skinny(b200q_ctx *ctx, Scratch &sc, const b200q_weight *const *
     buf.ws_bytes = ctx_ws_bytes(ctx);
     buf.img = sc.sk_img;
     buf.img_bytes = sc.sk_img_bytes;
-    buf.jobs_dev = nullptr;      // at most four products: their descriptions travel in the kernel parameters
     buf.status = ctx->status_dev;
     buf.sm_count = ctx->sm_count;
     cudaError_t e = skinny_run(prods, n, buf, st, &ctx->last_launches);
@@ -609,7 +607,7 @@ b200q_status ensure_host_path(b200q_ctx *ctx, size_t xb, size_t yb) {
 
 // A plan on the skinny route (3..16 activation rows by default): consecutive products of one block type form a group that one
 // skinny launch runs (a job that reads what earlier jobs wrote starts a new group, so stream order
-// provides the dependency); the plan owns their images, the sums and counts of shared tiles and the job tables.
+// provides the dependency); the plan owns their images and the sums and counts of shared tiles.
 b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job *jobs, int n_jobs, int M) {
     struct Group { std::vector<SkinnyProduct> prods; };
     std::vector<Group> groups;
@@ -663,15 +661,12 @@ b200q_status plan_create_skinny(b200q_ctx *ctx, b200q_plan *pl, const b200q_job 
         img = std::max(img, sum);
     }
     CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_img), img));
-    CU_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->sk_jobs), groups.size() * skinny_job_table_bytes()));
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const Group &g = groups[gi];
+    for (const Group &g : groups) {
         SkinnyBuffers buf{};
         buf.ws = pl->sk_ws;
         buf.ws_bytes = ws_bytes;
         buf.img = pl->sk_img;
         buf.img_bytes = img;
-        buf.jobs_dev = pl->sk_jobs + gi * skinny_job_table_bytes();
         buf.status = ctx->status_dev;
         buf.sm_count = ctx->sm_count;
         SkinnySet *set = nullptr;
@@ -1247,7 +1242,6 @@ void b200q_plan_destroy(b200q_plan *plan) {
     for (SkinnySet *set : plan->sets) skinny_set_destroy(set);
     if (plan->sk_ws) cudaFree(plan->sk_ws);
     if (plan->sk_img) cudaFree(plan->sk_img);
-    if (plan->sk_jobs) cudaFree(plan->sk_jobs);
     delete plan;
 }
 

@@ -110,7 +110,6 @@ struct SkinnyBuffers {
     size_t ws_bytes;
     uint8_t *img;            // activation images: skinny_image_bytes of every product of its own x.  Launches that follow
     size_t img_bytes;        // each other in a stream may share both
-    void *jobs_dev;          // skinny_job_table_bytes() of device memory for calls with more than one product
     int *status;
     int sm_count;
 };
@@ -120,11 +119,9 @@ int skinny_max_products();
 size_t skinny_ws_bytes(int M, int sm_count);      // grows with M: what serves 48 rows serves fewer, too
 cudaError_t skinny_ws_init(uint8_t *ws, size_t bytes, bool own_stream);
 size_t skinny_image_bytes(const SkinnyProduct &a);
-size_t skinny_job_table_bytes();
-// at most four products (their descriptions travel in the kernel parameters): prepare, launch, forget
+// at most four products: prepare, launch, forget
 cudaError_t skinny_run(const SkinnyProduct *prods, int n, const SkinnyBuffers &buf, cudaStream_t st, int *launches);
-// up to skinny_max_products() products prepared once and launched many times (plans): buf.jobs_dev,
-// and buf.ws stay owned by the caller and must outlive the set
+// up to skinny_max_products() products prepared once and launched many times (plans); buf's memory must outlive the set
 struct SkinnySet;
 cudaError_t skinny_set_create(const SkinnyProduct *prods, int n, const SkinnyBuffers &buf, SkinnySet **out);
 cudaError_t skinny_set_launch(const SkinnySet *set, cudaStream_t st);

@@ -2,7 +2,6 @@
 // operand fragments.
 #include <algorithm>
 #include <new>
-#include <vector>
 
 #include "kernels.h"
 #include "skinny_image.cuh"
@@ -19,11 +18,11 @@ SK_TYPES(SK_DECLARE)
 namespace {
 
 // One warp per (product, record, token).
-template <int MAP> __global__ void __launch_bounds__(128) skinny_prep_kernel(const __grid_constant__ SkParams p) {
+template <int MAP, int N> __global__ void __launch_bounds__(128) skinny_prep_kernel(const __grid_constant__ SkParamsOf<N> p) {
     pdl_launch_dependents();
     const int wid = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (wid >= p.xwarps) return;
-    const SkJob *jobs = p.jobs ? p.jobs : p.inl;
+    const SkJob *jobs = p.jobs;
     int ji = p.njobs - 1;
     while (jobs[ji].xwarp0 > wid || jobs[ji].xwarp0 < 0) --ji;
     const SkJob &J = jobs[ji];
@@ -94,9 +93,7 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
     p.xwarps = 0;
     const int rows = sk_tile_rows(p.NT), rec4 = rec_bytes(qt) / 4;
     size_t img_off = 0;
-    std::vector<SkJob> table;
-    if (n > kSkInline) table.resize((size_t)n);
-    SkJob *jobs = n > kSkInline ? table.data() : p.inl;
+    SkJob *jobs = p.jobs;
     int slots = 0;
     for (int i = 0; i < n; ++i) {
         const SkinnyProduct &a = prods[i];
@@ -137,14 +134,6 @@ static cudaError_t set_fill(SkinnySet *set, const SkinnyProduct *prods, int n, c
         if (ok && qt == QT_Q6_K && whole) ok = sk_encode(enc, &J.d, a.w, qt, J.nsb, groups, 0, J.nfull, 4, rows);
         if (ok && qt == QT_Q6_K && tail) ok = sk_encode(enc, &J.dtail, a.w, qt, J.nsb, groups, J.nfull, 1, 4, rows);
         if (!ok) return cudaErrorInvalidValue;
-    }
-    p.jobs = nullptr;
-    if (n > kSkInline) {
-        if (!buf.jobs_dev) return cudaErrorInvalidValue;
-        cudaError_t e = cudaMemcpy(buf.jobs_dev, jobs, sizeof(SkJob) * (size_t)n, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);     // a copy from pageable memory may return before it has arrived
-        if (e != cudaSuccess) return e;
-        p.jobs = reinterpret_cast<const SkJob *>(buf.jobs_dev);
     }
     p.count = reinterpret_cast<unsigned *>(buf.ws);
     p.sums = reinterpret_cast<double *>(buf.ws + kSkCountBytes);
@@ -188,7 +177,7 @@ cudaError_t skinny_set_create(const SkinnyProduct *prods, int n, const SkinnyBuf
 
 void skinny_set_destroy(SkinnySet *set) { delete set; }
 
-static cudaError_t launch_prep(const SkinnySet *set, cudaStream_t st) {
+template <int MAP, int N> static cudaError_t launch_prep_t(const SkinnySet *set, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)((set->p.xwarps + 3) / 4));
     cfg.blockDim = dim3(128);
@@ -198,17 +187,22 @@ static cudaError_t launch_prep(const SkinnySet *set, cudaStream_t st) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    void *args[] = {const_cast<SkParams *>(&set->p)};            // its first N jobs
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(&skinny_prep_kernel<MAP, N>), args);
+}
+
+template <int N> static cudaError_t launch_prep(const SkinnySet *set, cudaStream_t st) {
     switch (sk_map(set->qt)) {
-    case SK_K: return cudaLaunchKernelEx(&cfg, skinny_prep_kernel<SK_K>, set->p);
-    case SK_Q6: return cudaLaunchKernelEx(&cfg, skinny_prep_kernel<SK_Q6>, set->p);
-    default: return cudaLaunchKernelEx(&cfg, skinny_prep_kernel<SK_BLOCK>, set->p);
+    case SK_K: return launch_prep_t<SK_K, N>(set, st);
+    case SK_Q6: return launch_prep_t<SK_Q6, N>(set, st);
+    default: return launch_prep_t<SK_BLOCK, N>(set, st);
     }
 }
 
 // The images (unless the blocks make their own), then the products; both with programmatic stream serialization.
 cudaError_t skinny_set_launch(const SkinnySet *set, cudaStream_t st) {
     if (!set) return cudaErrorInvalidValue;
-    cudaError_t e = set->p.direct ? cudaSuccess : launch_prep(set, st);
+    cudaError_t e = set->p.direct ? cudaSuccess : set->p.njobs > kSkInline ? launch_prep<kSkMaxJobs>(set, st) : launch_prep<kSkInline>(set, st);
     if (e != cudaSuccess) return e;
     switch (set->qt) {
 #define SK_LAUNCH(NAME, QT) \
@@ -221,7 +215,7 @@ cudaError_t skinny_set_launch(const SkinnySet *set, cudaStream_t st) {
 int skinny_set_launches(const SkinnySet *set) { return set ? (set->p.direct ? 1 : 2) : 0; }
 
 cudaError_t skinny_run(const SkinnyProduct *prods, int n, const SkinnyBuffers &buf, cudaStream_t st, int *launches) {
-    if (n > kSkInline) return cudaErrorInvalidValue;     // larger sets go through a plan, whose job table is uploaded once
+    if (n > kSkInline) return cudaErrorInvalidValue;     // larger sets go through a plan
     SkinnySet set;
     cudaError_t e = set_fill(&set, prods, n, buf);
     if (e != cudaSuccess) return e;
@@ -230,7 +224,6 @@ cudaError_t skinny_run(const SkinnyProduct *prods, int n, const SkinnyBuffers &b
     return e;
 }
 
-size_t skinny_job_table_bytes() { return sizeof(SkJob) * kSkMaxJobs; }
 int skinny_max_products() { return kSkMaxJobs; }
 
 cudaError_t skinny_set_wait_limit_ns(unsigned long long ns) {

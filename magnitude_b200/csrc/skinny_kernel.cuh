@@ -401,7 +401,7 @@ __device__ __forceinline__ bool sk_wait(uint32_t bar, uint32_t parity, volatile 
     return false;
 }
 
-// (product, tile, record) of a slot, stepped without dividing and without reading the table (a plan's lies in global memory)
+// (product, tile, record) of a slot, stepped without dividing and without reading the table
 struct SkCursor {
     int ji, tile, rec, nsb, tiles;
     __device__ __forceinline__ void start(const SkJob *jobs, int njobs, int slot) {
@@ -428,30 +428,22 @@ __device__ __forceinline__ void sk_tma_4d(uint32_t dst, const CUtensorMap *map, 
         : "memory");
 }
 
-// A tensor map in global memory is read through a proxy of its own: without this the copy engine may use what it still
-// holds of an older map at the same address (the table of a plan destroyed before).  Maps in kernel parameters need none.
-// A kernel that merely contains it starts later (4096 x 14336 Q6_K, 8 rows, maps in the parameters: 22.6 us a call against
-// 22.0), so launches with a table are a form of their own.
-__device__ __forceinline__ void sk_map_acquire(const CUtensorMap *map) {
-    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
-}
-
 __device__ __forceinline__ void sk_store_y(const SkJob &J, int n, int m, float v) {
     if (n >= J.N || m >= J.M) return;
     const long long at = (long long)m * J.ldy + n;
     if (J.y_is_bf16) reinterpret_cast<__nv_bfloat16 *>(J.y)[at] = __float2bfloat16_rn(v);
     else reinterpret_cast<float *>(J.y)[at] = v;
 }
-// TABLE: the products' descriptions are in global memory (p.jobs), else in the parameters
-template <int QT, int NT, int P, bool TABLE>
-__global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel(const __grid_constant__ SkParams p) {
+// N: products the parameters have room for
+template <int QT, int NT, int P, int N>
+__global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel(const __grid_constant__ SkParamsOf<N> p) {
     using S = SkShape<QT, NT, P>;
     constexpr int kSkConsumers = S::kWarps, D = S::kDepth, REC = rec_bytes(QT);
     extern __shared__ __align__(128) uint8_t smem[];
     SkHead &head = *reinterpret_cast<SkHead *>(smem);
     const uint32_t full0 = smem_u32(head.full), empty0 = smem_u32(head.empty), ring0 = smem_u32(smem + S::kHead);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const SkJob *jobs = TABLE ? p.jobs : p.inl;
+    const SkJob *jobs = p.jobs;
     const int begin = sk_slot_begin(p.slots, gridDim.x, blockIdx.x), end = sk_slot_begin(p.slots, gridDim.x, blockIdx.x + 1);
     volatile int *fail = &head.fail;
 
@@ -474,18 +466,6 @@ __global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel
 
     if (warp == kSkConsumers) {
         // ===== producer ======================================================================================
-        if constexpr (TABLE) {               // at most 32 products (kSkMaxJobs): a lane for each
-            const int ji = cur.ji + lane;
-            if (ji < p.njobs && jobs[ji].slot0 < end) {
-                const SkJob &J = jobs[ji];
-                const bool whole = J.nsb >= kChunkRecs, rest = J.nsb % kChunkRecs != 0;
-                if (whole) sk_map_acquire(&J.w);
-                if (rest) sk_map_acquire(&J.wtail);
-                if (QT == QT_Q6_K && whole) sk_map_acquire(&J.d);
-                if (QT == QT_Q6_K && rest) sk_map_acquire(&J.dtail);
-            }
-            __syncwarp();
-        }
         if (lane == 0) {
             auto fetch_w = [&](const SkCursor &at, int stg) {
                 const SkJob &J = jobs[at.ji];
@@ -626,9 +606,9 @@ __global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel
     }
 }
 
-template <int QT, int NT, int P, bool TABLE = false> cudaError_t sk_launch_t(const SkParams &p, int grid, cudaStream_t st) {
+template <int QT, int NT, int P, int N = kSkInline> cudaError_t sk_launch_t(const SkParams &p, int grid, cudaStream_t st) {
     using S = SkShape<QT, NT, P>;
-    auto kern = skinny_kernel<QT, NT, P, TABLE>;
+    auto kern = skinny_kernel<QT, NT, P, N>;
     constexpr size_t smem = S::kHead + size_t(S::kDepth) * S::kStage;
     static_assert(smem <= 232448, "shared-memory plan exceeds the 227 KB a block may use");
     static std::atomic<int> configured_dev{-1};     // contexts on several threads may launch at once
@@ -649,16 +629,17 @@ template <int QT, int NT, int P, bool TABLE = false> cudaError_t sk_launch_t(con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    void *args[] = {const_cast<SkParams *>(&p)};     // its first N jobs
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(kern), args);
 }
 
 template <int QT> cudaError_t sk_launch_type(const SkParams &p, int NT, int P, int grid, cudaStream_t st) {
-    if (p.jobs) {                            // plans, of up to 16 rows
+    if (p.njobs > kSkInline) {               // plans, of up to 16 rows
         switch (NT * 4 + P) {
-        case 1 * 4 + 1: return sk_launch_t<QT, 1, 1, true>(p, grid, st);
-        case 1 * 4 + 2: return sk_launch_t<QT, 1, 2, true>(p, grid, st);
-        case 2 * 4 + 1: return sk_launch_t<QT, 2, 1, true>(p, grid, st);
-        case 2 * 4 + 2: return sk_launch_t<QT, 2, 2, true>(p, grid, st);
+        case 1 * 4 + 1: return sk_launch_t<QT, 1, 1, kSkMaxJobs>(p, grid, st);
+        case 1 * 4 + 2: return sk_launch_t<QT, 1, 2, kSkMaxJobs>(p, grid, st);
+        case 2 * 4 + 1: return sk_launch_t<QT, 2, 1, kSkMaxJobs>(p, grid, st);
+        case 2 * 4 + 2: return sk_launch_t<QT, 2, 2, kSkMaxJobs>(p, grid, st);
         default: return cudaErrorInvalidValue;
         }
     }

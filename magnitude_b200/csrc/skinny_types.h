@@ -1,6 +1,8 @@
 // What the host side of the small-batch route (skinny.cu) and its kernels (skinny_kernel.cuh) share.
 #pragma once
 
+#include <cstddef>
+
 #include <cuda.h>
 
 #include "common.cuh"
@@ -43,18 +45,23 @@ struct SkJob {
     int xwarp0;                        // first warp of the preparation that works on this job (none if the image is another job's)
 };
 constexpr int kSkMaxJobs = 32;
-constexpr int kSkInline = 4;           // products whose descriptions travel in the kernel parameters
+constexpr int kSkInline = 4;           // products of a call
 constexpr int kSkMaxGrid = 160;
 
-struct SkParams {
-    SkJob inl[kSkInline];
-    const SkJob *jobs;                 // device table, or null when the (at most kSkInline) jobs are in `inl`
+// Kernel parameters.  The products' descriptions travel in them, a plan's too (20 KB of the 32 that a launch may have): tensor maps
+// in global memory need a proxy fence before every use, which cost more (us, fence / parameters: sixteen Q4_K 6144 x 4096 products
+// as a plan, 4 rows 66.6 / 64.9; six Q6_K 4096 x 14336 calls, 8 rows 135.7 / 132.0), and an upload to wait for.
+template <int N> struct SkParamsOf {
     double *sums;                      // [grid][consumer warps][accumulators][32] sums of the tile that begins in a block and goes on
     unsigned *count;                   // [grid][consumer warps] parts of it seen so far; both zero between launches
     int *status;
     int njobs, slots;
     int direct;                        // 1: every block makes the images of its slots (at most sk_depth of them) itself
     int NT, P, xwarps;                 // token tiles, activation planes, warps of the preparation
+    SkJob jobs[N];
 };
+using SkParams = SkParamsOf<kSkMaxJobs>;
+using SkFew = SkParamsOf<kSkInline>;   // the same but for the jobs that are not there
+static_assert(sizeof(SkParams) <= 32764 && offsetof(SkFew, jobs) == offsetof(SkParams, jobs), "kernel parameters");
 
 }  // namespace b200q

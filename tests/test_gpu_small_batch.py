@@ -137,8 +137,8 @@ def test_host_calls_beside_device_calls(backend, orc, m, m_host):
         _check(torch.from_numpy(y).cuda(), torch.from_numpy(xh).cuda(), hrows, hindex, rel)
 
 
-# Plans of more than four products keep the tensor maps of their weights in device memory.  A plan made after another one was
-# destroyed may get the same address for other weights; run on a stream that is not ordered after the upload by itself.
+# A plan made after another one was destroyed may get the same addresses for other weights and images; run on a stream that is
+# not ordered after anything its creation uploads.
 @pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K])
 def test_plans_made_and_destroyed_in_turn(backend, orc, qt):
     stream = torch.cuda.Stream()
