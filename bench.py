@@ -668,7 +668,7 @@ def run_b200(args):
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
         "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "u8 x s16 integer block dots (dp4a), fp32 accumulate", "data": "synthetic",
+        "dtype": "u8 x s16 integer block dots (mma.sync s8), fp32 accumulate", "data": "synthetic",
         "config": workload_config(world), "roofline": roofline, "cpu_baseline": cpu_baseline, "e2e": e2e,
         # a plan run = the activation-prep launch + the streaming launch; the unfused TP mode adds the all-reduce kernel
         "gpu_launches": launches_per_step * ((2 if plans is not None else 1) + (1 if (use_peer and not fused) else 0)) * args.steps,
@@ -936,7 +936,7 @@ def run_skinny(args, emit=True):
                 algo = wbytes + m * k * 2 + m * n * 4
                 cases.append({"weight": name, "N": n, "K": k, "M": m, "us_per_product": us, "GB/s": algo / us / 1e3,
                               "frac_of_hbm_peak": algo / us / 1e3 / peak,
-                              "route": {mb.ROUTE_GEMV: "dp4a stream kernel", mb.ROUTE_SKINNY: "skinny kernel (mma.sync, exact bf16)",
+                              "route": {mb.ROUTE_GEMV: "stream kernel (integer mma.sync)", mb.ROUTE_SKINNY: "skinny kernel (mma.sync, exact bf16)",
                                         mb.ROUTE_GEMM: "tcgen05 GEMM, K split"}.get(route, str(route))})
                 tot_bytes += algo
                 tot_s += us * 1e-6
@@ -947,7 +947,7 @@ def run_skinny(args, emit=True):
     line = {
         "metric": "skinny_gemm_weight_bandwidth", "value": value, "unit": UNIT, "n_gpus": 1, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": tot_s * 1e3, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "M <= 2: u8 x s16 dp4a; M >= 3: exact integer weights x bf16 in mma.sync, fp32 accumulate", "data": "synthetic",
+        "dtype": "M <= 2: u8 x s16 integer mma.sync; M >= 3: exact integer weights x bf16 in mma.sync, fp32 accumulate", "data": "synthetic",
         "config": {"workload": "configs[2]: skinny verify batches, Q4_K 6144x4096 and Q6_K 4096x14336, M in {2,4,8,16}, bf16 tokens, fp32 out",
                    "l2": f"{copies} distinct weight copies per case", "parallelism": "single",
                    "form": "the 16 products of a case as one decode plan" if args.skinny_plan else "one product per call"},
@@ -1175,7 +1175,7 @@ def run_layer32b(args, emit=True):
         dist.barrier()
     line = {"metric": "layer32b_projection_throughput", "value": result["decode"]["value"], "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": 3, "ms_per_step": result["decode"]["ms_per_step"], "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-            "dtype": "decode: u8 x s16 dp4a; prefill: fp16 tcgen05.mma; fp32 accumulate", "data": "synthetic",
+            "dtype": "decode: u8 x s16 integer mma.sync; prefill: fp16 tcgen05.mma; fp32 accumulate", "data": "synthetic",
             "config": {"workload": "configs[4]: all projections of one decoder layer of a 32B-class dense model (Q4_K_M mix), M = 1 and M = 4096",
                        "layers_per_step": layers, "weight_bytes_per_layer": weight_bytes, "parallelism": f"tp{world}" if world > 1 else "single",
                        "l2": f"{layers} distinct copies of the layer per step ({layers * weight_bytes / world / 1e6:.0f} MB per rank)"},

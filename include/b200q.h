@@ -80,7 +80,7 @@ enum {
 /* Which kernel family b200q_matmul picked (b200q_last_route). */
 enum {
     B200Q_ROUTE_NONE = 0,
-    B200Q_ROUTE_GEMV = 1,   /* M <= 2 (up to 4 on request): dp4a streaming kernel on 16-bit fixed-point activations, HBM-bound */
+    B200Q_ROUTE_GEMV = 1,   /* M <= 2 (up to 4 on request): streaming kernel, integer tensor-core products with 16-bit fixed-point activations, HBM-bound */
     B200Q_ROUTE_SKINNY = 2, /* 3 <= M <= 16: streaming kernel, exact integer weights x exact bf16 activations in
                                mma.sync with fp32 accumulation */
     B200Q_ROUTE_GEMM = 3    /* larger M: activations converted to fp16, weights to fp16 or fp16-exact integers, fp32

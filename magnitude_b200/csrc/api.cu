@@ -120,7 +120,7 @@ struct b200q_ctx {
     int mid_max_m = 48;               // largest M that runs on the small-batch kernels (17 and more rows)
     int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1, gemm_dense = -1;
     // tunables (environment overrides for experiments)
-    int gemv_warps = 0, gemv_depth = 0, gemv_grid = 0, gemv_smem = 0, gemv_rows = 0, gemv_debug = 0, gemv_pdl = 1, gemv_teams = 2, gemv_xprep = 1, gemv_nap = 0;
+    int gemv_grid = 0, gemv_smem = 0, gemv_pdl = 1, gemv_xprep = 1;
     // tensor parallel
     NcclComm comm = nullptr;
     int tp_rank = 0, tp_world = 1;
@@ -135,6 +135,7 @@ struct b200q_plan {
     int device = 0;                   // the context's device, kept here: the plan may outlive the context
     std::vector<StreamJob> jobs;
     StreamJob *jobs_dev = nullptr;
+    unsigned *counter = nullptr;      // completion counter of plans whose jobs wait for one another
     uint8_t *xq_dev = nullptr;        // fixed-point activation images of the jobs (filled by the prep launch of every run)
     bool has_xq = false;
     int M = 0;
@@ -245,7 +246,13 @@ b200q_status check_ctx(b200q_ctx *ctx) {
     return B200Q_OK;
 }
 
-void fill_job(StreamJob &J, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int64_t ldx,
+int stream_grid(const b200q_ctx *ctx) { return ctx->gemv_grid > 0 ? ctx->gemv_grid : ctx->sm_count; }
+
+size_t stream_smem(const b200q_ctx *ctx) {
+    return (ctx->gemv_smem > 0 && (size_t)ctx->gemv_smem < ctx->smem_optin) ? (size_t)ctx->gemv_smem : ctx->smem_optin;
+}
+
+void fill_job(const b200q_ctx *ctx, StreamJob &J, const b200q_weight *const *w, int nw, const void *x, int x_dtype, int64_t ldx,
               void *const *y, int y_dtype, const int64_t *ldy, int flags) {
     J = StreamJob{};
     J.nseg = nw;
@@ -258,7 +265,6 @@ void fill_job(StreamJob &J, const b200q_weight *const *w, int nw, const void *x,
     J.qt = w[0]->type;
     J.K = (int)w[0]->K;
     J.Kpad = (int)w[0]->Kpad;
-    J.row_bytes = w[0]->row_bytes;
     J.x = x;
     J.ldx = ldx;
     J.x_is_bf16 = x_dtype == B200Q_TYPE_BF16;
@@ -266,12 +272,11 @@ void fill_job(StreamJob &J, const b200q_weight *const *w, int nw, const void *x,
     J.x_vec_ok = ((reinterpret_cast<uintptr_t>(x) & 15) == 0) && ((ldx * xelt) % 16 == 0);
     J.y_is_bf16 = y_dtype == B200Q_TYPE_BF16;
     J.flags = flags;
-    J.team = 0;
     J.xq = nullptr;
-    stream_job_finish(J);
+    stream_job_finish(J, stream_grid(ctx));
 }
 
-b200q_status run_stream(b200q_ctx *ctx, const StreamJob *jobs_host, const StreamJob *jobs_dev, int njobs, int M,
+b200q_status run_stream(b200q_ctx *ctx, const StreamJob *jobs_host, const StreamJob *jobs_dev, unsigned *counter, int njobs, int M,
                         cudaStream_t st) {
     StreamLaunch a{};
     a.jobs_host = jobs_host;
@@ -279,16 +284,11 @@ b200q_status run_stream(b200q_ctx *ctx, const StreamJob *jobs_host, const Stream
     a.njobs = njobs;
     a.M = M;
     a.status = ctx->status_dev;
-    a.counter = reinterpret_cast<unsigned *>(ctx->status_dev) + 16;   // its own 64-byte line
+    a.counter = counter;
     a.sm_count = ctx->sm_count;
-    a.smem_limit = (ctx->gemv_smem > 0 && (size_t)ctx->gemv_smem < ctx->smem_optin) ? (size_t)ctx->gemv_smem : ctx->smem_optin;
-    a.warps = ctx->gemv_warps;
-    a.depth = ctx->gemv_depth;
-    a.grid = ctx->gemv_grid;
-    a.debug = ctx->gemv_debug;
+    a.smem_limit = stream_smem(ctx);
+    a.grid = stream_grid(ctx);
     a.pdl = ctx->gemv_pdl;
-    a.teams = ctx->gemv_teams;
-    a.producer_nap = ctx->gemv_nap;
     a.peer_rank = ctx->peer_rank;
     a.peer_world = ctx->peer_world;
     for (int r = 0; r < kPeerMaxWorld; ++r) a.peer_base[r] = ctx->peer_base[r];
@@ -301,8 +301,9 @@ b200q_status run_gemv(b200q_ctx *ctx, const b200q_weight *const *w, int nw, cons
                       int M, int64_t ldx, void *const *y, int y_dtype, const int64_t *ldy,
                       cudaStream_t st) {
     StreamJob J;
-    fill_job(J, w, nw, x, x_dtype, ldx, y, y_dtype, ldy, 0);
-    return run_stream(ctx, &J, nullptr, 1, M, st);
+    fill_job(ctx, J, w, nw, x, x_dtype, ldx, y, y_dtype, ldy, 0);
+    stream_fit_jobs(&J, 1, M, stream_grid(ctx), stream_smem(ctx));
+    return run_stream(ctx, &J, nullptr, nullptr, 1, M, st);
 }
 
 // scratch for the fp16 copy of M activation rows
@@ -723,19 +724,13 @@ b200q_status b200q_ctx_create(int32_t device, b200q_ctx **out) {
         delete ctx;
         return e == cudaErrorMemoryAllocation ? B200Q_ERR_OVERLOADED : B200Q_ERR_BACKEND;
     }
-    ctx->gemv_warps = env_int("B200Q_GEMV_WARPS", 0);
-    ctx->gemv_depth = env_int("B200Q_GEMV_DEPTH", 0);
     ctx->gemv_grid = env_int("B200Q_GEMV_GRID", 0);
     ctx->gemv_smem = env_int("B200Q_GEMV_SMEM", 0);
-    ctx->gemv_rows = env_int("B200Q_GEMV_ROWS", 0);
 #ifdef B200Q_TIMING_EXPERIMENTS      // pipeline parts switched off for timing: results are invalid, never in a shipped build
-    ctx->gemv_debug = env_int("B200Q_GEMV_DEBUG", 0);
     ctx->gemm_debug = env_int("B200Q_GEMM_DEBUG", 0);
 #endif
     ctx->gemv_pdl = env_int("B200Q_GEMV_PDL", 1);
-    ctx->gemv_teams = env_int("B200Q_GEMV_TEAMS", 2);
     ctx->gemv_xprep = env_int("B200Q_GEMV_XPREP", 1);
-    ctx->gemv_nap = env_int("B200Q_GEMV_NAP", 0);
     ctx->gemm_bn = env_int("B200Q_GEMM_BN", 0);
     ctx->gemm_pair = env_int("B200Q_GEMM_PAIR", 1);
     ctx->mid_max_m = std::min(env_int("B200Q_MID_MAX", skinny_max_mid_m()), skinny_max_mid_m());
@@ -1157,7 +1152,7 @@ b200q_status b200q_plan_create(b200q_ctx *ctx, const b200q_job *jobs, int32_t n_
         if (glu) jflags |= STREAM_JOB_SWIGLU;
         if (j.flags & B200Q_JOB_ACCUMULATE) jflags |= STREAM_JOB_ACCUM;
         StreamJob J;
-        fill_job(J, j.w, j.n_weights, j.x_dev, j.x_dtype, j.ldx, j.y_dev, j.y_dtype, j.ldy, jflags);
+        fill_job(ctx, J, j.w, j.n_weights, j.x_dev, j.x_dtype, j.ldx, j.y_dev, j.y_dtype, j.ldy, jflags);
         if (j.norm_weight) {
             if (!(j.norm_eps >= 0.f) || (reinterpret_cast<uintptr_t>(j.norm_weight) & 3)) {
                 delete pl;
@@ -1187,10 +1182,13 @@ b200q_status b200q_plan_create(b200q_ctx *ctx, const b200q_job *jobs, int32_t n_
         }
     }
     if (!pl->jobs.empty()) {
-        stream_assign_teams(pl->jobs.data(), (int)pl->jobs.size());
-        const size_t bytes = pl->jobs.size() * sizeof(StreamJob);
-        cudaError_t e = cudaMalloc(&pl->jobs_dev, bytes);
+        stream_fit_jobs(pl->jobs.data(), (int)pl->jobs.size(), (int)M, stream_grid(ctx), stream_smem(ctx));
+        // the table, and behind it the plan's completion counter in a line of its own
+        const size_t bytes = pl->jobs.size() * sizeof(StreamJob), counter_at = (bytes + 127) & ~size_t(127);
+        cudaError_t e = cudaMalloc(&pl->jobs_dev, counter_at + 128);
+        if (e == cudaSuccess) e = cudaMemset(pl->jobs_dev, 0, counter_at + 128);
         if (e == cudaSuccess) e = cudaMemcpy(pl->jobs_dev, pl->jobs.data(), bytes, cudaMemcpyHostToDevice);
+        pl->counter = reinterpret_cast<unsigned *>(reinterpret_cast<uint8_t *>(pl->jobs_dev) + counter_at);
         if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) {
             if (pl->jobs_dev) cudaFree(pl->jobs_dev);
@@ -1227,7 +1225,7 @@ b200q_status b200q_plan_run(b200q_ctx *ctx, b200q_plan *plan, void *stream) {
         cudaError_t e = stream_xprep_launch(plan->jobs_dev, (int)plan->jobs.size(), plan->M, (cudaStream_t)stream);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "activation prep launch");
     }
-    s = run_stream(ctx, plan->jobs.data(), plan->jobs_dev, (int)plan->jobs.size(), plan->M, (cudaStream_t)stream);
+    s = run_stream(ctx, plan->jobs.data(), plan->jobs_dev, plan->counter, (int)plan->jobs.size(), plan->M, (cudaStream_t)stream);
     if (s != B200Q_OK) return s;
     ctx->last_route = B200Q_ROUTE_GEMV;
     ctx->last_launches = plan->has_xq ? 2 : 1;

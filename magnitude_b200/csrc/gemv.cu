@@ -1,29 +1,28 @@
-// Decode GEMV (M = 1) and M <= 4 product: the HBM-bound streaming kernel.
+// Decode GEMV (M = 1, 2; plans with fused epilogues up to M = 4): the HBM-bound streaming kernel.
 //
 // Y[m][n] = sum_k X[m][k] * dequant(W)[n][k]   for the streaming layout of common.cuh.
 //
 // One launch runs a list of projection jobs (one job for b200q_matmul, a whole decode step for a
 // plan) on persistent CTAs, one per SM, no CPU fallback, no cluster multicast:
-//   * CW consumer warps and one producer warp.  Every consumer warp owns a private ring of
-//     shared-memory slots; lane w of the producer warp keeps consumer w's ring full with 1-D
-//     bulk copies (cp.async.bulk, completion counted on a "full" mbarrier) and learns that a slot
-//     was consumed from an "empty" mbarrier.  A work item is one tile of the streaming layout
-//     (4 rows x 8 superblock records = 4 x 2048 weights), fetched with a single bulk copy.  The rings run on across job boundaries, so the weights of
-//     the next job stream in while the consumers still finish, reduce and store the current one:
-//     HBM reads never wait for a launch, a prologue or a grid-wide barrier.
-//   * per job each CTA owns a contiguous range of 4-row groups; items are dealt round-robin to
-//     the consumer warps and each item's result goes to its own shared-memory cell, so the final
-//     sum over K-chunks runs in a fixed order (bit-reproducible results).
-//   * the activation is converted once per CTA and job into a 16-bit fixed-point form in shared
-//     memory: per 32 weights one fp32 scale sx and per weight two signed bytes (x ~= sx * (256*hi
-//     + lo), lo in [-128, 127]; relative step 2^-15 of the block maximum).  The packed 4/6/8-bit
-//     weights multiply the two byte planes with dp4a, four weights per instruction, and block
-//     results are scaled and accumulated in fp32.
-//   * sub-block scales and mins are unpacked in registers; the min term of Q4_K and the -32
-//     offset of Q6_K use per-block integer sums of the activation computed in the prologue.
-//   * one lane handles one 64-weight unit of each of the item's 4 rows, so the activation bytes
-//     it loads are reused 4 times; a row's partial sums live in the lanes of one warp and are
-//     combined by warp shuffles.
+//   * sixteen consumer warps and four producer warps.  The producers keep a ring of slots in shared
+//     memory filled with 1-D bulk copies (cp.async.bulk, completion counted on a "full" mbarrier per
+//     slot).  A slot holds a quad: up to four tiles of the streaming layout, 16 rows x 8 superblock
+//     records (18 KB of Q4_K).  The slots run on across job boundaries: the weights of the next job
+//     stream in while the consumers still sum and store the current one or wait for other CTAs at a
+//     dependency.  HBM reads never wait for a launch, a conversion or a grid-wide meeting, up to the
+//     ring's size (about 150 KB, 3.5 us of one SM's share of the bandwidth).
+//   * up to four teams of four consumer warps take the slots in turn; in a slot each warp owns two
+//     records of all sixteen rows and multiplies each with eight integer mma.m16n8k32
+//     (gemv_units.cuh).  What bounds the kernel is instructions: 240 per 2304 bytes of Q4_K with all
+//     bookkeeping, 60 % of the schedulers' slots at 5.9 TB/s; dp4a, at half rate, took 250 slots for the
+//     products alone.  A record per warp and two teams (331 instructions) reached 4.6 TB/s, the dp4a
+//     kernel before 4.2 (ten independent 25600 x 5120 Q4_K products in a plan; 6.2 of Q8_0, 4.6 of Q6_K).
+//   * per job each CTA owns a contiguous range of 4-row groups; a row's partial sums go to shared
+//     memory cells by (chunk, record mod 4) and are added in fixed order: results do not depend on
+//     the partition or the ring and are bit-reproducible.
+//   * the activation is converted once per CTA and job into a 16-bit fixed-point image in shared
+//     memory; plans of several independent jobs have a small launch convert all their activations and
+//     the CTA fetches each image with one bulk copy, one job ahead where two images fit.
 //   * a job may declare that it reads what earlier jobs of the same launch wrote; the CTAs then
 //     meet at a counter in global memory before converting that job's activation.
 //   * every wait (mbarrier, counter) is bounded; on expiry the waiter raises the status word and
@@ -32,6 +31,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <vector>
 
 #include "gemv_units.cuh"
 #include "kernels.h"
@@ -40,57 +40,57 @@ namespace b200q {
 
 namespace {
 
-// timing experiments (parts of the pipeline switched off; results invalid) exist only in builds that ask for them
-#ifdef B200Q_TIMING_EXPERIMENTS
-#define GEMV_DBG(bit) (p.debug & (bit))
-#else
-#define GEMV_DBG(bit) (false)
-#endif
-
-constexpr int kMaxWarps = 15;    // consumer warps (+1 producer = 512 threads, 128 registers each)
-constexpr int kMaxDepth = 8;
-constexpr int KC = kChunkRecs;   // superblock records per chunk: 32 units of 64 weights, one per lane
-constexpr int R = kRowGroup;     // rows per item
-
-constexpr int chunk_bytes(int qt) { return (qt == QT_Q4_K || qt == QT_Q4_0 || qt == QT_MXFP4) ? KC * 144 : qt == QT_Q5_K ? KC * 176 : qt == QT_Q8_0 ? KC * 272 : 1680; }
+constexpr int kTeams = 4, kTeamWarps = 4;       // a warp has two records of a chunk: fewer barriers per record, two chains to overlap
+constexpr int kWarps = kTeams * kTeamWarps;     // consumer warps
+constexpr int kConsumers = kWarps * 32;
+constexpr int kSlots = 16;                      // ring slots at most
+constexpr int KC = kChunkRecs;
+constexpr int R = kRowGroup;                    // rows per tile
+constexpr int QG = 4;                           // row groups per quad: the 16 rows of an MMA
+constexpr int kProducers = kTeams;              // producer warps
+constexpr int kThreads = kConsumers + kProducers * 32;
+// Five warps per scheduler leave 96 registers a thread; the producers give up most of theirs
+constexpr int kLaunchRegs = 96, kConsumerRegs = 112, kProducerRegs = 32;
+static_assert(kConsumers * kConsumerRegs + kProducers * 32 * kProducerRegs <= kThreads * kLaunchRegs, "register split");
+// What the partial sums of a section (the quads between two final passes) may take; they are there twice.  A pass takes
+// about 2000 cycles with its meeting (25600 x 5120 Q4_K, eleven quads: 5570 GB/s in sections of five, 5890 in one), but the
+// ring comes first: a launch takes the largest of these sizes that leaves six slots (5120 x 25600 Q6_K beside a 61 KB
+// image: 4380 GB/s with five slots, 4660 with six).
+constexpr int kSectionBytes[] = {10240, 6144, 3840, 1};
+constexpr int quad_bytes(int mt, int nchunks) { return 16 * 16 * mt * nchunks; }
+constexpr int kZeroBytes = 384;                 // what the B loads of foreign columns read
 
 struct StreamParams {
     const StreamJob *jobs;   // device table, or nullptr when the single job is `inl`
     StreamJob inl;
     int njobs;
     int M;
-    int depth;               // ring slots per warp
-    int chunk_stride;        // bytes between the rows of a slot (largest chunk of the launch's types)
     int jobs_bytes;          // shared-memory bytes of the job table
-    int x_bytes;             // ... reserved for the fixed-point activation
-    int partial_bytes;       // ... for the per-(row, chunk) partial sums
+    int x_bytes;             // ... of one activation image area
+    int x_bufs;              // 1 or 2 areas
+    int partial_floats;      // size of one copy of a section's partial sums
+    int slots, slot_bytes;   // ring slots; bytes of one (the largest of the launch's jobs)
+    int turn;                // producers and consumer teams at work
     int has_dep;             // some job waits for earlier jobs: CTAs count completions
-    int teams;               // 2: the consumer warps work as two teams on different jobs at the same time
-    int has_xq;              // some job's activation arrives already in fixed point (StreamJob::xq)
-    int producer_nap;        // ns the producer warp sleeps when no ring slot is free (0 = spin)
-    int debug;               // experiments only: 1 stream without computing, 2 compute without
-                             // streaming, 4 skip the activation prologue, 8 skip the final pass,
-                             // 64 do not wait for the peers' partial sums
     int *status;
-    unsigned *counter;       // grid-wide completion counter (zeroed before the launch)
+    unsigned *counter;       // grid-wide completion counter (zero between launches)
     uint8_t *peer_base[kPeerMaxWorld];   // exchange buffers of the tensor-parallel ranks (peer memory)
     int peer_rank, peer_world;           // peer_world <= 1: jobs flagged SUM_RANKS store their own sums
 };
 
-// shared-memory header: barriers and failure bookkeeping (the job table follows it)
+// shared-memory header: barriers and failure bookkeeping (the zero area and the job table follow it)
 struct SmemHead {
-    uint64_t full[kMaxWarps * kMaxDepth];
-    uint64_t empty[kMaxWarps * kMaxDepth];
-    uint64_t xfull[2];       // per team: the job's pre-quantized activation has landed in the team's area
-    int fail;                // raised by any warp that gave up a wait; everybody then drains and leaves
-    int decide[2];           // per team: its first thread's sample of `fail`, taken before a barrier so all its warps agree
-    int prod_done;           // the producer warp has stopped issuing copies
-    int issued[kMaxWarps];   // ... after issuing this many items into each consumer's ring
-    unsigned xepoch[2];      // per team: exchanges posted so far (loaded from the exchange buffer)
-    int xfail;               // a wait for a peer's partial sums ran out
-    int xdone[2];            // per team: warps x jobs finished so far (a job's activation area may be refilled once all
-                             // the team's warps have left the job before it)
+    uint64_t full[kSlots];
+    uint64_t empty[kSlots];
+    uint64_t xfull[2];           // per image area: the prepared image has landed
+    float squares[kWarps];       // RMSNorm: the warps' sums of squares
+    int fetched[2];              // images sent for, per area
+    int fail;                    // raised by any warp that gave up a wait; everybody then drains and leaves
+    int decide[2];               // first thread's sample of `fail`, taken before a barrier so all warps agree
+    unsigned xepoch;             // exchanges posted so far (loaded from the exchange buffer)
+    int xfail;                   // a wait for a peer's partial sums ran out
 };
+constexpr size_t kHeadBytes = (sizeof(SmemHead) + 127) & ~size_t(127);
 
 // (value, exchange number) pairs of the in-launch rank sums: one 8-byte store / load each
 __device__ __forceinline__ void st_pair(unsigned long long *p, float v, unsigned e) {
@@ -102,7 +102,6 @@ __device__ __forceinline__ unsigned long long ld_pair(const unsigned long long *
     asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
     return w;
 }
-constexpr size_t kHeadBytes = (sizeof(SmemHead) + 127) & ~size_t(127);
 
 // (segment, row group inside it) of virtual group vg; segments are concatenated in launch order.
 // A SWIGLU job interleaves its two segments instead (even groups gate, odd groups up), so that a
@@ -121,296 +120,236 @@ __device__ __forceinline__ void locate_group(const StreamJob &J, int vg, int &s,
     g = vg - J.seg[s].group_begin;
 }
 
-// virtual groups [gb, ge) of job J that CTA b of `grid` works on (whole gate/up pairs for SWIGLU)
+// virtual groups [gb, ge) of job J that CTA b works on: the shares of the job's CTAs differ by one group (one gate/up pair
+// for SWIGLU), the others have none
 template <bool FUSED = true>
-__host__ __device__ __forceinline__ void cta_groups(const StreamJob &J, int b, int grid, int &gb, int &ge) {
-    if (FUSED && (J.flags & STREAM_JOB_SWIGLU)) {
-        const long long pairs = J.total_groups >> 1;
-        gb = 2 * (int)(pairs * b / grid);
-        ge = 2 * (int)(pairs * (b + 1) / grid);
-    } else if (J.total_groups < (1 << 21)) {
-        // (32-bit division: this runs once per job in every warp, the producer's included)
-        gb = (int)((unsigned)J.total_groups * (unsigned)b / (unsigned)grid);
-        ge = (int)((unsigned)J.total_groups * (unsigned)(b + 1) / (unsigned)grid);
-    } else {
-        gb = (int)((long long)J.total_groups * b / grid);
-        ge = (int)((long long)J.total_groups * (b + 1) / grid);
-    }
+__device__ __forceinline__ void cta_groups(const StreamJob &J, int b, int &gb, int &ge) {
+    const int unit = FUSED && (J.flags & STREAM_JOB_SWIGLU) ? 2 : 1;
+    b -= J.cta0;
+    gb = unit * (b * J.share + min(b, J.share_rest));
+    ge = gb + unit * (J.share + (b < J.share_rest ? 1 : 0));
+    if ((unsigned)b >= (unsigned)J.ctas) gb = ge = 0;
 }
 
-// barrier of one consumer team (hardware barrier 1 + team; barrier 0 is __syncthreads)
-__device__ __forceinline__ void team_sync(int team, int T) { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "r"(T) : "memory"); }
+// barrier of the consumer warps (hardware barrier 1; barrier 0 is __syncthreads)
+__device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory"); }
 
-// one item (a tile: up to 4 rows x one chunk) of one job for this lane's 64-weight unit;
-// `sl` = shared address of the tile, `stride` = byte distance between its rows
-template <int QT, int MT, typename Flush>
-__device__ __forceinline__ void item_dot(int nsb, uint32_t sl, int stride, int sb0, int lsb, int j, int nr,
-                                         const XView (&xv)[MT], int units16, bool whole, float (&acc)[R][MT],
-                                         Flush &&flush_pending) {
-    const int gsb = sb0 + lsb;
-    const int gu = gsb * 4 + j;
-    const uint32_t rec0 = sl + lsb * rec_bytes(QT);
-    float d6[R];
-    if constexpr (QT == QT_Q6_K) {
-        const uint32_t doff = sl + (uint32_t)(q6k_d_off(gsb, nsb) - rec_off(QT, sb0));
-#pragma unroll
-        for (int r = 0; r < R; ++r) d6[r] = (r < nr) ? half_bits_to_float(lds16(doff + r * stride)) : 0.f;
-    }
-    auto load_w = [&](WRegs<QT> &w, int r) {
-        if constexpr (QT == QT_Q6_K) w.load(rec0 + r * stride, j, d6[r]);
-        else w.load(rec0 + r * stride, j);
-    };
-    if constexpr (MT <= 1 || (MT == 2 && QT != QT_Q6_K)) {
-        // one or two activation rows: keep their bytes in registers, stream the weight rows past them
-        XRegs<QT> xr[MT];
-#pragma unroll
-        for (int m = 0; m < MT; ++m) xr[m].load(xv[m], gu, gsb, j, units16);
-        if (whole) flush_pending();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            if (r < nr) {
-                WRegs<QT> w;
-                load_w(w, r);
-#pragma unroll
-                for (int m = 0; m < MT; ++m) acc[r][m] += w.dot(xr[m]);
-            }
-        }
-    } else if constexpr (QT != QT_Q6_K && MT >= 3) {
-        // three or four activation rows: two passes over the tile, two rows resident in each
-        if (whole) flush_pending();
+// What a consumer warp needs to walk the slots of a section ...
+struct Walk {
+    int q0, q1, nchunks, nsb, wr, lane;
+    int bytes_full, bytes_tail, tile_stride, slots, slot_bytes;
+    int turn, turn_q, turn_c;      // from one of the team's slots to its next: slots, and as quads and chunks
+    uint32_t full0, empty0, ring, img_bytes, partial;
+    volatile int *fail;
+};
+// ... and where it is: the team's next slot (ring index and parity of its full barrier), quad and chunk in it
+struct Place {
+    int slot, parity, q, c;
+};
+
+// A consumer warp's part of a section: records wr and wr + 4 of the team's slots of quads q0..q1-1, the row sums into
+// the partial sums.  False if a wait ran out.
+template <int QT, int MT>
+__device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLane &xl) {
+    // The lane's two rows of a quad: row g / 2 of tiles (g & 1) and (g & 1) + 2, g = lane / 4.  Neighbouring lane
+    // groups read different tiles, whose places in the slot are offset so that their 16-byte loads meet no bank twice.
+    const int c4 = t.lane & 3, row_tile = (t.lane >> 2) & 1, row_in_tile = t.lane >> 3;
+    const uint32_t lane_full = t.ring + row_tile * t.tile_stride + t.wr * rec_bytes(QT) + row_in_tile * t.bytes_full;
+    const uint32_t tail_less = row_in_tile * (t.bytes_full - t.bytes_tail);
+    const uint32_t step = 2 * t.tile_stride;
+    // where the lane leaves its row sums, [quad][m][row][chunk][wr]: lane group h stores row h's
+    const int h = c4 & 1;
+    const uint32_t row_cells = 16 * t.nchunks, quad_cells = MT * 16 * row_cells;
+    const uint32_t cell0 = t.partial + ((row_tile + 2 * h) * R + row_in_tile) * row_cells + 4 * t.wr;
 #pragma unroll 1
-        for (int m0 = 0; m0 < MT; m0 += 2) {
-            XRegs<QT> xa, xb;
-            xa.load(xv[m0], gu, gsb, j, units16);
-            const bool two = m0 + 1 < MT;
-            if (two) xb.load(xv[m0 + 1 < MT ? m0 + 1 : m0], gu, gsb, j, units16);
+    while (at.q < t.q1) {
+        const uint32_t bar = t.full0 + 8 * at.slot;
+        if (!mbar_try_wait(bar, at.parity)) {
+            if (!__all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, at.parity) && !*t.fail)) return false;
+        }
+        const int rec = at.c * KC + t.wr, q = at.q, c = at.c;
+        float acc[2][MT];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-                if (r < nr) {
-                    WRegs<QT> w;
-                    load_w(w, r);
-                    const float va = w.dot(xa);
-                    const float vb = two ? w.dot(xb) : 0.f;
+        for (int m = 0; m < MT; ++m) acc[0][m] = acc[1][m] = 0.f;
+        uint32_t a = lane_full + at.slot * t.slot_bytes;
+        if (c == t.nchunks - 1) a -= tail_less;
+        uint32_t d = 0;
+        if (QT == QT_Q6_K) d = a + min(KC, t.nsb - c * KC) * 208 - t.wr * 206;     // fp16 d behind the octet
+        auto give_back = [&]() {       // one of the team's warps has what it needs of the slot
+            __syncwarp();
+            if (t.lane == 0) mbar_arrive(t.empty0 + 8 * at.slot);
+        };
+        if (rec >= t.nsb) give_back();
 #pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        if (m == m0) acc[r][m] += va;
-                        if (m == m0 + 1) acc[r][m] += vb;
-                    }
+        for (int k = 0; k < 2; ++k) {
+            if (rec + 4 * k < t.nsb) {
+                WRec<QT> r0, r1;
+                r0.load(a + 4 * k * rec_bytes(QT), d + 8 * k, c4);
+                r1.load(a + 4 * k * rec_bytes(QT) + step, d + 8 * k + step, c4);
+                if (k == 1 || rec + 4 >= t.nsb) give_back();       // everything is in registers
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    RecSums<QT> sums;
+                    XScales<QT> xs;
+                    sums.run(r0, r1, xl, rec + 4 * k, m * t.img_bytes, c4);
+                    xs.load(xl, rec + 4 * k, m * t.img_bytes, c4);
+                    acc[0][m] += sums.finish(0, r0.s, xs, c4);
+                    acc[1][m] += sums.finish(1, r1.s, xs, c4);
                 }
             }
         }
-    } else {
-        // more activation rows than registers can hold: one weight row at a time, activations re-read
-        if (whole) flush_pending();
-#pragma unroll 1
-        for (int r = 0; r < nr; ++r) {
-            WRegs<QT> w;
-            load_w(w, r);
+        // the teams take the slots in turn
+        at.slot += t.turn;
+        const bool wrap = at.slot >= t.slots;
+        at.slot -= wrap ? t.slots : 0;
+        at.parity ^= wrap;
+        at.q += t.turn_q;
+        at.c += t.turn_c;
+        const bool over = at.c >= t.nchunks;
+        at.c -= over ? t.nchunks : 0;
+        at.q += over;
+        // One cell per (row, chunk, record mod 4), for the final sum in a fixed order: results depend neither on the team
+        // nor on the partition.  The four lane groups' shares are added up.
+        const uint32_t cell = cell0 + (q - t.q0) * quad_cells + 16 * c;
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                XRegs<QT> xr;
-                xr.load(xv[m], gu, gsb, j, units16);
-                const float v = w.dot(xr);
-#pragma unroll
-                for (int rr = 0; rr < R; ++rr)
-                    if (rr == r) acc[rr][m] += v;
-            }
+        for (int m = 0; m < MT; ++m) {
+            float v = (h ? acc[1][m] : acc[0][m]) + __shfl_xor_sync(0xFFFFFFFFu, h ? acc[0][m] : acc[1][m], 1);
+            v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+            if (c4 < 2) sts32f(cell + m * 16 * row_cells, v);
         }
     }
+    return true;
 }
-
-// TYPES is the set of block types the launch's jobs use (bit 0 Q4_K, bit 1 Q6_K, bit 2 Q8_0): a
-// single-type launch compiles only that type's unpacking, which keeps it free of register spills.
-constexpr int TY_Q4K = 1, TY_Q6K = 2, TY_Q80 = 4, TY_Q5K = 8, TY_Q40 = 16, TY_MX4 = 32;
 
 // VAR: which optional code the instantiation carries.  Bit 0: the fused epilogues (SWIGLU, ACCUM, norm on
 // the load) for launches that hold such jobs; bit 1: the rank-sum exchange, for launches of attached
-// tensor-parallel ranks.  Every form carries only what it needs: the kernel is sensitive to the
-// registers and code of what it does not use.
-template <int MT, int TYPES, int VAR>
-__global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const StreamParams p) {
+// tensor-parallel ranks.
+template <int MT, int VAR>
+__global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr bool FUSED = (VAR & 1) != 0, PEER = (VAR & 2) != 0;
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int CW = (blockDim.x >> 5) - 1;     // consumer warps; warp CW is the producer
-    const int D = p.depth;
-    const int cw0 = p.teams == 2 ? (CW + 1) / 2 : CW;     // team 0 = consumer warps [0, cw0), team 1 = [cw0, CW)
 
-    // shared-memory carve-up: header, activation planes, partial sums, rings
+    // shared-memory carve-up: header, zero area, job table, activation images, partial sums, ring
     SmemHead &head = *reinterpret_cast<SmemHead *>(smem);
     const uint32_t full0 = smem_u32(head.full), empty0 = smem_u32(head.empty);
-    StreamJob *jobs_s = reinterpret_cast<StreamJob *>(smem + kHeadBytes);
-    uint8_t *xbase0 = smem + kHeadBytes + p.jobs_bytes;                       // one activation area per team
-    float *partial0 = reinterpret_cast<float *>(xbase0 + p.teams * p.x_bytes); // [row][chunk][MT], one per team
-    uint8_t *rings = reinterpret_cast<uint8_t *>(partial0) + p.teams * p.partial_bytes;
-    // Two teams: while one team sums, stores and prepares the next activation (the per-job work
-    // that keeps no data moving), the other is in the middle of its own job, so the SM always has
-    // warps doing block dots.  Team 0 = consumer warps [0, cw0), team 1 = [cw0, CW).
+    uint8_t *zero_area = smem + kHeadBytes;
+    StreamJob *jobs_s = reinterpret_cast<StreamJob *>(zero_area + kZeroBytes);
+    uint8_t *ximg0 = zero_area + kZeroBytes + p.jobs_bytes;
+    float *partial0 = reinterpret_cast<float *>(ximg0 + p.x_bufs * p.x_bytes);      // two copies: [quad][m][row][chunk][wr]
+    const int partial_floats = p.partial_floats;
+    const uint32_t ring = smem_u32(partial0 + 2 * partial_floats);
+    volatile int *fail_flag = &head.fail;
 
-    const int slot_bytes = R * p.chunk_stride;
-    const int ring_bytes = D * slot_bytes;
-
-    if (threadIdx.x < CW) {
-        for (int i = 0; i < D; ++i) {
-            mbar_init(full0 + (threadIdx.x * kMaxDepth + i) * 8, 1);
-            mbar_init(empty0 + (threadIdx.x * kMaxDepth + i) * 8, 1);
-        }
+    if (threadIdx.x < kSlots) {
+        mbar_init(full0 + 8 * threadIdx.x, QG);
+        mbar_init(empty0 + 8 * threadIdx.x, kTeamWarps);
+        if (threadIdx.x < 2) mbar_init(smem_u32(&head.xfull[threadIdx.x]), 1);
         mbar_fence_init();
         fence_proxy_async();
     }
-    if (threadIdx.x == 0) {
-        head.fail = 0; head.prod_done = 0; head.xfail = 0;
-        head.xdone[0] = head.xdone[1] = 0;
-        for (int t = 0; t < 2; ++t) mbar_init(smem_u32(&head.xfull[t]), 1);
-        mbar_fence_init();
-        fence_proxy_async();
-    }
+    if (threadIdx.x == 0) head.fail = head.xfail = head.fetched[0] = head.fetched[1] = 0;
+    if (threadIdx.x < kZeroBytes / 4) reinterpret_cast<int *>(zero_area)[threadIdx.x] = 0;
     // the job table (written by the host when the plan was made) moves to shared memory once
     if (p.jobs) {
         const int words = p.njobs * (int)(sizeof(StreamJob) / 4);
         const int *src = reinterpret_cast<const int *>(p.jobs);
         int *dst = reinterpret_cast<int *>(jobs_s);
         for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-    } else if (threadIdx.x == 0) {
-        jobs_s[0] = p.inl;
+    } else if (threadIdx.x < sizeof(StreamJob) / 4) {
+        reinterpret_cast<int *>(jobs_s)[threadIdx.x] = reinterpret_cast<const int *>(&p.inl)[threadIdx.x];
     }
     // let the next kernel in the stream start early (it waits in pdl_wait before touching data)
     pdl_launch_dependents();
     __syncthreads();
 
+    // Producer warps and consumer teams take the slots in turn, from the first job's first to the last job's last.  A
+    // warp may only wait for a use of a ring slot when it has seen the use before (two uses ahead have the same parity),
+    // so the ring has a multiple of `turn` slots, two for each of the `turn` producers and teams at work.
+    const int turn = p.turn;
+
     // =========================================================================================
-    // producer warp: lane w feeds consumer warp w.  All lanes poll together (no lane blocks the
-    // others): a lane issues its next item as soon as its consumer has released the slot.
+    // Producer warps: warp i copies slots i, i + 4, ... of all jobs, lane j of it tile j.  (A slot's wait, address
+    // arithmetic and copies are a chain of 700 to 1300 cycles, as long as HBM takes for one slot, so four warps share them.)
     // =========================================================================================
-    if (warp == CW) {
-        const unsigned mask = 0xFFFFFFFFu;
-        const bool feeder = lane < CW && !GEMV_DBG(2);
-        const uint32_t ring_s = smem_u32(rings + lane * ring_bytes);
-        const uint32_t fbar = full0 + lane * kMaxDepth * 8, ebar = empty0 + lane * kMaxDepth * 8;
-        // the consumer this lane feeds: its team, its index and the number of warps in that team
-        const int my_team = lane >= cw0 ? 1 : 0;
-        const int twarp = lane - (my_team ? cw0 : 0), tcw = my_team ? CW - cw0 : cw0;
-        int slot = 0, k = 0;
-        uint32_t phase = 0;            // parity of the release this slot's next reuse waits for
-        bool dead = false;
-        // every lane walks its own team's jobs: job cursor, item cursor inside the job
-        int jb = -1, n_items = 0, item = 0, g = 0, c = 0, gb = 0;
-        bool glu = false;
-        auto next_job = [&]() {
-            do { ++jb; } while (jb < p.njobs && p.teams == 2 && jobs_s[jb].team != my_team);
-            if (!feeder) jb = p.njobs;
-            if (jb >= p.njobs) return;
-            const StreamJob &J = jobs_s[jb];
-            glu = FUSED && (J.flags & STREAM_JOB_SWIGLU) != 0;
-            int ge;
-            cta_groups<FUSED>(J, blockIdx.x, gridDim.x, gb, ge);
-            n_items = (ge - gb) * J.nchunks;
-            item = twarp;
-            g = 0, c = twarp;          // item = g * nchunks + c, kept without dividing
-            while (c >= J.nchunks) { c -= J.nchunks; ++g; }
-        };
-        next_job();
-        // Lanes 30 and 31 feed the activation areas of team 0 and team 1: one bulk copy per job whose
-        // activation was converted to fixed point by the prep launch, as soon as the team has left
-        // the area's previous contents behind.
-        const bool xfeeder = p.has_xq && lane >= 30 && (lane - 30) < p.teams && !GEMV_DBG(2);
-        const int xteam = lane - 30;
-        int xjb = -1, xseq = 0;        // job cursor; how many of the team's jobs lie before it
-        auto next_xjob = [&]() {
-            if (xjb >= 0) ++xseq;
-            do { ++xjb; } while (xjb < p.njobs && p.teams == 2 && jobs_s[xjb].team != xteam);
-        };
-        if (xfeeder) next_xjob();
-        else xjb = p.njobs;
-        if (p.has_xq) pdl_wait();      // the prep launch's output is visible from here
-        uint64_t t_first = 0;
-        bool timing = false;
-        int idle = 0;
+    if (warp >= kWarps) {
+        setmaxnreg_dec<kProducerRegs>();
+        const int me = warp - kWarps;
+        if (lane >= QG || me >= turn) return;
+        const unsigned mask = (1u << QG) - 1;
+        int slot = me, uses = 0;       // the warp's next slot: ring index, earlier uses of it
+        int c = me;                    // slots from the job's first to it
+        int n = 0;                     // slots copied
+        bool ok = true;
 #pragma unroll 1
-        while (true) {
-            bool progressed = false;
-            if (*reinterpret_cast<volatile int *>(&head.fail)) { dead = true; break; }
-            if (jb < p.njobs) {
-                if (item >= n_items) {
-                    next_job();
-                    progressed = true;
-                } else {
-                    const StreamJob &J = jobs_s[jb];
-                    const bool free_slot = (k < D) || mbar_test_wait(ebar + 8 * slot, phase ^ 1u);
-                    if (free_slot) {
-                        int sg, lg;
-                        locate_group(J, gb + g, sg, lg, glu);
-                        const uint32_t bytes = R * ((c == J.nchunks - 1) ? J.bytes_tail : J.bytes_full);   // whole tile, padding rows included
-                        const uint32_t bar = fbar + 8 * slot;
-                        fence_proxy_async();   // the consumer's reads of this slot precede the engine's writes
-                        mbar_expect_tx(bar, bytes);
-                        // tile (row group lg, chunk c): both strides were worked out when the job was made, so the
-                        // producer's per-item path has no type logic
-                        bulk_g2s(ring_s + slot * slot_bytes, J.seg[sg].w + (long long)lg * J.tile_group_stride + c * J.tile_chunk_stride,
-                                 bytes, bar);
-                        item += tcw;
-                        c += tcw;
-                        while (c >= J.nchunks) { c -= J.nchunks; ++g; }
-                        ++k;
-                        if (++slot == D) { slot = 0; phase ^= 1u; }
-                        progressed = true;
+        for (int jb = 0; jb < p.njobs && ok; ++jb) {
+            const StreamJob &J = jobs_s[jb];
+            const bool glu = FUSED && (J.flags & STREAM_JOB_SWIGLU) != 0;
+            int gb, ge;
+            cta_groups<FUSED>(J, blockIdx.x, gb, ge);
+            const int nchunks = J.nchunks;
+            const uint32_t bytes_full = R * J.bytes_full, bytes_tail = R * J.bytes_tail;      // a whole tile, padding rows included
+            const uint32_t dst0 = ring + lane * J.tile_stride;
+            const long long group_stride = J.tile_group_stride;
+            const int chunk_stride = J.tile_chunk_stride;
+            int g = gb;
+#pragma unroll 1
+            while (true) {
+                while (c >= nchunks && g < ge) {
+                    c -= nchunks;
+                    g += QG;
+                }
+                if (g >= ge) break;                    // (c slots into the next job)
+                const uint32_t fbar = full0 + 8 * slot;
+                if (uses > 0) {
+                    const uint32_t ebar = empty0 + 8 * slot;
+                    if (!mbar_try_wait(ebar, (uses - 1) & 1)) {
+                        uint64_t t0 = 0;
+#pragma unroll 1
+                        for (int spin = 1; !mbar_try_wait(ebar, (uses - 1) & 1); ++spin) {
+                            if (*fail_flag) ok = false;
+                            if ((spin & 63) == 0) {
+                                const uint64_t now = globaltimer_ns();
+                                if (t0 == 0) t0 = now;
+                                else if (now - t0 > kWaitLimitNs) {
+                                    atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
+                                    *fail_flag = 1;
+                                    ok = false;
+                                }
+                            }
+                            if (!ok) break;
+                        }
+                        ok = __all_sync(mask, ok);
+                        if (!ok) break;
                     }
                 }
-            }
-            if (xjb < p.njobs) {
-                const StreamJob &J = jobs_s[xjb];
-                // Every job, with or without an image, is passed only once all warps of the team have
-                // finished the job before it (a plain count: nothing to confuse however far either side
-                // runs ahead).  Passing earlier would overwrite the activation area of a job still in
-                // progress and arrive twice in one phase of the image barrier.
-                const int xwarps = xteam ? CW - cw0 : cw0;
-                if (xseq != 0 && *reinterpret_cast<volatile int *>(&head.xdone[xteam]) < xseq * xwarps) {
-                    // the previous job of the team is still running
-                } else if (!J.xq) {
-                    next_xjob();
-                    progressed = true;
+                if (g + lane < ge) {                   // (the CTA's last quad may have fewer tiles)
+                    int sg = 0, lg = g + lane;
+                    if (FUSED || J.nseg > 1) locate_group(J, g + lane, sg, lg, glu);
+                    const uint32_t bytes = c == nchunks - 1 ? bytes_tail : bytes_full;
+                    fence_proxy_async();               // the consumers' reads of these bytes precede the engine's writes
+                    mbar_expect_tx(fbar, bytes);
+                    bulk_g2s(dst0 + slot * p.slot_bytes, J.seg[sg].w + lg * group_stride + (long long)c * chunk_stride, bytes, fbar);
                 } else {
-                    const int n_isum = (J.qt == QT_Q6_K) ? (J.Kpad >> 4) : (J.Kpad >> 5);
-                    const uint32_t bytes = (uint32_t)p.M * (uint32_t)(2 * J.Kpad + (J.Kpad >> 5) * 4 + n_isum * 4);
-                    const uint32_t bar = smem_u32(&head.xfull[xteam]);
-                    fence_proxy_async();
-                    mbar_expect_tx(bar, bytes);
-                    bulk_g2s(smem_u32(xbase0 + xteam * p.x_bytes), J.xq, bytes, bar);
-                    next_xjob();
-                    progressed = true;
+                    mbar_arrive(fbar);
                 }
-            }
-            if (__all_sync(mask, jb >= p.njobs && xjb >= p.njobs)) break;
-            if (__any_sync(mask, progressed)) {
-                idle = 0;
-                timing = false;
-                continue;
-            }
-            // nothing to do right now: step aside for a moment instead of taking issue slots from the
-            // consumer warps that share this scheduler (a slot frees up every ~150 ns on average)
-            if (p.producer_nap) __nanosleep(p.producer_nap);
-            if (++idle >= 1024) {   // nobody moved for a while: look at the clock
-                idle = 0;
-                const uint64_t now = globaltimer_ns();
-                if (!timing) {
-                    timing = true;
-                    t_first = now;
-                } else if (now - t_first > kWaitLimitNs) {
-                    if (lane == 0) atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
-                    *reinterpret_cast<volatile int *>(&head.fail) = 1;
-                    dead = true;
-                    break;
+                ++n;
+                c += turn;
+                slot += turn;
+                if (slot >= p.slots) {
+                    slot -= p.slots;
+                    ++uses;
                 }
             }
         }
-        (void)dead;
-        // tell the consumers how much is (or was) in flight, so a failing CTA can wait for exactly
-        // those copies before its shared memory is released
-        if (lane < CW) head.issued[lane] = k;
-        __syncwarp();
-        if (lane == 0) {
-            __threadfence_block();
-            *reinterpret_cast<volatile int *>(&head.prod_done) = 1;
+        // shared memory may only be released when the copies have landed
+        for (int i = min(n, p.slots / turn); i > 0; --i) {
+            slot -= turn;
+            if (slot < 0) {
+                slot += p.slots;
+                --uses;
+            }
+            if (!mbar_wait_bounded(full0 + 8 * slot, uses & 1)) break;
         }
         return;
     }
@@ -418,30 +357,49 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
     // =========================================================================================
     // consumer warps
     // =========================================================================================
-    const int team = warp >= cw0 ? 1 : 0;
-    const int tw0 = team ? cw0 : 0;                 // first warp of this thread's team
-    const int tcw = team ? CW - cw0 : cw0;          // warps in the team
-    const int T = tcw * 32;                         // threads in the team
-    const int tid = threadIdx.x - tw0 * 32;         // thread index inside the team
-    const int twarp = warp - tw0;
-    uint8_t *xbase = xbase0 + team * p.x_bytes;
-    float *partial_t = partial0 + team * (p.partial_bytes >> 2);      // two copies, used by alternate jobs
-    int tjobs = 0, xq_seen = 0;                                         // the team's jobs so far; those with a pre-quantized activation
-    const uint32_t ring_sa = smem_u32(rings + warp * ring_bytes);
-    const uint32_t fbar = full0 + warp * kMaxDepth * 8, ebar = empty0 + warp * kMaxDepth * 8;
-    const int lsb = lane >> 2, j = lane & 3;   // this lane's record and 64-weight group in a chunk
-    volatile int *fail_flag = &head.fail;
-    int slot = 0, consumed = 0;
-    uint32_t phase = 0;
-    XRaw xraw;                 // the next job's activation, loaded early (M = 1, bf16)
-    bool have_raw = false;
-    auto job_xsrc = [&](const StreamJob &Jx) {
-        XSrc xs;
-        xs.x = Jx.x; xs.ldx = Jx.ldx; xs.x_is_bf16 = Jx.x_is_bf16; xs.x_vec_ok = Jx.x_vec_ok;
-        xs.K = Jx.K; xs.Kpad = Jx.Kpad;
-        xs.gamma = FUSED ? Jx.gamma : nullptr;
-        xs.rs = 1.f;
-        return xs;
+    setmaxnreg_inc<kConsumerRegs>();
+    const int tid = threadIdx.x;
+    const int team = warp / kTeamWarps, wr = warp & (kTeamWarps - 1);      // wr: the warp's first record in a chunk
+    int first_slot = 0;                // number of the job's first slot, modulo turn
+    Place at;
+    at.slot = team;
+    at.parity = 0;
+    int section_no = 0;
+    uint32_t images = 0;               // images waited for: area 0 in the low half, area 1 in the high one
+
+    // image of job jn (if it has one) into its area, by one thread
+    auto fetch_image = [&](int jn, int area) {
+        if (jn >= p.njobs || !jobs_s[jn].xq) return;
+        const StreamJob &Jn = jobs_s[jn];
+        const uint32_t bytes = (uint32_t)MT * Jn.nsb * ximg_rec_bytes(Jn.qt);
+        const uint32_t bar = smem_u32(&head.xfull[area]);
+        fence_proxy_async();           // reads of the area's last image precede the engine's writes
+        *reinterpret_cast<volatile int *>(&head.fetched[area]) += 1;
+        mbar_expect_tx(bar, bytes);
+        bulk_g2s(smem_u32(ximg0 + area * p.x_bytes), Jn.xq, bytes, bar);
+    };
+    // the next job from jb on that has something for this CTA (jobs of few rows run on a part of the grid); launches whose
+    // jobs wait, and rank sums, are walked through by every CTA
+    auto next_job = [&](int jb) {
+        for (; jb < p.njobs; ++jb) {
+            int gb, ge;
+            cta_groups<FUSED>(jobs_s[jb], blockIdx.x, gb, ge);
+            if (ge > gb || p.has_dep || (PEER && (jobs_s[jb].flags & STREAM_JOB_SUM_RANKS))) break;
+        }
+        return jb;
+    };
+    int own = 0;                       // jobs of this CTA so far
+
+    // n more jobs of this CTA are done, the last of them number jb (first thread; their stores come before).  The launch's
+    // last arrival of all puts the counter back: nobody waits any more.
+    auto publish = [&](unsigned n, int jb) {
+        if (jb + 1 < p.njobs) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p.counter), "r"(n) : "memory");
+        } else {
+            __threadfence();
+            const unsigned total = gridDim.x * (unsigned)p.njobs;
+            if (atomicAdd(p.counter, n) + n == total) *reinterpret_cast<volatile unsigned *>(p.counter) = 0;
+        }
     };
 
     // ---- sums over tensor-parallel ranks, inside the launch -----------------------------------
@@ -461,16 +419,16 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
     auto exchange_complete = [&](int job, unsigned e) {
         const StreamJob &Jc = jobs_s[job];
         const unsigned long long *slots = reinterpret_cast<const unsigned long long *>(p.peer_base[p.peer_rank] + kPeerFusedSlotOff) +
-                                          (size_t)(team * 2 + (e & 1)) * kPeerMaxWorld * kPeerSlotFloats;
+                                          (size_t)(e & 1) * kPeerMaxWorld * kPeerSlotFloats;
         int gbc, gec;
-        cta_groups<FUSED>(Jc, blockIdx.x, gridDim.x, gbc, gec);
+        cta_groups<FUSED>(Jc, blockIdx.x, gbc, gec);
         const int n = Jc.seg[0].n;
         const bool accum = FUSED && (Jc.flags & STREAM_JOB_ACCUM) != 0;
         const int cells = (gec - gbc) * R * MT;
         // Eight lanes share one output: lane r of the group fetches rank r's pair (and waits for it, with the
         // usual limit), so all ranks' pairs travel at the same time; lane 0 then adds them in rank order.
         const bool dead = *reinterpret_cast<volatile int *>(&head.xfail) != 0;
-        for (int base = 0; base < cells; base += T / kPeerMaxWorld) {
+        for (int base = 0; base < cells; base += kConsumers / kPeerMaxWorld) {
             const int t = base + (tid >> 3), r = lane & 7;
             const int rl = t / MT, m = t - rl * MT;
             const int row = gbc * R + rl;
@@ -481,7 +439,7 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
             if (valid && r < p.peer_world && ok) {
                 const unsigned long long *q = slots + (size_t)r * kPeerSlotFloats + si;
                 w = ld_pair(q);
-                if ((unsigned)(w >> 32) != e && !GEMV_DBG(64)) {
+                if ((unsigned)(w >> 32) != e) {
                     const uint64_t t0 = globaltimer_ns();
                     int spins = 0;
                     while ((unsigned)((w = ld_pair(q)) >> 32) != e) {
@@ -510,15 +468,17 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
         }
     };
 
-    bool first_job = true;
+    // what the conversions need of HBM may start its way now: RMSNorm weights are nobody's output
+    if (FUSED)
+        for (int jb = 0; jb < p.njobs; ++jb)
+            if (jobs_s[jb].gamma && !jobs_s[jb].xq && tid * 32 < jobs_s[jb].K) asm volatile("prefetch.global.L2 [%0];" ::"l"(jobs_s[jb].gamma + tid * 32));
+    pdl_wait();   // the previous kernel's writes (activations, images) are visible from here
+    if (p.x_bufs == 2 && tid == 0) fetch_image(next_job(0), 0);
 #pragma unroll 1
-    for (int jb = 0; jb < p.njobs; ++jb) {
+    for (int jb = next_job(0); jb < p.njobs; jb = next_job(jb + 1), ++own) {
         const StreamJob &J = jobs_s[jb];
-        if (p.teams == 2 && J.team != team) continue;      // the other team's job
 
         // ---- dependencies --------------------------------------------------------------------
-        if (first_job) pdl_wait();   // the previous kernel's writes (activations) are visible from here
-        first_job = false;
         if (J.flags & STREAM_JOB_WAITS) {
             // every CTA has stored all earlier jobs' outputs once the counter reaches grid * jb
             if (tid == 0) {
@@ -536,229 +496,63 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
                     }
                 }
             }
-            team_sync(team, T);
+            consumers_sync();
         }
 
         // ---- this job's geometry -------------------------------------------------------------
         int gb, ge;
-        cta_groups<FUSED>(J, blockIdx.x, gridDim.x, gb, ge);
-        const int n_items = (ge - gb) * J.nchunks;
+        cta_groups<FUSED>(J, blockIdx.x, gb, ge);
+        const int nquads = (ge - gb + QG - 1) / QG;
         const int nchunks = J.nchunks, nsb = J.nsb, qt = J.qt;
         const bool glu = FUSED && (J.flags & STREAM_JOB_SWIGLU) != 0;
-        const int units16 = (J.Kpad >> 6) * 16;
-        const int plane = J.Kpad;
-        const int n_isum = (qt == QT_Q6_K) ? (J.Kpad >> 4) : (J.Kpad >> 5);
-        const int per_m = 2 * plane + (J.Kpad >> 5) * 4 + n_isum * 4;        // xh, xl, sx, isum
+        const uint32_t img_bytes = (uint32_t)nsb * ximg_rec_bytes(qt);
 
-        // ---- prologue: activation rows -> fixed point ----------------------------------------
-        // partial sums alternate between two copies: the previous job's are still being added up by
-        // slower threads of the team when this job's first items are flushed
-        float *partial = partial_t + (tjobs & 1) * (p.partial_bytes >> 3);
-        ++tjobs;
-        const bool pre_x = J.xq != nullptr && !GEMV_DBG(2);
-        XView xv[MT];
-        {
-            XSrc xs = job_xsrc(J);
-            const bool norm = FUSED && xs.gamma != nullptr && !pre_x;
-#pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                if (norm && m < p.M) {
-                    // RMSNorm on the load: the team adds up the row's squares first (partials through the
-                    // partial-sum table, which no item of this job has touched yet)
-                    float ss = row_square_share(xs, m, tid, T);
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
-                    team_sync(team, T);
-                    if (lane == 0) partial[twarp] = ss;
-                    team_sync(team, T);
-                    float tot = 0.f;
-                    for (int w = 0; w < tcw; ++w) tot += partial[w];
-                    xs.rs = rsqrtf(tot / (float)xs.K + J.norm_eps);
-                }
-                uint8_t *b = xbase + m * per_m;
-                float *sxp = reinterpret_cast<float *>(b + 2 * plane);
-                int *isp = reinterpret_cast<int *>(b + 2 * plane + (J.Kpad >> 5) * 4);
-                xv[m].xh = smem_u32(b);
-                xv[m].xl = smem_u32(b + plane);
-                xv[m].sx = smem_u32(sxp);
-                xv[m].isum = smem_u32(isp);
-                if (m < p.M && !GEMV_DBG(4) && !pre_x) {
-                    const bool q6 = (TYPES & TY_Q6K) && (TYPES == TY_Q6K || qt == QT_Q6_K);
-                    if (MT == 1 && have_raw && !norm) {
-                        if (q6) prep_from_raw<QT_Q6_K>(xs, tid, T, xraw, b, b + plane, sxp, isp, units16);
-                        else if (TYPES & ~TY_Q6K) prep_from_raw<QT_Q4_K>(xs, tid, T, xraw, b, b + plane, sxp, isp, units16);
-                    } else {
-                        if (q6) prep_row<QT_Q6_K, FUSED>(xs, m, tid, T, b, b + plane, sxp, isp, units16);
-                        else if (TYPES & ~TY_Q6K) prep_row<QT_Q4_K, FUSED>(xs, m, tid, T, b, b + plane, sxp, isp, units16);
-                    }
-                }
-            }
+        // ---- activation image ----------------------------------------------------------------
+        // All warps have left the job before this one (its last barrier), so with one area it is free now and with
+        // two the other one is: the next job's image can travel while this job runs, sent for by the team whose turn is last.
+        const int area = p.x_bufs == 2 ? own & 1 : 0;
+        uint8_t *ximg = ximg0 + area * p.x_bytes;
+        if (p.x_bufs == 2) {
+            if (tid == kTeamWarps * 32 * (first_slot == 0 ? turn - 1 : first_slot - 1)) fetch_image(next_job(jb + 1), area ^ 1);
+        } else if (tid == 0) {
+            fetch_image(jb, 0);
         }
-        if (pre_x) {
-            // the fixed-point image arrives by bulk copy: every thread waits for it itself, no team barrier
-            bool okx = mbar_wait_bounded(smem_u32(&head.xfull[team]), (uint32_t)xq_seen & 1u);
-            ++xq_seen;
-            if (!okx) {
+        if (J.xq) {
+            // every thread waits for the image itself, no barrier
+            if (!mbar_wait_bounded(smem_u32(&head.xfull[area]), (images >> (16 * area)) & 1u)) {
                 atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
                 *fail_flag = 1;
+            } else {
+                images += 1u << (16 * area);
             }
         } else {
-            team_sync(team, T);
-        }
-
-        // ---- items ---------------------------------------------------------------------------
-        // The cross-lane sum of an item's results is taken one iteration late, after the next
-        // item's shared-memory loads have been issued, so its shuffle chain hides behind them.
-        float pend[R][MT];
-        int pend_cell = -1, pend_nr = 0;   // first partial-sum cell of the pending item
-        auto flush_pending = [&]() {
-            if (pend_cell < 0) return;
-            if constexpr (MT == 1) {
-                float a[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) a[r] = pend[r][0];
-                const float v = fold_rows<R>(a, lane);
-                const int r = lane / (32 / R);
-                if ((lane & (32 / R - 1)) == 0 && r < pend_nr) partial[pend_cell + r * nchunks] = v;
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        float v = pend[r][m];
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-                        if (lane == 0 && r < pend_nr) partial[(pend_cell + r * nchunks) * MT + m] = v;
-                    }
-                }
-            }
-            pend_cell = -1;
-        };
-
-        // item = g * nchunks + c; stepping by CW items without dividing in the loop
-        const int step_g = tcw / nchunks, step_c = tcw - step_g * nchunks;
-        int g = twarp / nchunks, c = twarp - g * nchunks;
+            XSrc xs;
+            xs.x = J.x; xs.ldx = J.ldx; xs.x_is_bf16 = J.x_is_bf16; xs.x_vec_ok = J.x_vec_ok;
+            xs.K = J.K; xs.Kpad = J.Kpad;
+            xs.gamma = FUSED ? J.gamma : nullptr;
+            xs.rs = 1.f;
 #pragma unroll 1
-        for (int item = GEMV_DBG(16) ? n_items : twarp; item < n_items; item += tcw) {
-            // the common case is a slot that is already full: one probe, and the abort flag is only looked at
-            // when the warp has to wait
-            bool ok = GEMV_DBG(2) || mbar_test_wait(fbar + 8 * slot, phase);
-            if (!__all_sync(0xFFFFFFFFu, ok)) {
-                ok = mbar_wait_bounded(fbar + 8 * slot, phase);
-                ok = __all_sync(0xFFFFFFFFu, ok && !*fail_flag);
-            }
-            if (!ok) {
-                if (lane == 0) {
-                    atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
-                    *fail_flag = 1;
+            for (int m = 0; m < MT; ++m) {
+                if (FUSED && xs.gamma) {
+                    // RMSNorm on the load: the CTA adds up the row's squares first
+                    float ss = row_square_share(xs, m, tid, kConsumers);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+                    if (m > 0) consumers_sync();       // the row before has been read
+                    if (lane == 0) head.squares[warp] = ss;
+                    consumers_sync();
+                    float tot = 0.f;
+#pragma unroll
+                    for (int w = 0; w < kWarps; ++w) tot += head.squares[w];
+                    xs.rs = rsqrtf(tot / (float)xs.K + J.norm_eps);
                 }
-                break;
+                prep_row<FUSED>(xs, qt == QT_Q6_K, m, tid, kConsumers, ximg + m * img_bytes);
             }
-            int sg, lg;
-            locate_group(J, gb + g, sg, lg, glu);
-            const int nr = group_rows(lg, J.seg[sg].n);
-            const int cb = (c == nchunks - 1) ? (int)J.bytes_tail : (int)J.bytes_full;   // bytes per tile row
-            const int sb0 = c * KC;
-            float acc[R][MT];
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
-
-            // the pending sum uses full-warp shuffles, so it may sit inside the branch below only
-            // when every lane takes that branch (a chunk of 8 whole records)
-            const bool whole = (sb0 + KC <= nsb) && !GEMV_DBG(1);
-            if (!whole) flush_pending();
-            if (sb0 + lsb < nsb && !GEMV_DBG(1)) {
-                const uint32_t sl = ring_sa + slot * slot_bytes;
-                if ((TYPES & TY_Q4K) && (TYPES == TY_Q4K || qt == QT_Q4_K))
-                    item_dot<QT_Q4_K, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-                else if ((TYPES & TY_Q6K) && (TYPES == TY_Q6K || qt == QT_Q6_K))
-                    item_dot<QT_Q6_K, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-                else if ((TYPES & TY_Q5K) && (TYPES == TY_Q5K || qt == QT_Q5_K))
-                    item_dot<QT_Q5_K, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-                else if ((TYPES & TY_Q40) && (TYPES == TY_Q40 || qt == QT_Q4_0))
-                    item_dot<QT_Q4_0, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-                else if ((TYPES & TY_MX4) && (TYPES == TY_MX4 || qt == QT_MXFP4))
-                    item_dot<QT_MXFP4, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-                else if (TYPES & TY_Q80)
-                    item_dot<QT_Q8_0, MT>(nsb, sl, cb, sb0, lsb, j, nr, xv, units16, whole, acc, flush_pending);
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(ebar + 8 * slot);   // slot may be refilled
-            if (++slot == D) { slot = 0; phase ^= 1u; }
-            ++consumed;
-
-            // one shared-memory cell per (row, chunk, m): the final sum over chunks runs in a
-            // fixed order whatever warp produced which cell
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int m = 0; m < MT; ++m) pend[r][m] = acc[r][m];
-            pend_cell = GEMV_DBG(32) ? -1 : (g * R) * nchunks + c;
-            pend_nr = nr;
-            if constexpr (MT > 1) flush_pending();   // several activation rows: registers are scarce, sum at once
-            g += step_g;
-            c += step_c;
-            if (c >= nchunks) { c -= nchunks; ++g; }
+            consumers_sync();
         }
-        flush_pending();
-        // start loading the next job's activation now: the loads fly while this job is summed and
-        // stored (not possible when that activation is still being produced by this launch)
-        // this warp is done with the activation area: the next pre-quantized image may overwrite it
-        if (p.has_xq) {
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence_block();
-                atomicAdd(&head.xdone[team], 1);
-            }
-        }
-        have_raw = false;
-        if (MT == 1 && !GEMV_DBG(4)) {
-            int jn = jb + 1;
-            while (jn < p.njobs && p.teams == 2 && jobs_s[jn].team != team) ++jn;
-            if (jn < p.njobs) {
-                const StreamJob &Jn = jobs_s[jn];
-                const XSrc xn = job_xsrc(Jn);
-                if (!(Jn.flags & STREAM_JOB_WAITS) && !Jn.xq && !xn.gamma && prep_can_prefetch(xn, T)) {
-                    prep_prefetch(xn, tid, T, xraw);
-                    have_raw = true;
-                }
-            }
-        }
-        if (tid == 0) head.decide[team] = *fail_flag;
-        team_sync(team, T);
+        const XLane xl = xlane(qt, smem_u32(ximg), smem_u32(zero_area), lane, wr & 1);
 
-        if (head.decide[team]) {
-            // Some wait ran out.  Copies already issued into this warp's ring must land before
-            // the CTA's shared memory is released: learn from the producer how many were issued
-            // and wait for exactly those, each wait again with a limit.
-            const uint64_t t0 = globaltimer_ns();
-            while (!*reinterpret_cast<volatile int *>(&head.prod_done) && globaltimer_ns() - t0 < kWaitLimitNs) {}
-            const int outstanding = *reinterpret_cast<volatile int *>(&head.issued[warp]) - consumed;
-            for (int i = 0; i < outstanding && i < D; ++i) {
-                if (!mbar_wait_bounded(fbar + 8 * slot, phase)) break;
-                if (++slot == D) { slot = 0; phase ^= 1u; }
-            }
-            return;
-        }
-
-        // ---- final pass: sum the chunks of every row of this CTA in order and store ------------
         const bool xsum = xenabled && (J.flags & STREAM_JOB_SUM_RANKS);
-        if (xsum) {
-            if (!xe_loaded) {   // exchanges posted by earlier launches (after pdl_wait: their last write is visible)
-                if (tid == 0)
-                    head.xepoch[team] = *(reinterpret_cast<const unsigned *>(p.peer_base[p.peer_rank] + kPeerFusedEpochOff) + team * kPeerCtas + blockIdx.x);
-                team_sync(team, T);
-                xe = head.xepoch[team];
-                xe_loaded = true;
-            }
-            if (xpending >= 0) {
-                exchange_complete(xpending, xe);
-                xpending = -1;
-            }
-            ++xe;
-        }
         const bool accum = FUSED && (J.flags & STREAM_JOB_ACCUM) != 0;
         auto store_out = [&](const StreamSeg &S, long long idx, float v) {
             if (J.y_is_bf16) {
@@ -769,58 +563,143 @@ __global__ void __launch_bounds__((kMaxWarps + 1) * 32, 1) stream_kernel(const S
                 *yp = accum ? *yp + v : v;
             }
         };
-        if (glu) {
-            // local groups alternate gate, up: output row = silu(gate row) * up row, to the first segment's y
-            const int outs = GEMV_DBG(8) ? 0 : ((ge - gb) >> 1) * R * MT;
-            for (int t = tid; t < outs; t += T) {
-                const int ro = t / MT, m = t - ro * MT;          // ro = local pair * 4 + row in group
-                const int pair = ro / R, r = ro & (R - 1);
-                const int row = ((gb >> 1) + pair) * R + r;
-                if (row < J.seg[0].n && m < p.M) {
-                    float gv = 0.f, uv = 0.f;
-                    const int cg = ((2 * pair) * R + r) * nchunks, cu = ((2 * pair + 1) * R + r) * nchunks;
-                    for (int cc = 0; cc < nchunks; ++cc) {
-                        gv += partial[(cg + cc) * MT + m];
-                        uv += partial[(cu + cc) * MT + m];
+
+        // ---- sections: a few quads, then their final pass ----------------------------------------
+        // (quotients of small numbers: a division takes longer)
+        int job_team;
+        const int turn_q = (turn >= nchunks) + (turn >= 2 * nchunks) + (turn >= 3 * nchunks) + (turn >= 4 * nchunks);
+        const int turn_c = turn - turn_q * nchunks;
+        {
+            int ahead = team - first_slot;
+            if (ahead < 0) ahead += turn;
+            at.q = (ahead >= nchunks) + (ahead >= 2 * nchunks) + (ahead >= 3 * nchunks);
+            at.c = ahead - at.q * nchunks;
+            if (team >= turn) at.q = nquads;
+            job_team = first_slot;
+            first_slot += nquads * nchunks;
+            first_slot = turn == 3 ? first_slot % 3 : first_slot & (turn - 1);
+        }
+        int q0 = 0;
+#pragma unroll 1
+        do {
+
+            const int q1 = min(nquads, q0 + J.section);
+            // partial sums alternate between two copies: the section before is still being added up by
+            // slower threads while this one's first quads are written
+            float *partial = partial0 + (section_no & 1) * partial_floats;
+            Walk t;
+            t.q0 = q0; t.q1 = q1; t.nchunks = nchunks; t.nsb = nsb; t.wr = wr; t.lane = lane;
+            t.bytes_full = (int)J.bytes_full; t.bytes_tail = (int)J.bytes_tail; t.tile_stride = J.tile_stride;
+            t.slots = p.slots; t.slot_bytes = p.slot_bytes; t.turn = turn; t.turn_q = turn_q; t.turn_c = turn_c;
+            t.full0 = full0; t.empty0 = empty0; t.ring = ring; t.img_bytes = img_bytes;
+            t.partial = smem_u32(partial);
+            t.fail = fail_flag;
+            bool ok;
+            if (qt == QT_Q4_K) ok = section_dot<QT_Q4_K, MT>(t, at, xl);
+            else if (qt == QT_Q6_K) ok = section_dot<QT_Q6_K, MT>(t, at, xl);
+            else if (qt == QT_Q8_0) ok = section_dot<QT_Q8_0, MT>(t, at, xl);
+            else if (qt == QT_Q5_K) ok = section_dot<QT_Q5_K, MT>(t, at, xl);
+            else if (qt == QT_Q4_0) ok = section_dot<QT_Q4_0, MT>(t, at, xl);
+            else ok = section_dot<QT_MXFP4, MT>(t, at, xl);
+            if (!ok && lane == 0) {
+                atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
+                *fail_flag = 1;
+            }
+            if (tid == 0) head.decide[section_no & 1] = *fail_flag;
+            consumers_sync();
+            if (head.decide[section_no & 1]) {
+                // Some wait ran out.  The producer waits for its own copies; this CTA's share of the completion count is
+                // made up so that the counter returns to zero.
+                if (tid == 0) {
+                    for (int a = 0; a < p.x_bufs; ++a) {
+                        const int seen = (images >> (16 * a)) & 0xFFFF;
+                        if (*reinterpret_cast<volatile int *>(&head.fetched[a]) > seen) (void)mbar_wait_bounded(smem_u32(&head.xfull[a]), seen & 1);
                     }
-                    store_out(J.seg[0], (long long)m * J.seg[0].ldy + row, gv / (1.f + __expf(-gv)) * uv);
+                    if (p.has_dep) publish((unsigned)(p.njobs - jb), p.njobs - 1);
                 }
+                return;
             }
-        }
-        const int cells = (GEMV_DBG(8) || glu) ? 0 : (ge - gb) * R * MT;
-        for (int t = tid; t < cells; t += T) {
-            const int rl = t / MT, m = t - rl * MT;      // rl = local group * 4 + row in group
-            int sg, lg;
-            locate_group(J, gb + rl / R, sg, lg, false);
-            const int row = lg * R + (rl & (R - 1));
-            if (row < J.seg[sg].n && m < p.M) {
+            ++section_no;
+
+            // ---- final pass: every row's partial sums in order, epilogue, store ------------------------
+            if (xsum && q0 == 0) {
+                if (!xe_loaded) {   // exchanges posted by earlier launches (after pdl_wait: their last write is visible)
+                    if (tid == 0)
+                        head.xepoch = *(reinterpret_cast<const unsigned *>(p.peer_base[p.peer_rank] + kPeerFusedEpochOff) + blockIdx.x);
+                    consumers_sync();
+                    xe = head.xepoch;
+                    xe_loaded = true;
+                }
+                if (xpending >= 0) {
+                    exchange_complete(xpending, xe);
+                    xpending = -1;
+                }
+                ++xe;
+            }
+            // Row r of quad q: four neighbouring threads take every fourth chunk, all get the sum.  (Where there is work for a
+            // few warps only, it falls to the team that had the job's first slot, as late as possible in turn again.)
+            const int ftid = (tid - kTeamWarps * 32 * job_team) & (kConsumers - 1), fsub = ftid & 3, fidx = ftid >> 2;
+            auto row_sum = [&](int q, int m, int r) {
+                const uint32_t a = smem_u32(partial) + 16 * ((q * MT + m) * 16 + r) * nchunks;
                 float v = 0.f;
-                for (int cc = 0; cc < nchunks; ++cc) v += partial[(rl * nchunks + cc) * MT + m];
-                if (xsum) {     // one segment, fp32 output (checked when the plan was made)
-                    const size_t si = (size_t)((team * 2 + (xe & 1)) * kPeerMaxWorld + p.peer_rank) * kPeerSlotFloats + m * J.seg[0].n + row;
-                    for (int r = 0; r < p.peer_world; ++r)
-                        st_pair(reinterpret_cast<unsigned long long *>(p.peer_base[r] + kPeerFusedSlotOff) + si, v, xe);
-                    continue;
+#pragma unroll 1
+                for (int c = fsub; c < nchunks; c += 4) {
+                    const float4 w = lds128f(a + 16 * c);
+                    v += (w.x + w.y) + (w.z + w.w);
                 }
-                store_out(J.seg[sg], (long long)m * J.seg[sg].ldy + row, v);
+                v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+                v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+                return v;
+            };
+            const int gs = gb + q0 * QG, groups = min(ge - gs, (q1 - q0) * QG);      // the section's row groups
+            if (glu) {
+                // groups alternate gate, up: output row = silu(gate row) * up row, to the first segment's y
+                const int outs = (groups >> 1) * R;
+                for (int t0 = 0; t0 < outs * MT; t0 += kConsumers / 4) {
+                    const int t = min(t0 + fidx, outs * MT - 1);       // (whole warps stay for the shuffles)
+                    const int m = MT == 1 ? 0 : t / outs, o = t - m * outs;      // o = pair * 4 + row in group
+                    const int pair = o / R, r = o & (R - 1);
+                    const int row = ((gs >> 1) + pair) * R + r;
+                    const float gv = row_sum(pair >> 1, m, (pair & 1) * 8 + r), uv = row_sum(pair >> 1, m, (pair & 1) * 8 + 4 + r);
+                    if (fsub == 0 && t0 + fidx < outs * MT && row < J.seg[0].n)
+                        store_out(J.seg[0], (long long)m * J.seg[0].ldy + row, gv / (1.f + __expf(-gv)) * uv);
+                }
+            } else {
+                const int rows = groups * R;
+                for (int t0 = 0; t0 < rows * MT; t0 += kConsumers / 4) {
+                    const int t = min(t0 + fidx, rows * MT - 1);
+                    const int m = MT == 1 ? 0 : t / rows, o = t - m * rows;      // o = group * 4 + row in group
+                    const float v = row_sum(o >> 4, m, o & 15);
+                    if (fsub != 0 || t0 + fidx >= rows * MT) continue;
+                    int sg, lg;
+                    locate_group(J, gs + o / R, sg, lg, false);
+                    const int row = lg * R + (o & (R - 1));
+                    if (row < J.seg[sg].n) {
+                        if (xsum) {     // one segment, fp32 output (checked when the plan was made)
+                            const size_t si = (size_t)((xe & 1) * kPeerMaxWorld + p.peer_rank) * kPeerSlotFloats + m * J.seg[0].n + row;
+                            for (int r = 0; r < p.peer_world; ++r)
+                                st_pair(reinterpret_cast<unsigned long long *>(p.peer_base[r] + kPeerFusedSlotOff) + si, v, xe);
+                            continue;
+                        }
+                        store_out(J.seg[sg], (long long)m * J.seg[sg].ldy + row, v);
+                    }
+                }
             }
-        }
+            q0 = q1;
+        } while (q0 < nquads);
         if (xsum) {
             if (p.has_dep) exchange_complete(jb, xe);   // a later job may read y: finish now
             else xpending = jb;
         }
         if (p.has_dep) {
             // publish: this CTA's outputs of job jb are stored
-            team_sync(team, T);
-            if (tid == 0) {
-                __threadfence();
-                atomicAdd(p.counter, 1u);
-            }
+            consumers_sync();
+            if (tid == 0) publish(1, jb);
         }
     }
     if (xpending >= 0) exchange_complete(xpending, xe);
     if (xe_loaded && tid == 0)
-        *(reinterpret_cast<unsigned *>(p.peer_base[p.peer_rank] + kPeerFusedEpochOff) + team * kPeerCtas + blockIdx.x) = xe;
+        *(reinterpret_cast<unsigned *>(p.peer_base[p.peer_rank] + kPeerFusedEpochOff) + blockIdx.x) = xe;
 }
 
 }  // namespace
@@ -834,9 +713,8 @@ int gemv_max_m() { return 4; }
 namespace {
 
 // Converts the activation of every job that has an image buffer (StreamJob::xq) to the fixed-point
-// form the streaming kernel works on, once per job instead of once per CTA and job: block (job, part)
-// handles every `parts`-th run of 8 elements.  The image has the layout of the kernel's
-// shared-memory activation area ([row][xh | xl | sx | isum]), so a CTA fetches it with one bulk copy.
+// image the streaming kernel works on, once per job instead of once per CTA and job: block (job, part)
+// handles every `parts`-th run of 8 elements.
 __global__ void __launch_bounds__(256) xprep_kernel(const StreamJob *jobs, int M) {
     pdl_launch_dependents();       // the streaming launch may start (it waits before reading the images)
     const StreamJob &J = jobs[blockIdx.x];
@@ -847,14 +725,8 @@ __global__ void __launch_bounds__(256) xprep_kernel(const StreamJob *jobs, int M
     xs.gamma = J.gamma;
     xs.rs = 1.f;
     __shared__ float warp_ss[8];
-    const int units16 = (J.Kpad >> 6) * 16, plane = J.Kpad;
-    const int n_isum = (J.qt == QT_Q6_K) ? (J.Kpad >> 4) : (J.Kpad >> 5);
-    const int per_m = 2 * plane + (J.Kpad >> 5) * 4 + n_isum * 4;
     const int tid = blockIdx.y * blockDim.x + threadIdx.x, T = gridDim.y * blockDim.x;
     for (int m = 0; m < M; ++m) {
-        uint8_t *b = const_cast<uint8_t *>(J.xq) + (size_t)m * per_m;
-        float *sxp = reinterpret_cast<float *>(b + 2 * plane);
-        int *isp = reinterpret_cast<int *>(b + 2 * plane + (J.Kpad >> 5) * 4);
         if (xs.gamma) {
             // RMSNorm on the load: every block of the job adds up the whole row's squares itself
             float ss = row_square_share(xs, m, threadIdx.x, blockDim.x);
@@ -867,18 +739,13 @@ __global__ void __launch_bounds__(256) xprep_kernel(const StreamJob *jobs, int M
             for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += warp_ss[w];
             xs.rs = rsqrtf(tot / (float)xs.K + J.norm_eps);
         }
-        if (J.qt == QT_Q6_K) prep_row<QT_Q6_K, true>(xs, m, tid, T, b, b + plane, sxp, isp, units16);
-        else prep_row<QT_Q4_K, true>(xs, m, tid, T, b, b + plane, sxp, isp, units16);
+        prep_row<true>(xs, J.qt == QT_Q6_K, m, tid, T, const_cast<uint8_t *>(J.xq) + (size_t)m * J.nsb * ximg_rec_bytes(J.qt));
     }
 }
 
 }  // namespace
 
-size_t stream_xq_bytes(const StreamJob &J, int M) {
-    const size_t n_isum = J.qt == QT_Q6_K ? J.Kpad / 16 : J.Kpad / 32;
-    const size_t per_m = 2 * (size_t)J.Kpad + (J.Kpad / 32) * 4 + n_isum * 4;
-    return ((size_t)M * per_m + 255) & ~size_t(255);
-}
+size_t stream_xq_bytes(const StreamJob &J, int M) { return ((size_t)M * J.nsb * ximg_rec_bytes(J.qt) + 255) & ~size_t(255); }
 
 cudaError_t stream_xprep_launch(const StreamJob *jobs_dev, int njobs, int M, cudaStream_t st) {
     if (njobs < 1) return cudaSuccess;
@@ -888,53 +755,59 @@ cudaError_t stream_xprep_launch(const StreamJob *jobs_dev, int njobs, int M, cud
 
 namespace {
 
-template <int MT, int TYPES, int VAR = 0>
-cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStream_t st) {
-    int warps = a.warps > 0 ? a.warps : kMaxWarps;
-    if (warps > kMaxWarps) warps = kMaxWarps;
-    // shared-memory needs: the largest activation form and partial-sum table over the jobs
-    size_t x_bytes = 0, partial = 0;
-    int stride = 0;
-    for (int i = 0; i < a.njobs; ++i) {
-        const StreamJob &J = a.jobs_host[i];
-        const size_t n_isum = J.qt == QT_Q6_K ? J.Kpad / 16 : J.Kpad / 32;
-        const size_t per_m = 2 * (size_t)J.Kpad + (J.Kpad / 32) * 4 + n_isum * 4;
-        x_bytes = std::max(x_bytes, (MT * per_m + 127) & ~size_t(127));
-        int groups = (J.total_groups + grid - 1) / grid;
-        if (J.flags & STREAM_JOB_SWIGLU) groups = 2 * ((J.total_groups / 2 + grid - 1) / grid);
-        partial = std::max(partial, (((size_t)groups * R * J.nchunks * MT * 4) + 127) & ~size_t(127));
-        stride = std::max(stride, chunk_bytes(J.qt));
-    }
-    p.x_bytes = (int)x_bytes;
-    p.partial_bytes = (int)(2 * partial);          // two copies per team, used by alternate jobs
-    p.chunk_stride = stride;
-    p.jobs_bytes = (int)(((size_t)a.njobs * sizeof(StreamJob) + 127) & ~size_t(127));
-    const size_t budget = a.smem_limit;
-    // two consumer teams need two activation areas; keep them only while two ring slots per warp still fit
-    if (p.teams == 2 && kHeadBytes + p.jobs_bytes + 2 * (x_bytes + 2 * partial) + (size_t)warps * 2 * R * stride > budget) p.teams = 1;
-    if (warps < 4) p.teams = 1;
-    const size_t fixed = kHeadBytes + p.jobs_bytes + p.teams * (x_bytes + 2 * partial);
-    // fewer consumer warps when two slots each do not fit (very long rows, several activation rows)
-    while (warps > 4 && fixed + (size_t)warps * 2 * R * stride > budget) --warps;
-    if (fixed + (size_t)warps * 2 * R * stride > budget) return cudaErrorInvalidValue;
-    int depth = (int)((budget - fixed) / ((size_t)warps * R * stride));
-    if (depth > kMaxDepth) depth = kMaxDepth;
-    if (a.depth > 0 && a.depth < depth) depth = a.depth;
-    p.depth = depth;
-    const size_t smem = fixed + (size_t)warps * depth * R * stride;
+constexpr int kMaxJobsPerLaunch = 64;   // the job table lives in shared memory
 
-    if (VAR == 0) {      // pick the form once, from the plain entry
-        bool fused = false, sums = false;
-        for (int i = 0; i < a.njobs; ++i) {
-            fused = fused || (a.jobs_host[i].flags & (STREAM_JOB_SWIGLU | STREAM_JOB_ACCUM)) != 0 || a.jobs_host[i].gamma != nullptr;
-            sums = sums || (a.jobs_host[i].flags & STREAM_JOB_SUM_RANKS) != 0;
+// quads of the CTA with most of them
+int job_quads(const StreamJob &J) {
+    const int groups = ((J.flags & STREAM_JOB_SWIGLU) ? 2 : 1) * (J.share + (J.share_rest > 0));
+    return std::max(1, (groups + QG - 1) / QG);
+}
+// (no shorter than eight slots, two for every team)
+int section_quads(const StreamJob &J, int M, int bytes) {
+    return std::min(job_quads(J), std::max((8 + J.nchunks - 1) / J.nchunks, bytes / quad_bytes(M, J.nchunks)));
+}
+size_t section_bytes(const StreamJob &J, int M, int quads) { return ((size_t)quads * quad_bytes(M, J.nchunks) + 127) & ~size_t(127); }
+
+// shared memory of a launch: the largest activation image and ring slot over its jobs
+struct Fit {
+    size_t x_bytes = 0, slot = 0, jobs_bytes, partial, limit;
+    Fit(const StreamJob *jobs, int n, int M, size_t smem_limit, size_t partial_bytes) : partial(partial_bytes), limit(smem_limit) {
+        for (int i = 0; i < n; ++i) {
+            x_bytes = std::max(x_bytes, ((size_t)M * jobs[i].nsb * ximg_rec_bytes(jobs[i].qt) + 127) & ~size_t(127));
+            slot = std::max(slot, (size_t)jobs[i].slot_bytes);
         }
-        const bool peer = sums && p.peer_world > 1;
-        if (peer && fused) return launch_t<MT, TYPES, (VAR == 0 ? 3 : VAR)>(a, p, grid, st);
-        if (peer) return launch_t<MT, TYPES, (VAR == 0 ? 2 : VAR)>(a, p, grid, st);
-        if (fused) return launch_t<MT, TYPES, (VAR == 0 ? 1 : VAR)>(a, p, grid, st);
+        jobs_bytes = ((size_t)n * sizeof(StreamJob) + 127) & ~size_t(127);
     }
-    auto kern = stream_kernel<MT, TYPES, VAR>;
+    size_t fixed(int bufs) const { return kHeadBytes + kZeroBytes + jobs_bytes + bufs * x_bytes + 2 * partial; }
+    int slots(int bufs) const { return fixed(bufs) > limit ? 0 : (int)std::min<size_t>(kSlots, (limit - fixed(bufs)) / slot); }
+};
+
+template <int MT, int VAR>
+cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStream_t st) {
+    // what the partial sums, images and tables leave of the shared memory is the ring
+    size_t partial = 0;
+    bool images = false;
+    for (int i = 0; i < a.njobs; ++i) {
+        partial = std::max(partial, section_bytes(a.jobs_host[i], MT, a.jobs_host[i].section));
+        images = images || a.jobs_host[i].xq;
+    }
+    const Fit fit(a.jobs_host, a.njobs, MT, a.smem_limit, partial);
+    p.x_bytes = (int)fit.x_bytes;
+    p.jobs_bytes = (int)fit.jobs_bytes;
+    p.partial_floats = (int)(partial / 4);
+    p.slot_bytes = (int)fit.slot;
+    // Two slots for each team at work, so that one is filled while the other is read: four teams of eight slots and more,
+    // three of six, two of less (27 KB slots of Q6_K: four slots 4.4 TB/s with two teams, 4.2 with four)
+    auto turn_of = [](int slots) { return slots >= 8 ? 4 : slots >= 6 ? 3 : slots >= 2 ? 2 : 1; };
+    auto usable = [&](int bufs) { return fit.slots(bufs) - fit.slots(bufs) % turn_of(fit.slots(bufs)); };
+    // Two image areas let prepared images travel one job ahead; they pay while the ring keeps six slots or loses none.
+    p.x_bufs = (images && a.njobs > 1 && usable(2) >= std::min(6, std::max(1, usable(1)))) ? 2 : 1;
+    p.slots = usable(p.x_bufs);
+    p.turn = turn_of(p.slots);
+    if (p.slots < 1) return cudaErrorInvalidValue;
+    const size_t smem = fit.fixed(p.x_bufs) + p.slots * fit.slot;
+
+    auto kern = stream_kernel<MT, VAR>;
     static std::atomic<size_t> configured{0};   // per instantiation; a context on another device re-sets it
     static std::atomic<int> configured_dev{-1};  // (contexts on several threads may launch at once)
     int dev = 0;
@@ -945,34 +818,30 @@ cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStrea
         configured = smem;
         configured_dev = dev;
     }
-    if (p.has_dep) {
-        cudaError_t e = cudaMemsetAsync(p.counter, 0, sizeof(unsigned), st);
-        if (e != cudaSuccess) return e;
-    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)((warps + 1) * 32));
+    cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (a.pdl && !p.has_dep) ? 1 : 0;
+    // (Launches whose jobs wait for one another start early, too: a following launch's blocks only come in once every
+    // block of this one runs, so they never take the place of a block that others wait for.)
+    cfg.numAttrs = a.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-template <int TYPES>
+template <int VAR>
 cudaError_t launch_m(const StreamLaunch &a, StreamParams &p, int grid, cudaStream_t st) {
     switch (a.M) {
-    case 1: return launch_t<1, TYPES>(a, p, grid, st);
-    case 2: return launch_t<2, TYPES>(a, p, grid, st);
-    case 3: return launch_t<3, TYPES>(a, p, grid, st);
-    default: return launch_t<4, TYPES>(a, p, grid, st);
+    case 1: return launch_t<1, VAR>(a, p, grid, st);
+    case 2: return launch_t<2, VAR>(a, p, grid, st);
+    case 3: return launch_t<3, VAR>(a, p, grid, st);
+    default: return launch_t<4, VAR>(a, p, grid, st);
     }
 }
-
-constexpr int kMaxJobsPerLaunch = 64;   // the job table lives in shared memory
 
 cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
     if (a.njobs < 1 || a.M < 1 || a.M > 4 || !a.jobs_host) return cudaErrorInvalidValue;
@@ -984,27 +853,23 @@ cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
     }
     p.njobs = a.njobs;
     p.M = a.M;
-    p.debug = a.debug;
-    p.producer_nap = a.producer_nap;
     p.status = a.status;
     p.counter = a.counter;
     p.peer_rank = a.peer_rank;
     p.peer_world = a.peer_world;
     for (int r = 0; r < kPeerMaxWorld; ++r) p.peer_base[r] = a.peer_base[r];
-    p.has_dep = 0;
-    for (int i = 0; i < a.njobs; ++i)
-        if (a.jobs_host[i].flags & STREAM_JOB_WAITS) p.has_dep = 1;
-    p.has_xq = 0;
-    for (int i = 0; i < a.njobs; ++i)
-        if (a.jobs_host[i].xq) p.has_xq = 1;
-    // two teams when the launch holds jobs for both and no job waits for another
-    p.teams = 1;
-    if (!p.has_dep && a.teams != 1) {
-        bool t0 = false, t1 = false;
-        for (int i = 0; i < a.njobs; ++i) (a.jobs_host[i].team ? t1 : t0) = true;
-        if (t0 && t1) p.teams = 2;
+    bool fused = false, sums = false;
+    for (int i = 0; i < a.njobs; ++i) {
+        const StreamJob &J = a.jobs_host[i];
+        switch (J.qt) {
+        case QT_Q4_K: case QT_Q6_K: case QT_Q8_0: case QT_Q5_K: case QT_Q4_0: case QT_MXFP4: break;
+        default: return cudaErrorInvalidValue;
+        }
+        if (J.flags & STREAM_JOB_WAITS) p.has_dep = 1;
+        fused = fused || (J.flags & (STREAM_JOB_SWIGLU | STREAM_JOB_ACCUM)) != 0 || J.gamma != nullptr;
+        sums = sums || (J.flags & STREAM_JOB_SUM_RANKS) != 0;
     }
-    const int grid = a.grid > 0 ? a.grid : a.sm_count;
+    const int grid = a.grid;
     if (p.has_dep && grid > a.sm_count) return cudaErrorInvalidValue;   // the counter wait needs every CTA resident
     if (p.peer_world > 1) {
         for (int i = 0; i < a.njobs; ++i) {
@@ -1015,28 +880,14 @@ cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
                 return cudaErrorInvalidValue;
         }
     }
-    int types = 0;
-    for (int i = 0; i < a.njobs; ++i) {
-        const int qt = a.jobs_host[i].qt;
-        types |= qt == QT_Q4_K ? TY_Q4K : qt == QT_Q6_K ? TY_Q6K : qt == QT_Q8_0 ? TY_Q80 : qt == QT_Q5_K ? TY_Q5K : qt == QT_Q4_0 ? TY_Q40 : qt == QT_MXFP4 ? TY_MX4 : 64;
-    }
-    if (types & 64) return cudaErrorInvalidValue;
-    switch (types) {
-    case TY_Q4K: return launch_m<TY_Q4K>(a, p, grid, st);
-    case TY_Q6K: return launch_m<TY_Q6K>(a, p, grid, st);
-    case TY_Q80: return launch_m<TY_Q80>(a, p, grid, st);
-    case TY_Q5K: return launch_m<TY_Q5K>(a, p, grid, st);
-    case TY_Q40: return launch_m<TY_Q40>(a, p, grid, st);
-    case TY_MX4: return launch_m<TY_MX4>(a, p, grid, st);
-    default:
-        if (!(types & (TY_Q5K | TY_Q40 | TY_MX4))) return launch_m<TY_Q4K | TY_Q6K | TY_Q80>(a, p, grid, st);
-        return launch_m<TY_Q4K | TY_Q6K | TY_Q80 | TY_Q5K | TY_Q40 | TY_MX4>(a, p, grid, st);
-    }
+    const bool peer = sums && p.peer_world > 1;
+    if (peer) return fused ? launch_m<3>(a, p, grid, st) : launch_m<2>(a, p, grid, st);
+    return fused ? launch_m<1>(a, p, grid, st) : launch_m<0>(a, p, grid, st);
 }
 
 }  // namespace
 
-void stream_job_finish(StreamJob &J) {
+void stream_job_finish(StreamJob &J, int grid) {
     int groups = 0;
     for (int i = 0; i < J.nseg; ++i) {
         J.seg[i].group_begin = groups;
@@ -1049,19 +900,90 @@ void stream_job_finish(StreamJob &J) {
     J.bytes_tail = (unsigned)chunk_row_bytes(J.qt, J.nchunks - 1, J.nsb);
     J.tile_group_stride = tile_off(J.qt, 1, 0, 0, J.nsb);              // both offsets are linear in their index
     J.tile_chunk_stride = (int)tile_off(J.qt, 0, 1, 0, J.nsb);
+    // Tiles of a slot: eight lanes read 64 bytes of a row of one tile and 64 of the next tile's (Q8_0: every other 16
+    // bytes of 128, Q6_K: two pieces of 32).  Rows of a full chunk are a multiple of 128 bytes (Q6_K: 16 more), so the
+    // padding behind a tile is what keeps the two apart in the banks.
+    J.tile_stride = R * (int)J.bytes_full + (J.qt == QT_Q8_0 ? 16 : J.qt == QT_Q6_K ? 32 : 64);
+    J.slot_bytes = QG * J.tile_stride;
+    const int units = (J.flags & STREAM_JOB_SWIGLU) ? groups / 2 : groups;      // SWIGLU: gate and up groups in pairs
+    J.cta0 = 0;
+    J.ctas = grid;
+    J.share = units / grid;
+    J.share_rest = units % grid;
 }
 
-void stream_assign_teams(StreamJob *jobs, int n) {
-    // greedy: each job goes to the team whose streamed bytes per warp are lower so far
-    // (team 0 has 8 of the 15 consumer warps, team 1 has 7)
-    const double warps[2] = {(kMaxWarps + 1) / 2, kMaxWarps / 2};
-    double load[2] = {0, 0};
+// A job of a plan costs every CTA that takes part in it about 2 us whatever its share: measured 2.3 us for 16 KB of a CTA
+// (1024 x 4096 Q4_K), 2.9 for 64 KB (4096 x 4096), 5.1 for 170 KB.  So independent jobs with small shares are dealt to halves
+// or quarters of the grid, each to the one with the least to do so far, if by this estimate the plan gets shorter
+// (twenty 1024 x 4096 products 2.3 -> 1.2 us each).
+static void deal_small_jobs(StreamJob *jobs, int n, int grid) {
+    for (int i = 0; i < n; ++i)
+        if (jobs[i].flags & (STREAM_JOB_WAITS | STREAM_JOB_SUM_RANKS)) return;
+    if (n < 2 || grid < 8) return;
+    constexpr double kBytesPerUs = 42500, kMostUs = 4;     // one SM's share of the HBM bandwidth; the largest share to make
+    auto us = [&](const StreamJob &J, int parts) { return (double)J.total_groups * J.tile_group_stride * parts / (grid * kBytesPerUs); };
+    auto cost = [](double stream_us) { return std::max(2.0 + 0.6 * stream_us, 1.25 * stream_us); };
+    std::vector<int> part(n), parts(n), best_part(n), best_parts(n, 1);
+    double best = 0;
+    for (int i = 0; i < n; ++i) best += cost(us(jobs[i], 1));
+    best *= 0.97;
+    for (int most : {2, 4}) {
+        double load[4] = {0, 0, 0, 0};
+        for (int i = 0; i < n; ++i) {
+            int np = (jobs[i].flags & STREAM_JOB_SWIGLU) ? 1 : most;
+            while (np > 1 && us(jobs[i], np) > kMostUs) np >>= 1;
+            int at = 0;
+            double least = 1e30;
+            for (int k = 0; k < np; ++k) {
+                double l = 0;
+                for (int r = k * 4 / np; r < (k + 1) * 4 / np; ++r) l = std::max(l, load[r]);
+                if (l < least) {
+                    least = l;
+                    at = k;
+                }
+            }
+            const double c = cost(us(jobs[i], np));
+            for (int r = at * 4 / np; r < (at + 1) * 4 / np; ++r) load[r] = least + c;
+            part[i] = at;
+            parts[i] = np;
+        }
+        const double t = *std::max_element(load, load + 4);
+        if (t < best) {
+            best = t;
+            best_part = part;
+            best_parts = parts;
+        }
+    }
     for (int i = 0; i < n; ++i) {
-        double bytes = 0;
-        for (int s = 0; s < jobs[i].nseg; ++s) bytes += (double)jobs[i].seg[s].n * jobs[i].row_bytes;
-        const int t = (load[1] + bytes) / warps[1] < (load[0] + bytes) / warps[0] ? 1 : 0;
-        jobs[i].team = t;
-        load[t] += bytes;
+        if (best_parts[i] == 1) continue;
+        StreamJob &J = jobs[i];
+        J.cta0 = grid * best_part[i] / best_parts[i];
+        J.ctas = grid * (best_part[i] + 1) / best_parts[i] - J.cta0;
+        J.share = J.total_groups / J.ctas;
+        J.share_rest = J.total_groups % J.ctas;
+    }
+}
+
+void stream_fit_jobs(StreamJob *jobs, int n, int M, int grid, size_t smem_limit) {
+    for (int j0 = 0; j0 < n; j0 += kMaxJobsPerLaunch) deal_small_jobs(jobs + j0, std::min(kMaxJobsPerLaunch, n - j0), grid);
+    for (int j0 = 0; j0 < n; j0 += kMaxJobsPerLaunch) {
+        const int nj = std::min(kMaxJobsPerLaunch, n - j0);
+        int best = -1, best_rank = -1;
+        for (int b : kSectionBytes) {
+            size_t partial = 0;
+            for (int i = 0; i < nj; ++i) partial = std::max(partial, section_bytes(jobs[j0 + i], M, section_quads(jobs[j0 + i], M, b)));
+            const int s = std::max(0, Fit(jobs + j0, nj, M, smem_limit, partial).slots(1));
+            const int rank = s >= 6 ? 6 : s >= 2 ? 2 : s;
+            if (rank > best_rank) {
+                best = b;
+                best_rank = rank;
+            }
+        }
+        for (int i = 0; i < nj; ++i) {       // even sections
+            StreamJob &J = jobs[j0 + i];
+            const int most = section_quads(J, M, best), all = job_quads(J), sections = (all + most - 1) / most;
+            J.section = (all + sections - 1) / sections;
+        }
     }
 }
 

@@ -50,7 +50,6 @@ struct StreamJob {
     int qt;
     int K, Kpad;
     int nsb, nchunks;                  // filled by stream_job_finish
-    long long row_bytes;
     unsigned bytes_full, bytes_tail;   // filled: bytes one row adds to a chunk, all but the last / the last
     long long tile_group_stride;       // filled: bytes between the tiles of consecutive row groups (same chunk)
     int tile_chunk_stride;             // filled: bytes between the tiles of consecutive chunks (same row group)
@@ -58,7 +57,10 @@ struct StreamJob {
     long long ldx;
     int x_is_bf16, x_vec_ok, y_is_bf16;
     int flags;                         // STREAM_JOB_*
-    int team;                          // which half of the consumer warps runs the job (see stream_assign_teams)
+    int tile_stride, slot_bytes;       // filled: bytes between the tiles of a ring slot / of a slot
+    int section;                       // quads (16 rows) per final pass (filled by stream_fit_jobs)
+    int cta0, ctas;                    // filled: the CTAs that run the job
+    int share, share_rest;             // filled: row groups of a CTA; the first share_rest CTAs have one more
     const float *gamma;                // RMSNorm weight [K]: the activation is normalised on the load (null = none)
     float norm_eps;
     const uint8_t *xq;                 // device buffer for the activation in fixed point, filled by stream_xprep_launch
@@ -71,21 +73,19 @@ struct StreamLaunch {
     int njobs;
     int M;                        // 1..4
     int *status;                  // device status word
-    unsigned *counter;            // device word for grid-wide completion counting
+    unsigned *counter;            // device word for grid-wide completion counting, zero between launches; launches that
+                                  // may run at the same time have words of their own
     int sm_count;
     size_t smem_limit;            // opt-in shared memory per block
-    int warps, depth, grid;       // 0 = default
-    int debug;                    // experiments only (see gemv.cu)
+    int grid;                     // CTAs, the number the jobs were finished for
     int pdl;                      // launch with programmatic stream serialization
-    int teams;                    // 1 = never split the consumer warps into two teams
-    int producer_nap;             // ns the producer warp sleeps when it finds nothing to do (0 = spin)
     uint8_t *peer_base[8];        // every rank's exchange buffer (jobs flagged STREAM_JOB_SUM_RANKS); null = none
     int peer_rank, peer_world;
 };
 int gemv_max_m();
-void stream_job_finish(StreamJob &job);
-// Spreads the jobs of a plan over the two consumer-warp teams of a CTA, balancing streamed bytes.
-void stream_assign_teams(StreamJob *jobs, int n);
+void stream_job_finish(StreamJob &job, int grid);
+// Fits the jobs of a call or plan to each other, once all of them are known: the part of the grid each runs on, sections.
+void stream_fit_jobs(StreamJob *jobs, int n, int M, int grid, size_t smem_limit);
 size_t stream_xq_bytes(const StreamJob &J, int M);
 cudaError_t stream_xprep_launch(const StreamJob *jobs_dev, int njobs, int M, cudaStream_t st);
 cudaError_t stream_launch(const StreamLaunch &a, cudaStream_t st);

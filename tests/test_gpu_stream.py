@@ -1,0 +1,90 @@
+"""The streaming kernel's rules: ring sizes (and with them the number of teams), row quads that are not full, last chunks
+of every length, parts of the grid for plans of small products.  A result never depends on any of them."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+import magnitude_b200 as mb  # noqa: E402
+
+TYPES = [mb.TYPE_Q4_K, mb.TYPE_Q5_K, mb.TYPE_Q6_K, mb.TYPE_Q8_0, mb.TYPE_Q4_0, mb.TYPE_MXFP4]
+REL = 1e-3      # the decode route's bound: activations in 16-bit fixed point, seen 7e-5
+
+
+def _weights(orc, qt, n, k, seed):
+    return orc.quantize(qt, np.random.default_rng(seed).standard_normal((n, k), dtype=np.float32) * np.float32(0.02))
+
+
+def _acts(m, k, seed):
+    return torch.from_numpy(np.random.default_rng(seed).standard_normal((m, k), dtype=np.float32)).cuda().to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (1, 2367, 256 * 9), (2, 17, 256 * 11), (1, 700, 256 * 20), (2, 4700, 256 * 7), (1, 13, 256 * 33)])
+def test_rows_and_chunks_of_every_length(backend, orc, qt, m, n, k):
+    p = _weights(orc, qt, n, k, n + k)
+    x = _acts(m, k, 3)
+    y = backend.project(backend.upload(qt, p, n, k), x)
+    backend.sync()
+    assert backend.last_route()[0] == mb.ROUTE_GEMV
+    ref = orc.matmul_exact(qt, p, n, k, x.float().cpu().numpy())
+    assert orc.within_tolerance(y.cpu().numpy(), ref, REL)[0]
+
+
+@pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K, mb.TYPE_Q8_0])
+@pytest.mark.parametrize("m", [1, 2])
+def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
+    """One slot (one team), two, four, six (three teams) and more, alone and in a plan of jobs that wait."""
+    n, k = 5000, 256 * 21
+    p, p2 = _weights(orc, qt, n, k, 1), _weights(orc, qt, 300, 2304, 2)
+    x, x2 = _acts(m, k, 5), _acts(m, 2304, 6)
+    ref = None
+    slot = {mb.TYPE_Q4_K: 18688, mb.TYPE_Q6_K: 27008, mb.TYPE_Q8_0: 34880}[qt]
+    for slots in (None, 1, 2, 3, 4, 6):
+        if slots:
+            os.environ["B200Q_GEMV_SMEM"] = str(min(232448, 2000 + 21 * 608 * m + 2 * 16 * 16 * m * 3 * 3 + slots * slot + 6000))
+        be = mb.Backend(0)
+        os.environ.pop("B200Q_GEMV_SMEM", None)
+        w, w2 = be.upload(qt, p, n, k), be.upload(qt, p2, 300, 2304)
+        out = [be.project(w, x), torch.zeros((m, n), device="cuda"), torch.zeros((m, 300), device="cuda"), torch.zeros((m, n), device="cuda")]
+        plan = be.plan([([w], x, out[1:2]), ([w2], x2, out[2:3]), ([w], x, out[3:4])], waits=[False, True, True])
+        for _ in range(2):
+            plan.run()
+        be.sync()
+        if ref is None:
+            ref = out
+            assert orc.within_tolerance(out[0].cpu().numpy(), orc.matmul_exact(qt, p, n, k, x.float().cpu().numpy()), REL)[0]
+            assert orc.within_tolerance(out[2].cpu().numpy(), orc.matmul_exact(qt, p2, 300, 2304, x2.float().cpu().numpy()), REL)[0]
+        for a, b in zip(out, ref):
+            assert torch.equal(a, b), slots
+        assert torch.equal(out[1], out[0]) and torch.equal(out[3], out[0])
+        be.close()
+
+
+@pytest.mark.parametrize("m", [1, 2])
+def test_plans_of_small_products_share_the_grid(backend, orc, m):
+    """Products of few rows run on halves and quarters of the grid, beside a large one and a SWIGLU job; three runs alike."""
+    shapes = [(mb.TYPE_Q4_K, 512, 1024), (mb.TYPE_Q4_K, 1000, 4096), (mb.TYPE_Q6_K, 37, 512), (mb.TYPE_Q8_0, 4096, 4096), (mb.TYPE_Q4_K, 14336, 4096)]
+    shapes = (shapes * 5)[:23]
+    jobs, outs, want = [], [], []
+    for i, (qt, n, k) in enumerate(shapes):
+        w = backend.upload(qt, _weights(orc, qt, n, k, i % 5), n, k)
+        x = _acts(m, k, i)
+        y = torch.zeros((m, n), device="cuda")
+        jobs.append(([w], x, [y]))
+        outs.append(y)
+        want.append(backend.project(w, x))
+    g, u = jobs[0][0][0], jobs[5][0][0]
+    act = torch.zeros((m, 512), device="cuda")
+    for extra in (False, True):
+        plan = backend.plan(jobs + ([([g, u], jobs[0][1], [act])] if extra else []), **({"swiglu": [False] * len(jobs) + [True]} if extra else {}))
+        for _ in range(3):
+            for y in outs:
+                y.zero_()
+            plan.run()
+            backend.sync()
+            for a, b in zip(outs, want):
+                assert torch.equal(a, b)
