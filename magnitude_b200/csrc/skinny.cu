@@ -192,9 +192,11 @@ template <int MAP, int N> static cudaError_t launch_prep_t(const SkinnySet *set,
 }
 
 template <int N> static cudaError_t launch_prep(const SkinnySet *set, cudaStream_t st) {
-    switch (sk_map(set->qt)) {
+    switch (sk_map(set->qt, set->p.NT)) {
     case SK_K: return launch_prep_t<SK_K, N>(set, st);
     case SK_Q6: return launch_prep_t<SK_Q6, N>(set, st);
+    case SK_SUB32: return launch_prep_t<SK_SUB32, N>(set, st);
+    case SK_SUB16: return launch_prep_t<SK_SUB16, N>(set, st);
     default: return launch_prep_t<SK_BLOCK, N>(set, st);
     }
 }

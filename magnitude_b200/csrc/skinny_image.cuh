@@ -12,13 +12,24 @@ __device__ __forceinline__ uint32_t sk_u32(__half2 v) { return *reinterpret_cast
 
 // ---- activations -> fragments ---------------------------------------------------------------------------
 // Lane L of a warp holds elements 8 L .. 8 L + 7 of a record; they are the 16 bytes that MMA lane t of a token's quad
-// reads for unit u.  Which weights a lane meets there is set by the packed layout:
-//   K  (Q4_K, Q5_K): a 16-byte load at 64 jj + 16 t of the nibbles brings weights 128 jj + 64 (t >> 1) + 16 (t & 1) + i
-//                    (low) and + 32 (high); unit = 4 jj + 2 high + (i >> 3)
-//   Q6 (Q6_K):       a 16-byte load at 64 hh + 16 t brings 128 hh + 16 t + i (low) and + 64 (high); unit = 4 hh + 2 high + (i >> 3)
-//   BLOCK (others):  unit = 32-weight block, lane t its weights 8 t .. 8 t + 7
-enum { SK_K = 0, SK_Q6 = 1, SK_BLOCK = 2 };
-__host__ __device__ constexpr int sk_map(int qt) { return qt == QT_Q4_K || qt == QT_Q5_K ? SK_K : qt == QT_Q6_K ? SK_Q6 : SK_BLOCK; }
+// reads for unit u (SUB16: 8 bytes each of lanes t and t + 1).  Which weights a lane meets there is set by the packed
+// layout and by the kernel's loads:
+//   K (Q4_K; Q5_K at more than 16 tokens): a 16-byte load at 64 jj + 16 t of the nibbles brings weights
+//                    128 jj + 64 (t >> 1) + 16 (t & 1) + i (low) and + 32 (high); unit = 4 jj + 2 high + (i >> 3)
+//   Q6 (Q6_K at more than 16 tokens): a 16-byte load at 64 hh + 16 t brings 128 hh + 16 t + i (low) and + 64 (high);
+//                    unit = 4 hh + 2 high + (i >> 3)
+//   BLOCK:           unit = 32-weight block, lane t its weights 8 t .. 8 t + 7: an MMA stays inside one sub-block
+//   SUB32 (Q5_K up to 16 tokens): as BLOCK
+//   SUB16 (Q6_K up to 16 tokens): unit = 32-weight quadrant, its 16-weight sub-blocks one after the other, lane t weights
+//                    4 t .. 4 t + 3 of each
+// K, SUB32: sums over the 32-weight sub-blocks as one more fragment; SUB16: over the 16-weight ones as two (high, low).
+enum { SK_K = 0, SK_Q6 = 1, SK_BLOCK = 2, SK_SUB32 = 3, SK_SUB16 = 4 };
+__host__ __device__ constexpr int sk_map(int qt, int nt) {
+    return qt == QT_Q4_K || (qt == QT_Q5_K && nt > 2) ? SK_K
+           : qt == QT_Q5_K                            ? SK_SUB32
+           : qt == QT_Q6_K                            ? (nt <= 2 ? SK_SUB16 : SK_Q6)
+                                                      : SK_BLOCK;
+}
 template <int MAP> __device__ __forceinline__ void sk_unit(int L, int &u, int &t) {
     if (MAP == SK_K) {
         t = 2 * ((L >> 3) & 1) + ((L >> 1) & 1);
@@ -28,7 +39,7 @@ template <int MAP> __device__ __forceinline__ void sk_unit(int L, int &u, int &t
         u = (L >> 4) * 4 + ((L >> 3) & 1) * 2 + (L & 1);
     } else {
         u = L >> 2;
-        t = L & 3;
+        t = MAP == SK_SUB16 ? 2 * (L & 1) : L & 3;
     }
 }
 
@@ -94,10 +105,19 @@ template <int MAP> __device__ __forceinline__ void sk_put_image(const float (&v)
                           __byte_perm(h[2], h[3], 0x7632));
     };
     uint8_t *at = img + (nt * 8 + u) * 512 + (g * 4 + t) * 16;
-    *reinterpret_cast<uint4 *>(at) = order(hi);
-    if (P == 2) *reinterpret_cast<uint4 *>(at + NT * 4096) = order(lo);
+    auto put = [&](uint8_t *to, const uint4 &f) {
+        if (MAP == SK_SUB16) {
+            to += 8 * ((lane >> 1) & 1);
+            *reinterpret_cast<uint2 *>(to) = make_uint2(f.x, f.y);
+            *reinterpret_cast<uint2 *>(to + 16) = make_uint2(f.z, f.w);
+        } else {
+            *reinterpret_cast<uint4 *>(to) = f;
+        }
+    };
+    put(at, order(hi));
+    if (P == 2) put(at + NT * 4096, order(lo));
     uint8_t *xs = img + P * NT * 4096;
-    if (MAP == SK_K) {
+    if (MAP == SK_K || MAP == SK_SUB32) {
         // sum over the 32-weight sub-block = four lanes, as two fp16 halves: k slots 0..7 (high), 8..15 (low) by sub-block
         sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
         sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
@@ -109,7 +129,19 @@ template <int MAP> __device__ __forceinline__ void sk_put_image(const float (&v)
             q[2] = xl;
         }
     }
-    if (lane == 0) *reinterpret_cast<uint32_t *>(xs + NT * 256 + tok * 4) = (uint32_t)(127 - e) << 23;
+    if (MAP == SK_SUB16) {
+        // sum over the 16-weight sub-block = two lanes: k slot = sub-block (in weight order, as the scales), high halves
+        // in the first fragment, low ones in the second
+        sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
+        if ((lane & 1) == 0) {
+            const int b = lane >> 1;
+            const __half xh = __float2half_rn(sum), xl = __float2half_rn(sum - __half2float(xh));
+            __half *q = reinterpret_cast<__half *>(xs + (nt * 64 + g * 4 + ((b & 7) >> 1)) * 8 + (b >> 3) * 4 + (b & 1) * 2);
+            q[0] = xh;
+            q[128] = xl;
+        }
+    }
+    if (lane == 0) *reinterpret_cast<uint32_t *>(xs + NT * 512 + tok * 4) = (uint32_t)(127 - e) << 23;
 }
 
 template <int MAP> __device__ __forceinline__ void sk_make_image(const SkJob &J, int rec, int tok, int lane, uint8_t *img, int NT, int P) {

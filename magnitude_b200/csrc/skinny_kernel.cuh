@@ -21,18 +21,19 @@
 //   * the consumer warps each own 16 rows: they turn packed weights into fp16 operand fragments in registers and
 //     multiply with mma.sync.m16n8k16, accumulating in fp32.  The order of K inside a record is free, so a fragment
 //     is whatever weights a lane's 16-byte load brings, and the activations are laid out to match.
-// Weights enter as exact integers.  Q4_K / Q5_K: sub-block scale x level is an integer below 2^11, exact in fp16,
-// so d and dmin are applied once per record instead of a scale per 32 weights, and the minimum term is one more
-// MMA with the sub-block sums of the activations (high and low fp16 halves).  Q6_K up to 16 tokens: scale x (level - 32)
-// may take 13 bits and enters as two exact terms (low four bits; upper two bits and the offset); above 16 tokens
-// it is rounded to fp16.  The types with a scale per 32 weights accumulate per block and scale in fp32.
+// Weights enter as exact integers.  Q4_K, and Q5_K above 16 tokens: sub-block scale x level is an integer below 2^11, exact
+// in fp16, so d and dmin are applied once per record instead of a scale per 32 weights, and the minimum term is one more
+// MMA with the sub-block sums of the activations (high and low fp16 halves).  Q5_K and Q6_K up to 16 tokens: the levels
+// alone, and the sums of a sub-block are scaled in fp32 (Q6_K's offset is such a term with the sums as well); Q6_K above 16
+// tokens: scale x (level - 32), which may take 13 bits, rounded to fp16.  The types with a scale per 32 weights accumulate
+// per block and scale in fp32.
 //
 // What bounds it: up to 16 tokens the instructions that make fragments, 1.1 per weight and lane for Q4_K (a nibble under a
 // high byte 0x64 or 0x54 reads as 1024 + v or 64 + v: one logic operation, on the half-rate pipe, and one fused
-// multiply-add per two weights) and twice that for Q6_K; above, mma.sync (0.5 of a 16x8x16 per clock and SM).  Measured,
+// multiply-add per two weights) and 1.7 times that for Q6_K; above, mma.sync (0.5 of a 16x8x16 per clock and SM).  Measured,
 // us, against a kernel with one scale per 32 weights and the K range of a tile cut by 2048: sixteen Q4_K 6144 x 4096
 // products as a plan, 4 rows 91 -> 65, 16 rows 141 -> 88; Q4_K 28672 x 4096 alone, 16 rows 50 -> 32; 4096 x 4096 8 rows
-// 10.4 -> 8.3, 16 rows 12.9 -> 11.3; Q6_K 4096 x 14336 in a plan, 8 rows 15.2 -> 14.7, 16 rows 24.8 -> 18.7.
+// 10.4 -> 8.3, 16 rows 12.9 -> 11.3; Q6_K 4096 x 14336 in a plan, 8 rows 15.2 -> 14.2, 16 rows 24.8 -> 17.5.
 // Every mbarrier wait is bounded; a wait that runs out raises the status word and a flag that every role polls,
 // copies in flight are awaited (again bounded) and the kernel returns.
 #pragma once
@@ -56,7 +57,7 @@ template <int QT, int NT, int P> struct SkShape {
     static constexpr int kRows = sk_tile_rows(NT);
     static constexpr int kW = sk_w_bytes(QT, NT), kD = sk_d_bytes(QT, NT);
     static constexpr int kB = P * NT * 4096;                       // image: activation fragments of 256 weights,
-    static constexpr int kX = NT * 256;                            // Q4_K / Q5_K: sub-block sums, as a fragment,
+    static constexpr int kX = NT * 512;                            // Q4_K / Q5_K / Q6_K: sub-block sums, as fragments,
     static constexpr int kImg = sk_image_bytes(NT, P);             // and per token 1 / scale
     static constexpr int kStage = sk_stage_bytes(QT, NT, P), kHead = kSkHeadBytes, kDepth = sk_depth(QT, NT, P);
     static_assert(kDepth >= 2, "stages");
@@ -237,8 +238,176 @@ template <int QT, int NT, int P> struct SkRecordK {      // Q4_K, Q5_K
         }
     }
 };
+
+// ---- Q5_K and Q6_K up to 16 tokens: sums per sub-block -----------------------------------------------------
+// With one or two token tiles it is cheaper to scale sums than weights: every MMA stays inside one sub-block, and its sum is
+// multiplied by the sub-block's scale, one fused multiply-add per accumulator where a scale per pair of weights took a
+// half-rate one each, and for Q6_K a second term and its products (no fp16 pair holds scale x level exactly).  Levels then
+// enter as they are, as fp16 subnormals: bits without an exponent, exact, two or three logic operations per pair.  They are
+// shifted to the top of the ten mantissa bits (32 x a 5-bit level, 16 x a 6-bit one; the factor goes into d): the tensor
+// core aligns its sums to the exponent and not to the leading bit, and levels at the bottom lost six bits (error against 64
+// bits 2.6e-6; shifted 2e-7, scaled weights 4e-7 to 7e-7).
+// Measured (us per call, inputs larger than L2), scaled weights -> scaled sums, bf16 plan of one type's calls:
+//   Q6_K 4096 x 14336: 8 tokens 16.0 -> 14.2, 16 tokens 20.3 -> 17.5; fp32 4 tokens 19.6 -> 16.4
+//   Q5_K 4096 x 14336: 8 tokens 13.3 -> 12.5, 16 tokens 15.7 -> 15.3; fp32 4 tokens 15.0 -> 14.0
+//   Q4_K 6144 x  4096: 8 tokens 4.78 -> 4.90, 16 tokens 5.98 -> 6.28: 392 instructions per 16-row record instead of 347 (a
+//   4-bit level needs one logic operation and one multiply-add as it is), so Q4_K keeps the scaled weights.
+// Bound by instruction issue: Q6_K 4096 x 14336, 8 tokens: 92.7 -> 80.2 us for 6 calls under counters, 60 -> 68 % of issue
+// slots, tensor pipe 22.7 -> 14.7 %.
+
+// byte k of w minus off as fp32
+__device__ __forceinline__ float sk_byte(uint32_t w, int k, float off) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7650 | k)) - (8388608.f + off);      // 2^23 + byte
+}
+template <int NT, int P>
+__device__ __forceinline__ void sk_mma_16(float (&c)[NT][4], const uint32_t (&a)[4], uint32_t bs, int u, int half, bool first) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int pl = 0; pl < P; ++pl) {
+            const uint2 b = ldsn64(bs + pl * NT * 4096 + (nt * 8 + u) * 512 + 8 * half);
+            if (first && pl == 0) mma0(c[nt], a, b.x, b.y);
+            else mma(c[nt], a, b.x, b.y);
+        }
+}
+template <int NT>
+__device__ __forceinline__ void sk_add_scaled(float (&e)[NT][4], const float (&c)[NT][4], float s0, float s1) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        e[nt][0] = fmaf(s0, c[nt][0], e[nt][0]);
+        e[nt][1] = fmaf(s0, c[nt][1], e[nt][1]);
+        e[nt][2] = fmaf(s1, c[nt][2], e[nt][2]);
+        e[nt][3] = fmaf(s1, c[nt][3], e[nt][3]);
+    }
+}
+
+template <int NT, int P> struct SkRecordSub32 {              // Q5_K
+    static __device__ __forceinline__ void run(const uint32_t (&row)[2], uint32_t, uint32_t bs, uint32_t xs, uint32_t inv, int t,
+                                               SkAcc<NT> (&acc)[NT][4]) {
+        uint32_t sc[2][2], am[4];                // scales of sub-blocks 0..3, 4..7; the minima as a fragment: k slots 2 t, 2 t + 1 (and + 8)
+        float d[2], dmin[2];
+        uint2 f[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint4 hd = ldsn128(row[i]);
+            d[i] = half_bits_to_float(hd.x) * 524288.f;       // 2^24 / 32
+            dmin[i] = half_bits_to_float(hd.x >> 16);
+            sc[i][0] = hd.y & 0x3F3F3F3Fu;
+            sc[i][1] = (hd.w & 0x0F0F0F0Fu) | ((hd.y >> 2) & 0x30303030u);
+            const uint32_t m = (t < 2 ? (hd.z & 0x3F3F3F3Fu) : (((hd.w >> 4) & 0x0F0F0F0Fu) | ((hd.z >> 2) & 0x30303030u))) >> (16 * (t & 1));
+            const uint32_t mh = hadd(__byte_perm(m, 0x64646464u, 0x4140), 0xE400E400u);
+            put(am, i, mh, mh);
+            f[i] = ldsn64(row[i] + 144 + 8 * t);
+        }
+        float e[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) e[nt][x] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {            // sub-blocks 2 j (low nibbles) and 2 j + 1
+            uint2 w[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) w[i] = ldsn64(row[i] + 16 + 32 * j + 8 * t);
+            uint32_t lo[2][4], hi[2][4];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t v = x ? w[i].y : w[i].x;
+                    const uint32_t b = (x ? f[i].y : f[i].x) >> (2 * j);       // fifth bit of sub-block s: bit s of the byte
+                    put(lo[x], i, and_or(b << 9, 0x02000200u, (v << 5) & 0x01E001E0u), and_or(b << 1, 0x02000200u, (v >> 3) & 0x01E001E0u));
+                    put(hi[x], i, and_or(b << 8, 0x02000200u, (v << 1) & 0x01E001E0u), and_or(b, 0x02000200u, (v >> 7) & 0x01E001E0u));
+                }
+            }
+            float c[NT][4];
+            sk_mma_planes<NT, P>(c, lo[0], lo[1], bs, 2 * j, true);
+            sk_add_scaled<NT>(e, c, sk_byte(sc[0][j >> 1], 2 * (j & 1), 0.f), sk_byte(sc[1][j >> 1], 2 * (j & 1), 0.f));
+            sk_mma_planes<NT, P>(c, hi[0], hi[1], bs, 2 * j + 1, true);
+            sk_add_scaled<NT>(e, c, sk_byte(sc[0][j >> 1], 2 * (j & 1) + 1, 0.f), sk_byte(sc[1][j >> 1], 2 * (j & 1) + 1, 0.f));
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const uint2 bx = ldsn64(xs + nt * 256);
+            const uint2 iv = ldsn64(inv + nt * 32);
+            const float i0 = __uint_as_float(iv.x), i1 = __uint_as_float(iv.y);
+            float x[4];
+            mma0(x, am, bx.x, bx.y);
+            SkAcc<NT>(&a)[4] = acc[nt];
+            a[0] += fmaf(d[0], e[nt][0], -dmin[0] * x[0]) * i0;
+            a[1] += fmaf(d[0], e[nt][1], -dmin[0] * x[1]) * i1;
+            a[2] += fmaf(d[1], e[nt][2], -dmin[1] * x[2]) * i0;
+            a[3] += fmaf(d[1], e[nt][3], -dmin[1] * x[3]) * i1;
+        }
+    }
+};
+
+template <int NT, int P> struct SkRecordSub16 {              // Q6_K: levels 0..63, the offset 32 by the sub-block sums
+    static __device__ __forceinline__ void run(const uint32_t (&row)[2], uint32_t dsm, uint32_t bs, uint32_t xs, uint32_t inv, int t,
+                                               SkAcc<NT> (&acc)[NT][4]) {
+        uint4 sc[2];                             // int8 scales + 128
+        uint32_t am[4];                          // scales as a fragment: k slot = sub-block
+        float d[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            sc[i] = ldsn128(row[i] + 192);
+            sc[i].x ^= 0x80808080u, sc[i].y ^= 0x80808080u, sc[i].z ^= 0x80808080u, sc[i].w ^= 0x80808080u;
+            uint16_t dv;
+            asm("ld.shared.u16 %0, [%1];" : "=h"(dv) : "r"(dsm + 8 * i * 16));
+            d[i] = half_bits_to_float(dv);
+            const uint32_t s0 = (t < 2 ? sc[i].x : sc[i].y) >> (16 * (t & 1)), s1 = (t < 2 ? sc[i].z : sc[i].w) >> (16 * (t & 1));
+            // byte under 0x64 reads 1024 + 128 + scale
+            d[i] *= 1048576.f;                   // 2^24 / 16
+            put(am, i, hadd(__byte_perm(s0, 0x64646464u, 0x4140), 0xE480E480u), hadd(__byte_perm(s1, 0x64646464u, 0x4140), 0xE480E480u));
+        }
+        float e[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) e[nt][x] = 0.f;
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+#pragma unroll
+            for (int ph = 0; ph < 2; ++ph) {     // positions 16 ph .. of the half's four 32-weight quadrants
+                uint32_t a[4][4];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const uint32_t l0 = ldsn32(row[i] + 64 * hh + 16 * ph + 4 * t), l1 = ldsn32(row[i] + 64 * hh + 32 + 16 * ph + 4 * t);
+                    const uint32_t q = ldsn32(row[i] + 128 + 32 * hh + 16 * ph + 4 * t);
+                    constexpr uint32_t n = 0x00F000F0u, u = 0x03000300u;       // 16 x level: nibble, upper two bits
+                    put(a[0], i, and_or(q << 8, u, (l0 << 4) & n), and_or(q, u, (l0 >> 4) & n));
+                    put(a[1], i, and_or(q << 6, u, (l1 << 4) & n), and_or(q >> 2, u, (l1 >> 4) & n));
+                    put(a[2], i, and_or(q << 4, u, l0 & n), and_or(q >> 4, u, (l0 >> 8) & n));
+                    put(a[3], i, and_or(q << 2, u, l1 & n), and_or(q >> 6, u, (l1 >> 8) & n));
+                }
+#pragma unroll
+                for (int qd = 0; qd < 4; ++qd) {
+                    float c[NT][4];
+                    sk_mma_16<NT, P>(c, a[qd], bs, 4 * hh + qd, ph, true);
+                    const int s = 8 * hh + 2 * qd + ph;
+                    sk_add_scaled<NT>(e, c, sk_byte(word_of(sc[0], s >> 2), s & 3, 128.f), sk_byte(word_of(sc[1], s >> 2), s & 3, 128.f));
+                }
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const uint2 bh = ldsn64(xs + nt * 512), bl = ldsn64(xs + nt * 512 + 256);
+            const uint2 iv = ldsn64(inv + nt * 32);
+            const float i0 = __uint_as_float(iv.x), i1 = __uint_as_float(iv.y);
+            float x[4];
+            mma0(x, am, bh.x, bh.y);
+            mma(x, am, bl.x, bl.y);
+            SkAcc<NT>(&a)[4] = acc[nt];
+            a[0] += d[0] * i0 * fmaf(-32.f / 1048576.f, x[0], e[nt][0]);
+            a[1] += d[0] * i1 * fmaf(-32.f / 1048576.f, x[1], e[nt][1]);
+            a[2] += d[1] * i0 * fmaf(-32.f / 1048576.f, x[2], e[nt][2]);
+            a[3] += d[1] * i1 * fmaf(-32.f / 1048576.f, x[3], e[nt][3]);
+        }
+    }
+};
+
 template <int NT, int P> struct SkRecord<QT_Q4_K, NT, P> : SkRecordK<QT_Q4_K, NT, P> {};
-template <int NT, int P> struct SkRecord<QT_Q5_K, NT, P> : SkRecordK<QT_Q5_K, NT, P> {};
+template <int NT, int P> struct SkRecord<QT_Q5_K, NT, P> : std::conditional<(NT <= 2), SkRecordSub32<NT, P>, SkRecordK<QT_Q5_K, NT, P>>::type {};
 
 // acc += d * inv * c, d of the lane's rows
 template <int NT>
@@ -255,10 +424,9 @@ __device__ __forceinline__ void sk_scale(SkAcc<NT> (&acc)[NT][4], const float (&
     }
 }
 
-template <int NT, int P> struct SkRecord<QT_Q6_K, NT, P> {
+template <int NT, int P> struct SkRecordQ6 {                 // more than 16 tokens: scale x (level - 32) rounded to fp16
     static __device__ __forceinline__ void run(const uint32_t (&row)[2], uint32_t dsm, uint32_t bs, uint32_t, uint32_t inv, int t,
                                                SkAcc<NT> (&acc)[NT][4]) {
-        constexpr bool kTwo = NT <= 2;               // exact in two terms
         const int h = t >> 1;
         const uint32_t sel = 0x4040u + 0x0101u * t;
         uint4 sc[2];
@@ -268,13 +436,13 @@ template <int NT, int P> struct SkRecord<QT_Q6_K, NT, P> {
             sc[i] = ldsn128(row[i] + 192);           // int8 scales: word 2 hh + high, byte t
             uint16_t dv;
             asm("ld.shared.u16 %0, [%1];" : "=h"(dv) : "r"(dsm + 8 * i * 16));
-            d[i] = half_bits_to_float(dv) * (kTwo ? 4.f : 1.f);
+            d[i] = half_bits_to_float(dv);
         }
         float c[NT][4];
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             uint4 l[2], q[2];
-            __half2 s[2][2], k[2][2], s16[2][2];
+            __half2 s[2][2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 l[i] = ldsn128(row[i] + 64 * hh + 16 * t);
@@ -282,49 +450,32 @@ template <int NT, int P> struct SkRecord<QT_Q6_K, NT, P> {
 #pragma unroll
                 for (int e = 0; e < 2; ++e)          // byte ^ 0x80 under 0x64 reads 1024 + 128 + scale
                     s[i][e] = h2(hadd(__byte_perm(word_of(sc[i], 2 * hh + e) ^ 0x80808080u, 0x64646464u, sel), 0xE480E480u));
-                if (kTwo) {
-                    s16[i][0] = __hmul2(s[i][0], h2(0x44004400u)), s16[i][1] = __hmul2(s[i][1], h2(0x44004400u));      // 16 s / 4
-                    k[i][0] = __hmul2(s[i][0], h2(0xDC00DC00u)), k[i][1] = __hmul2(s[i][1], h2(0xCC00CC00u));          // -1024 s / 4, -64 s / 4
-                    s[i][0] = __hmul2(s[i][0], h2(0x34003400u)), s[i][1] = __hmul2(s[i][1], h2(0x34003400u));          // s / 4
-                }
             }
 #pragma unroll
             for (int qq = 0; qq < 2; ++qq) {
-                uint32_t lo[2][4], hi[2][4], lo2[2][4], hi2[2][4];
+                uint32_t lo[2][4], hi[2][4];
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const uint32_t v = word_of(l[i], 2 * qq + e), x = word_of(q[i], 2 * qq + e);
                         // upper bits: field 2 h (low nibbles' weights) and 4 + 2 h (high nibbles')
-                        if (kTwo) {
-                            // two terms, each exact: scale x low four bits, 16 scale x (upper two - 2), all over 4 so that
-                            // 1024 x scale does not overflow (66 x scale would be rounded: that base is taken off first)
-                            const uint32_t v8 = v >> 8, xs = x >> (2 * h), xs8 = xs >> 8;
-                            auto two = [](uint32_t a, uint32_t off, __half2 m) { return u32(__hmul2(h2(hadd(a, off)), m)); };
-                            put(lo[e], i, hfma(and_or(v, 0x000F000Fu, 0x64006400u), s[i][0], k[i][0]), hfma(and_or(v8, 0x000F000Fu, 0x64006400u), s[i][0], k[i][0]));
-                            put(hi[e], i, hfma(and_or(v, 0x00F000F0u, 0x54005400u), s[i][1], k[i][1]), hfma(and_or(v8, 0x00F000F0u, 0x54005400u), s[i][1], k[i][1]));
-                            put(lo2[e], i, two(and_or(xs, 0x00030003u, 0x64006400u), 0xE402E402u, s16[i][0]), two(and_or(xs8, 0x00030003u, 0x64006400u), 0xE402E402u, s16[i][0]));
-                            put(hi2[e], i, two(and_or(xs, 0x00300030u, 0x54005400u), 0xD420D420u, s16[i][1]), two(and_or(xs8, 0x00300030u, 0x54005400u), 0xD420D420u, s16[i][1]));
-                        } else {
-                            const uint32_t v8 = v >> 8, xs = x >> (2 * h), xs8 = xs >> 8;          // low weights' field at bits 0-1, high at 4-5
-                            const uint32_t l0 = and_or(xs << 4, 0x00300030u, and_or(v, 0x000F000Fu, 0x64006400u)), l1 = and_or(xs8 << 4, 0x00300030u, and_or(v8, 0x000F000Fu, 0x64006400u));
-                            const uint32_t h0 = and_or(xs, 0x00300030u, and_or(v >> 4, 0x000F000Fu, 0x64006400u)), h1 = and_or(xs8, 0x00300030u, and_or(v8 >> 4, 0x000F000Fu, 0x64006400u));
-                            auto q6 = [](uint32_t a, __half2 sv) { return u32(__hmul2(h2(hadd(a, 0xE420E420u)), sv)); };      // (1024 + q - 1056) s
-                            put(lo[e], i, q6(l0, s[i][0]), q6(l1, s[i][0]));
-                            put(hi[e], i, q6(h0, s[i][1]), q6(h1, s[i][1]));
-                        }
+                        const uint32_t v8 = v >> 8, xs = x >> (2 * h), xs8 = xs >> 8;          // low weights' field at bits 0-1, high at 4-5
+                        const uint32_t l0 = and_or(xs << 4, 0x00300030u, and_or(v, 0x000F000Fu, 0x64006400u)), l1 = and_or(xs8 << 4, 0x00300030u, and_or(v8, 0x000F000Fu, 0x64006400u));
+                        const uint32_t h0 = and_or(xs, 0x00300030u, and_or(v >> 4, 0x000F000Fu, 0x64006400u)), h1 = and_or(xs8, 0x00300030u, and_or(v8 >> 4, 0x000F000Fu, 0x64006400u));
+                        auto q6 = [](uint32_t a, __half2 sv) { return u32(__hmul2(h2(hadd(a, 0xE420E420u)), sv)); };      // (1024 + q - 1056) s
+                        put(lo[e], i, q6(l0, s[i][0]), q6(l1, s[i][0]));
+                        put(hi[e], i, q6(h0, s[i][1]), q6(h1, s[i][1]));
                     }
                 }
                 sk_mma_planes<NT, P>(c, lo[0], lo[1], bs, 4 * hh + qq, hh == 0 && qq == 0);
-                if (kTwo) sk_mma_planes<NT, P>(c, lo2[0], lo2[1], bs, 4 * hh + qq, false);
                 sk_mma_planes<NT, P>(c, hi[0], hi[1], bs, 4 * hh + 2 + qq, false);
-                if (kTwo) sk_mma_planes<NT, P>(c, hi2[0], hi2[1], bs, 4 * hh + 2 + qq, false);
             }
         }
         sk_scale<NT>(acc, c, d, inv);
     }
 };
+template <int NT, int P> struct SkRecord<QT_Q6_K, NT, P> : std::conditional<(NT <= 2), SkRecordSub16<NT, P>, SkRecordQ6<NT, P>>::type {};
 
 // Types with one scale per 32 weights: units are blocks; e += d_block * c, then acc += inv * e
 template <int QT, int NT, int P> struct SkRecordBlock {
@@ -502,7 +653,10 @@ __global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel
     } else {
         // ===== products ======================================================================================
         const int g = lane >> 2, t = lane & 3;
-        const int rev = ((g & 1) << 2) | (g & 2) | (g >> 2);      // rows 4 apart in neighbouring g: conflict-free 16-byte loads
+        // the lane's row: neighbouring g read rows whose loads meet no bank twice (16 bytes: rows 4 apart; 8 bytes of 176:
+        // rows 2 apart; 4 bytes of 208: any)
+        constexpr int kMap = sk_map(QT, NT);
+        const int rev = kMap == SK_SUB32 ? ((g & 3) << 1) | (g >> 2) : kMap == SK_SUB16 ? g : ((g & 1) << 2) | (g & 2) | (g >> 2);
         const int row0 = warp * 16 + rev;
         if (p.direct) {                      // all the block's slots have a stage of their own: their images go straight there
             pdl_wait();
@@ -512,7 +666,7 @@ __global__ void __launch_bounds__(SkShape<QT, NT, P>::kThreads, 1) skinny_kernel
                 const SkJob &J = jobs[at.ji];
                 uint8_t *img = smem + S::kHead + (s - begin) * S::kStage + S::kW + S::kD;
                 for (int tok = (warp + kSkConsumers - from) % kSkConsumers; tok < J.M; tok += kSkConsumers)
-                    sk_make_image<sk_map(QT)>(J, at.rec, tok, lane, img, NT, P);
+                    sk_make_image<sk_map(QT, NT)>(J, at.rec, tok, lane, img, NT, P);
                 from = (from + J.M) % kSkConsumers;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(S::kWarps * 32) : "memory");

@@ -19,8 +19,8 @@ __host__ __device__ inline int sk_slot_begin(int slots, int grid, int b) { retur
 // the block that a slot belongs to
 __host__ __device__ inline int sk_slot_owner(int slots, int grid, int s) { return (int)((((long long)s + 1) * grid - 1) / slots); }
 // activation image of one record: fragments [plane][token tile][unit 8][lane 32] x 16 bytes, block-sum fragments
-// [token tile][lane 32] x 8 bytes, 1 / scale [token] x 4 bytes
-__host__ __device__ constexpr int sk_image_bytes(int nt, int planes) { return nt * (planes * 4096 + 256 + 32); }
+// [token tile][lane 32] x 8 bytes, one or (Q6_K) two, 1 / scale [token] x 4 bytes
+__host__ __device__ constexpr int sk_image_bytes(int nt, int planes) { return nt * (planes * 4096 + 512 + 32); }
 
 // shared memory: a stage holds a slot's packed records (Q6_K: and its rows' 16-byte groups of fp16 d) and the record's image
 constexpr int kSkHeadBytes = 256, kSkMaxDepth = 8;
