@@ -206,3 +206,31 @@ def test_config3_verify_batches_full_size(backend, orc, qt, n, k):
             assert ok, f"M={m} on the skinny route: worst error {worst:.3f} x tolerance"
     finally:
         backend.set_option(B.OPT_SKINNY_MIN_M, 3)
+
+
+@pytest.mark.parametrize("qt,size", [(mb.TYPE_Q5_K, 176), (mb.TYPE_Q6_K, 210)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [3, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(17, 256), (530, 1280)])
+def test_skinny_scaled_sums_are_exact(backend, orc, qt, size, dtype, m, n, k):
+    """Every scale and level (int8 scales down to -128) and rows of one sign, where the offset and minimum terms cancel most.
+    Levels, scales and bf16 values enter exactly, fp32 ones with 22 bits: what is left is fp32 sums, 16 products, 16
+    sub-blocks and k / 256 records deep, and the low halves of the sums: below 64 x 2^-24 of sum |x| (|scale x level| + |offset|)."""
+    rng = np.random.default_rng(7 * n + m)
+    blocks = rng.integers(0, 256, (n * k // 256, size), dtype=np.uint8)
+    d = lambda c: rng.uniform(1e-3, 2e-3, c).astype(np.float16).view(np.uint8).reshape(c, 2)  # noqa: E731
+    if qt == mb.TYPE_Q5_K:
+        blocks[:, 0:2], blocks[:, 2:4] = d(len(blocks)), d(len(blocks))
+        top = 2e-3 * 63 * 32
+    else:
+        blocks[:, 208:210] = d(len(blocks))
+        blocks[::3, 192:208] = 128                    # scale -128
+        top = 2e-3 * 128 * 96
+    packed = blocks.reshape(n, -1)
+    x = (_acts(m, k, seed=m, dtype=torch.float32).abs() + 0.5).to(dtype)
+    y = backend.project(backend.upload(qt, packed, n, k), x)
+    assert backend.last_route()[0] == mb.ROUTE_SKINNY
+    backend.sync()
+    ref = orc.matmul_exact(qt, packed, n, k, x.float().cpu().numpy())
+    bound = 64 * 2.0**-24 * top * x.float().abs().sum(1, keepdim=True).cpu().numpy()
+    assert (np.abs(y.cpu().numpy() - ref) <= bound).all()
