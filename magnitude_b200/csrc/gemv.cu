@@ -164,8 +164,11 @@ __device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLan
 #pragma unroll 1
     while (at.q < t.q1) {
         const uint32_t bar = t.full0 + 8 * at.slot;
-        if (!mbar_try_wait(bar, at.parity)) {
-            if (!__all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, at.parity) && !*t.fail)) return false;
+        // (Lanes may see the phase end at different moments: the warp votes on the probe before it branches, here and in the
+        // producers, so that no lane goes on while another waits for it in a vote.)
+        if (!__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, at.parity))) {
+            const bool ok = mbar_wait_bounded(bar, at.parity) && !*t.fail;
+            if (!__all_sync(0xFFFFFFFFu, ok)) return false;
         }
         const int rec = at.c * KC + t.wr, q = at.q, c = at.c;
         float acc[2][MT];
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
                 const uint32_t fbar = full0 + 8 * slot;
                 if (uses > 0) {
                     const uint32_t ebar = empty0 + 8 * slot;
-                    if (!mbar_try_wait(ebar, (uses - 1) & 1)) {
+                    if (!__all_sync(mask, mbar_try_wait(ebar, (uses - 1) & 1))) {
                         uint64_t t0 = 0;
 #pragma unroll 1
                         for (int spin = 1; !mbar_try_wait(ebar, (uses - 1) & 1); ++spin) {
@@ -525,6 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
             } else {
                 images += 1u << (16 * area);
             }
+            __syncwarp();
         } else {
             XSrc xs;
             xs.x = J.x; xs.ldx = J.ldx; xs.x_is_bf16 = J.x_is_bf16; xs.x_vec_ok = J.x_vec_ok;
