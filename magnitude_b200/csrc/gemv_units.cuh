@@ -396,8 +396,10 @@ __device__ __forceinline__ void prep_store8(bool q6, const float (&v)[8], int k0
     top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
     const bool bad = top > __float_as_uint(3.0e38f);
     const float amax = __uint_as_float(top);
-    constexpr float kTiny = 1.0e-33f;   // below this the reciprocal would overflow: a fixed step instead
-    const float inv = amax >= kTiny ? __fdividef(kXMax, amax) : kXMax / kTiny;
+    // Below kTiny the quotient would overflow: a fixed step instead, so there a block has the fewer bits the smaller it is.
+    // (A true division: __fdividef gives 0 for divisors above 2^126.)
+    constexpr float kTiny = 9.6e-35f;
+    const float inv = amax >= kTiny ? kXMax / amax : kXMax / kTiny;
     uint32_t h[2], l[2];
     int hs = 0, ls = 0;
 #pragma unroll

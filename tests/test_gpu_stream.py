@@ -34,6 +34,28 @@ def test_rows_and_chunks_of_every_length(backend, orc, qt, m, n, k):
     assert orc.within_tolerance(y.cpu().numpy(), ref, REL)[0]
 
 
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("peak,weight", [(2e-34, 1.0), (1e-33, 1.0), (9e37, 0.005), (1e38, 0.005), (2e38, 0.005), (2.9e38, 0.005)])
+@pytest.mark.parametrize("m", [1, 2])
+def test_blocks_of_extreme_size(backend, orc, qt, peak, weight, m):
+    """Every 32-element block's largest magnitude is `peak`: near the ends of what the fixed-point step's quotient can hold.
+    Calls, and a plan of two jobs (activations converted by a launch of their own), fp32 and bf16."""
+    n, k = 70, 1024
+    p = orc.quantize(qt, np.random.default_rng(qt).standard_normal((n, k), dtype=np.float32) * np.float32(weight))
+    w = backend.upload(qt, p, n, k)
+    rng = np.random.default_rng(9)
+    x = rng.uniform(-1, 1, (m, k)).astype(np.float32)
+    x[:, ::32] = rng.choice(np.float32([-1, 1]), (m, k // 32))
+    x = torch.from_numpy(x * np.float32(peak)).cuda()
+    for a in (x, x.to(torch.bfloat16)):
+        y, y1, y2 = backend.project(w, a), torch.zeros((m, n), device="cuda"), torch.zeros((m, n), device="cuda")
+        plan = backend.plan([([w], a, [y1]), ([w], a, [y2])])
+        plan.run()
+        backend.sync()
+        assert orc.within_tolerance(y.cpu().numpy(), orc.matmul_exact(qt, p, n, k, a.float().cpu().numpy()), REL)[0]
+        assert torch.equal(y1, y) and torch.equal(y2, y)
+
+
 @pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K, mb.TYPE_Q8_0])
 @pytest.mark.parametrize("m", [1, 2])
 def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
