@@ -831,9 +831,9 @@ cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStrea
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    // (Launches whose jobs wait for one another start early, too: a following launch's blocks only come in once every
-    // block of this one runs, so they never take the place of a block that others wait for.)
-    cfg.numAttrs = a.pdl ? 1 : 0;
+    // A launch whose jobs wait for one another holds its SMs until all its blocks run.  Started early it could share them with
+    // such a launch of another stream, each holding what the other lacks, so it starts when the launch before has ended.
+    cfg.numAttrs = (a.pdl && !p.has_dep) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, p);
 }
 

@@ -1,5 +1,6 @@
 """The streaming kernel's rules: ring sizes (and with them the number of teams), row quads that are not full, last chunks
 of every length, parts of the grid for plans of small products.  A result never depends on any of them."""
+import ctypes
 import os
 
 import numpy as np
@@ -110,3 +111,24 @@ def test_plans_of_small_products_share_the_grid(backend, orc, m):
             backend.sync()
             for a, b in zip(outs, want):
                 assert torch.equal(a, b)
+
+
+def _edge_types(graph):
+    """Types of a captured graph's edges: 0 ordinary, 1 programmatic (the later launch may start before the earlier has ended)."""
+    cu, count = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t(8)
+    nodes, data = (ctypes.c_void_p * 8)(), (ctypes.c_uint8 * 64)()
+    assert cu.cuGraphGetEdges_v2(ctypes.c_void_p(graph.raw_cuda_graph()), nodes, (ctypes.c_void_p * 8)(), data, ctypes.byref(count)) == 0
+    return [data[8 * i + 2] for i in range(count.value)]
+
+
+def test_only_independent_plans_start_before_the_launch_before_has_ended(backend, orc):
+    """A launch whose jobs wait holds SMs until all its blocks run, so it may not come in beside another stream's."""
+    n, k = 64, 512
+    w = backend.upload(mb.TYPE_Q4_K, _weights(orc, mb.TYPE_Q4_K, n, k, 1), n, k)
+    x, y = _acts(1, k, 2), [torch.zeros((1, n), device="cuda") for _ in range(2)]
+    for waits in (False, True):
+        plan = backend.plan([([w], x, [y[0]]), ([w], x, [y[1]])], waits=[False, waits])
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            plan.run()
+        assert _edge_types(graph) == [0 if waits else 1]       # activation preparation -> products
