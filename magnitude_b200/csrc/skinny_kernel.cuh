@@ -357,7 +357,6 @@ template <int NT, int P> struct SkRecordSub16 {              // Q6_K: levels 0..
             d[i] = half_bits_to_float(dv);
             const uint32_t s0 = (t < 2 ? sc[i].x : sc[i].y) >> (16 * (t & 1)), s1 = (t < 2 ? sc[i].z : sc[i].w) >> (16 * (t & 1));
             // byte under 0x64 reads 1024 + 128 + scale
-            d[i] *= 1048576.f;                   // 2^24 / 16
             put(am, i, hadd(__byte_perm(s0, 0x64646464u, 0x4140), 0xE480E480u), hadd(__byte_perm(s1, 0x64646464u, 0x4140), 0xE480E480u));
         }
         float e[NT][4];
@@ -398,10 +397,12 @@ template <int NT, int P> struct SkRecordSub16 {              // Q6_K: levels 0..
             mma0(x, am, bh.x, bh.y);
             mma(x, am, bl.x, bl.y);
             SkAcc<NT>(&a)[4] = acc[nt];
-            a[0] += d[0] * i0 * fmaf(-32.f / 1048576.f, x[0], e[nt][0]);
-            a[1] += d[0] * i1 * fmaf(-32.f / 1048576.f, x[1], e[nt][1]);
-            a[2] += d[1] * i0 * fmaf(-32.f / 1048576.f, x[2], e[nt][2]);
-            a[3] += d[1] * i1 * fmaf(-32.f / 1048576.f, x[3], e[nt][3]);
+            // 2^24 / 16 = 2^20 with the sums and 1 / scale last: in another order a factor may leave fp32's range where the product
+            // does not
+            a[0] += d[0] * fmaf(1048576.f, e[nt][0], -32.f * x[0]) * i0;
+            a[1] += d[0] * fmaf(1048576.f, e[nt][1], -32.f * x[1]) * i1;
+            a[2] += d[1] * fmaf(1048576.f, e[nt][2], -32.f * x[2]) * i0;
+            a[3] += d[1] * fmaf(1048576.f, e[nt][3], -32.f * x[3]) * i1;
         }
     }
 };

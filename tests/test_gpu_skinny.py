@@ -234,3 +234,28 @@ def test_skinny_scaled_sums_are_exact(backend, orc, qt, size, dtype, m, n, k):
     ref = orc.matmul_exact(qt, packed, n, k, x.float().cpu().numpy())
     bound = 64 * 2.0**-24 * top * x.float().abs().sum(1, keepdim=True).cpu().numpy()
     assert (np.abs(y.cpu().numpy() - ref) <= bound).all()
+
+
+@pytest.mark.parametrize("qt", TYPES)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [3, 16])
+@pytest.mark.parametrize("peak", [2.0**-100, 2.0**123])
+def test_skinny_activations_of_extreme_size(backend, orc, qt, dtype, m, peak):
+    """Records whose largest activation is far from 1, weights of order 0.1 to 1 with a large d: every factor of the result is
+    applied in an order that keeps what lies between in range."""
+    n, k = 40, 512
+    if qt == mb.TYPE_Q6_K:                            # scales -1..1, d = 2^-6: |w| <= 0.5
+        rng = np.random.default_rng(5)
+        blocks = rng.integers(0, 256, (n * k // 256, 210), dtype=np.uint8)
+        blocks[:, 192:208] = rng.integers(-1, 2, (len(blocks), 16), dtype=np.int8).view(np.uint8)
+        blocks[:, 208:210] = np.full(1, 2.0**-6, np.float16).view(np.uint8)
+        packed = blocks.reshape(n, -1)
+    else:
+        packed = orc.quantize(qt, np.random.default_rng(qt).standard_normal((n, k), dtype=np.float32) * np.float32(0.25))
+    x = (_acts(m, k, seed=m, dtype=torch.float32).clamp(-2, 2) * (peak / 2)).to(dtype)
+    y = backend.project(backend.upload(qt, packed, n, k), x)
+    assert backend.last_route()[0] == mb.ROUTE_SKINNY
+    backend.sync()
+    ref = orc.matmul_exact(qt, packed, n, k, x.float().cpu().numpy())
+    ok, worst = orc.within_tolerance(y.cpu().numpy(), ref, REL_DECODE)
+    assert ok, f"worst error {worst:.3f} x tolerance"
