@@ -28,7 +28,7 @@ template <int MAP, int N> __global__ void __launch_bounds__(128) skinny_prep_ker
     const SkJob &J = jobs[ji];
     const int rec = (wid - J.xwarp0) / J.M, tok = (wid - J.xwarp0) - rec * J.M;
     pdl_wait();                          // X may come from the launch before, which may also still read the images
-    sk_make_image<MAP>(J, rec, tok, lane, J.img + (size_t)rec * sk_image_bytes(p.NT, p.P), p.NT, p.P);
+    sk_make_image<MAP>(J, rec, tok, lane, J.img + (size_t)rec * sk_image_bytes(p.NT, p.P, kSumBytes<MAP>), p.NT, p.P);
 }
 
 // box0 words of every row of `rows` weight rows, over the chunks [c0, c0 + nc)
@@ -70,7 +70,7 @@ cudaError_t skinny_ws_init(uint8_t *ws, size_t bytes, bool own_stream) {
 }
 
 static int planes(const SkinnyProduct &a) { return !a.x_is_bf16 && a.M <= skinny_max_m() ? 2 : 1; }
-size_t skinny_image_bytes(const SkinnyProduct &a) { return (size_t)(a.Kpad / SB) * sk_image_bytes(token_tiles(a.M), planes(a)); }
+size_t skinny_image_bytes(const SkinnyProduct &a) { return (size_t)(a.Kpad / SB) * sk_image_bytes(token_tiles(a.M), planes(a), sk_sum_bytes(a.qt, token_tiles(a.M))); }
 
 // A prepared call: the kernel parameters of `n` products of one block type and one M.  Built once (per call, or
 // per plan) on the host; launching it touches no host memory the caller could have freed.

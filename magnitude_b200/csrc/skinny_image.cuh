@@ -30,6 +30,7 @@ __host__ __device__ constexpr int sk_map(int qt, int nt) {
            : qt == QT_Q6_K                            ? (nt <= 2 ? SK_SUB16 : SK_Q6)
                                                       : SK_BLOCK;
 }
+template <int MAP> constexpr int kSumBytes = MAP == SK_SUB16 ? 512 : 256;      // of a token tile (sk_sum_bytes)
 template <int MAP> __device__ __forceinline__ void sk_unit(int L, int &u, int &t) {
     if (MAP == SK_K) {
         t = 2 * ((L >> 3) & 1) + ((L >> 1) & 1);
@@ -141,7 +142,7 @@ template <int MAP> __device__ __forceinline__ void sk_put_image(const float (&v)
             q[128] = xl;
         }
     }
-    if (lane == 0) *reinterpret_cast<uint32_t *>(xs + NT * 512 + tok * 4) = (uint32_t)(127 - e) << 23;
+    if (lane == 0) *reinterpret_cast<uint32_t *>(xs + NT * kSumBytes<MAP> + tok * 4) = (uint32_t)(127 - e) << 23;
 }
 
 template <int MAP> __device__ __forceinline__ void sk_make_image(const SkJob &J, int rec, int tok, int lane, uint8_t *img, int NT, int P) {

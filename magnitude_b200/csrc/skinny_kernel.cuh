@@ -57,8 +57,9 @@ template <int QT, int NT, int P> struct SkShape {
     static constexpr int kRows = sk_tile_rows(NT);
     static constexpr int kW = sk_w_bytes(QT, NT), kD = sk_d_bytes(QT, NT);
     static constexpr int kB = P * NT * 4096;                       // image: activation fragments of 256 weights,
-    static constexpr int kX = NT * 512;                            // Q4_K / Q5_K / Q6_K: sub-block sums, as fragments,
-    static constexpr int kImg = sk_image_bytes(NT, P);             // and per token 1 / scale
+    static constexpr int kX = NT * sk_sum_bytes(QT, NT);           // Q4_K / Q5_K / Q6_K: sub-block sums, as fragments,
+    static constexpr int kImg = sk_image_bytes(NT, P, sk_sum_bytes(QT, NT));      // and per token 1 / scale
+    static_assert(kSumBytes<sk_map(QT, NT)> == sk_sum_bytes(QT, NT), "sums");
     static constexpr int kStage = sk_stage_bytes(QT, NT, P), kHead = kSkHeadBytes, kDepth = sk_depth(QT, NT, P);
     static_assert(kDepth >= 2, "stages");
 };

@@ -19,15 +19,16 @@ __host__ __device__ inline int sk_slot_begin(int slots, int grid, int b) { retur
 // the block that a slot belongs to
 __host__ __device__ inline int sk_slot_owner(int slots, int grid, int s) { return (int)((((long long)s + 1) * grid - 1) / slots); }
 // activation image of one record: fragments [plane][token tile][unit 8][lane 32] x 16 bytes, block-sum fragments
-// [token tile][lane 32] x 8 bytes, one or (Q6_K) two, 1 / scale [token] x 4 bytes
-__host__ __device__ constexpr int sk_image_bytes(int nt, int planes) { return nt * (planes * 4096 + 512 + 32); }
+// [token tile][one, Q6_K up to 16 tokens two][lane 32] x 8 bytes, 1 / scale [token] x 4 bytes
+__host__ __device__ constexpr int sk_sum_bytes(int qt, int nt) { return qt == QT_Q6_K && nt <= 2 ? 512 : 256; }
+__host__ __device__ constexpr int sk_image_bytes(int nt, int planes, int sum_bytes) { return nt * (planes * 4096 + sum_bytes + 32); }
 
 // shared memory: a stage holds a slot's packed records (Q6_K: and its rows' 16-byte groups of fp16 d) and the record's image
 constexpr int kSkHeadBytes = 256, kSkMaxDepth = 8;
 __host__ __device__ constexpr int sk_w_bytes(int qt, int nt) { return sk_tile_rows(nt) * rec_bytes(qt); }
 __host__ __device__ constexpr int sk_d_bytes(int qt, int nt) { return qt == QT_Q6_K ? sk_tile_rows(nt) * 16 : 0; }
 __host__ __device__ constexpr int sk_stage_bytes(int qt, int nt, int planes) {
-    return (sk_w_bytes(qt, nt) + sk_d_bytes(qt, nt) + sk_image_bytes(nt, planes) + 127) / 128 * 128;
+    return (sk_w_bytes(qt, nt) + sk_d_bytes(qt, nt) + sk_image_bytes(nt, planes, sk_sum_bytes(qt, nt)) + 127) / 128 * 128;
 }
 __host__ __device__ constexpr int sk_depth(int qt, int nt, int planes) {
     return (232448 - kSkHeadBytes) / sk_stage_bytes(qt, nt, planes) < kSkMaxDepth ? (232448 - kSkHeadBytes) / sk_stage_bytes(qt, nt, planes) : kSkMaxDepth;
