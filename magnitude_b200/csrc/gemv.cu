@@ -52,7 +52,8 @@ constexpr int kThreads = kConsumers + kProducers * 32;
 // Five warps per scheduler leave 96 registers a thread; the producers give up most of theirs
 constexpr int kLaunchRegs = 96, kConsumerRegs = 112, kProducerRegs = 32;
 static_assert(kConsumers * kConsumerRegs + kProducers * 32 * kProducerRegs <= kThreads * kLaunchRegs, "register split");
-// What the partial sums of a section (the quads between two final passes) may take; they are there twice.  A pass takes
+// What the partial sums of a section (the quads between two final passes) may take; they are there twice, unless that leaves no
+// room for a slot (one short row of 84992 Q4_K weights needs all 227 KB: the warps then meet after each final pass).  A pass takes
 // about 2000 cycles with its meeting (25600 x 5120 Q4_K, eleven quads: 5570 GB/s in sections of five, 5890 in one), but the
 // ring comes first: a launch takes the largest of these sizes that leaves six slots (5120 x 25600 Q6_K beside a 61 KB
 // image: 4380 GB/s with five slots, 4660 with six).
@@ -68,7 +69,8 @@ struct StreamParams {
     int jobs_bytes;          // shared-memory bytes of the job table
     int x_bytes;             // ... of one activation image area
     int x_bufs;              // 1 or 2 areas
-    int partial_floats;      // size of one copy of a section's partial sums
+    int partial_floats;      // from one copy of a section's partial sums to the other; 0: there is one
+    int ring;                // the ring's place in shared memory
     int slots, slot_bytes;   // ring slots; bytes of one (the largest of the launch's jobs)
     int turn;                // producers and consumer teams at work
     int has_dep;             // some job waits for earlier jobs: CTAs count completions
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
     uint8_t *ximg0 = zero_area + kZeroBytes + p.jobs_bytes;
     float *partial0 = reinterpret_cast<float *>(ximg0 + p.x_bufs * p.x_bytes);      // two copies: [quad][m][row][chunk][wr]
     const int partial_floats = p.partial_floats;
-    const uint32_t ring = smem_u32(partial0 + 2 * partial_floats);
+    const uint32_t ring = smem_u32(smem) + p.ring;
     volatile int *fail_flag = &head.fail;
 
     if (threadIdx.x < kSlots) {
@@ -689,6 +691,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
                     }
                 }
             }
+            if (partial_floats == 0) consumers_sync();
             q0 = q1;
         } while (q0 < nquads);
         if (xsum) {
@@ -775,14 +778,16 @@ size_t section_bytes(const StreamJob &J, int M, int quads) { return ((size_t)qua
 // shared memory of a launch: the largest activation image and ring slot over its jobs
 struct Fit {
     size_t x_bytes = 0, slot = 0, jobs_bytes, partial, limit;
+    int copies = 2;          // of the partial sums
     Fit(const StreamJob *jobs, int n, int M, size_t smem_limit, size_t partial_bytes) : partial(partial_bytes), limit(smem_limit) {
         for (int i = 0; i < n; ++i) {
             x_bytes = std::max(x_bytes, ((size_t)M * jobs[i].nsb * ximg_rec_bytes(jobs[i].qt) + 127) & ~size_t(127));
             slot = std::max(slot, (size_t)jobs[i].slot_bytes);
         }
         jobs_bytes = ((size_t)n * sizeof(StreamJob) + 127) & ~size_t(127);
+        if (slots(1) < 1) copies = 1;
     }
-    size_t fixed(int bufs) const { return kHeadBytes + kZeroBytes + jobs_bytes + bufs * x_bytes + 2 * partial; }
+    size_t fixed(int bufs) const { return kHeadBytes + kZeroBytes + jobs_bytes + bufs * x_bytes + copies * partial; }
     int slots(int bufs) const { return fixed(bufs) > limit ? 0 : (int)std::min<size_t>(kSlots, (limit - fixed(bufs)) / slot); }
 };
 
@@ -798,7 +803,7 @@ cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStrea
     const Fit fit(a.jobs_host, a.njobs, MT, a.smem_limit, partial);
     p.x_bytes = (int)fit.x_bytes;
     p.jobs_bytes = (int)fit.jobs_bytes;
-    p.partial_floats = (int)(partial / 4);
+    p.partial_floats = fit.copies == 2 ? (int)(partial / 4) : 0;
     p.slot_bytes = (int)fit.slot;
     // Two slots for each team at work, so that one is filled while the other is read: four teams of eight slots and more,
     // three of six, two of less (27 KB slots of Q6_K: four slots 4.4 TB/s with two teams, 4.2 with four)
@@ -809,7 +814,8 @@ cudaError_t launch_t(const StreamLaunch &a, StreamParams &p, int grid, cudaStrea
     p.slots = usable(p.x_bufs);
     p.turn = turn_of(p.slots);
     if (p.slots < 1) return cudaErrorInvalidValue;
-    const size_t smem = fit.fixed(p.x_bufs) + p.slots * fit.slot;
+    p.ring = (int)fit.fixed(p.x_bufs);
+    const size_t smem = p.ring + p.slots * fit.slot;
 
     auto kern = stream_kernel<MT, VAR>;
     static std::atomic<size_t> configured{0};   // per instantiation; a context on another device re-sets it
@@ -972,11 +978,12 @@ void stream_fit_jobs(StreamJob *jobs, int n, int M, int grid, size_t smem_limit)
     for (int j0 = 0; j0 < n; j0 += kMaxJobsPerLaunch) deal_small_jobs(jobs + j0, std::min(kMaxJobsPerLaunch, n - j0), grid);
     for (int j0 = 0; j0 < n; j0 += kMaxJobsPerLaunch) {
         const int nj = std::min(kMaxJobsPerLaunch, n - j0);
-        int best = -1, best_rank = -1;
+        int best = 1, best_rank = 0;
         for (int b : kSectionBytes) {
             size_t partial = 0;
             for (int i = 0; i < nj; ++i) partial = std::max(partial, section_bytes(jobs[j0 + i], M, section_quads(jobs[j0 + i], M, b)));
-            const int s = std::max(0, Fit(jobs + j0, nj, M, smem_limit, partial).slots(1));
+            const Fit fit(jobs + j0, nj, M, smem_limit, partial);
+            const int s = fit.copies == 2 ? fit.slots(1) : 0;
             const int rank = s >= 6 ? 6 : s >= 2 ? 2 : s;
             if (rank > best_rank) {
                 best = b;

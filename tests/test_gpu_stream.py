@@ -60,31 +60,44 @@ def test_blocks_of_extreme_size(backend, orc, qt, peak, weight, m):
 @pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K, mb.TYPE_Q8_0])
 @pytest.mark.parametrize("m", [1, 2])
 def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
-    """One slot (one team), two, four, six (three teams) and more, alone and in a plan of jobs that wait."""
-    n, k = 5000, 256 * 21
+    """From all of the shared memory down to what is refused, in steps smaller than a slot and then smaller than a copy of the
+    partial sums: every number of slots and teams down to one, and one copy of the sums.  Two to three row quads a block, a
+    final pass after each; calls, plans of independent jobs and of jobs that wait."""
+    n, k = 3000, 256 * 65
     p, p2 = _weights(orc, qt, n, k, 1), _weights(orc, qt, 300, 2304, 2)
     x, x2 = _acts(m, k, 5), _acts(m, 2304, 6)
-    ref = None
-    slot = {mb.TYPE_Q4_K: 18688, mb.TYPE_Q6_K: 27008, mb.TYPE_Q8_0: 34880}[qt]
-    for slots in (None, 1, 2, 3, 4, 6):
-        if slots:
-            os.environ["B200Q_GEMV_SMEM"] = str(min(232448, 2000 + 21 * 608 * m + 2 * 16 * 16 * m * 3 * 3 + slots * slot + 6000))
+    ref, limit, step, accepted = None, 232448, 8192, 0
+    while True:
+        os.environ["B200Q_GEMV_SMEM"] = str(limit)
         be = mb.Backend(0)
         os.environ.pop("B200Q_GEMV_SMEM", None)
         w, w2 = be.upload(qt, p, n, k), be.upload(qt, p2, 300, 2304)
-        out = [be.project(w, x), torch.zeros((m, n), device="cuda"), torch.zeros((m, 300), device="cuda"), torch.zeros((m, n), device="cuda")]
-        plan = be.plan([([w], x, out[1:2]), ([w2], x2, out[2:3]), ([w], x, out[3:4])], waits=[False, True, True])
-        for _ in range(2):
-            plan.run()
-        be.sync()
+        out = [torch.zeros((m, n), device="cuda") for _ in range(3)] + [torch.zeros((m, 300), device="cuda") for _ in range(2)]
+        try:
+            out.append(be.project(w, x))
+            for o, waits in ((out[0:2] + out[3:4], [False, True, True]), ([out[2], torch.zeros_like(out[2]), out[4]], None)):
+                plan = be.plan([([w], x, o[:1]), ([w2], x2, o[2:]), ([w], x, o[1:2])], waits=waits)
+                for _ in range(2):
+                    plan.run()
+                be.sync()
+                assert torch.equal(o[0], o[1])
+        except mb.B200QError:
+            be.close()
+            if step == 1024:
+                break
+            limit, step = limit + step - 1024, 1024
+            continue
         if ref is None:
             ref = out
             assert orc.within_tolerance(out[0].cpu().numpy(), orc.matmul_exact(qt, p, n, k, x.float().cpu().numpy()), REL)[0]
-            assert orc.within_tolerance(out[2].cpu().numpy(), orc.matmul_exact(qt, p2, 300, 2304, x2.float().cpu().numpy()), REL)[0]
+            assert orc.within_tolerance(out[3].cpu().numpy(), orc.matmul_exact(qt, p2, 300, 2304, x2.float().cpu().numpy()), REL)[0]
         for a, b in zip(out, ref):
-            assert torch.equal(a, b), slots
-        assert torch.equal(out[1], out[0]) and torch.equal(out[3], out[0])
+            assert torch.equal(a, b), limit
+        assert torch.equal(out[0], out[2]) and torch.equal(out[0], out[5]) and torch.equal(out[3], out[4])
         be.close()
+        accepted += 1
+        limit -= step
+    assert step == 1024 and accepted >= 8
 
 
 @pytest.mark.parametrize("m", [1, 2])
@@ -111,6 +124,26 @@ def test_plans_of_small_products_share_the_grid(backend, orc, m):
             backend.sync()
             for a, b in zip(outs, want):
                 assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q4_0, mb.TYPE_MXFP4])
+@pytest.mark.parametrize("m,k", [(1, 84992), (2, 42496), (4, 21248)])
+def test_rows_that_fill_the_shared_memory(backend, orc, qt, m, k):
+    """The longest activations that fit beside one ring slot, where the partial sums have one copy: calls, and jobs that wait and
+    add to what is there."""
+    n = 41 * 4 + 3
+    p = _weights(orc, qt, n, k, 4)
+    w, x = backend.upload(qt, p, n, k), _acts(m, k, 7)
+    ref = orc.matmul_exact(qt, p, n, k, x.float().cpu().numpy())
+    if m <= 2:
+        y = backend.project(w, x)
+        backend.sync()
+        assert orc.within_tolerance(y.cpu().numpy(), ref, REL)[0]
+    y = torch.zeros((m, n), device="cuda")
+    plan = backend.plan([([w], x, [y])] * 2, waits=[False, True], accumulate=[True, True])
+    plan.run()
+    backend.sync()
+    assert orc.within_tolerance(y.cpu().numpy(), 2 * ref, REL)[0]
 
 
 def _edge_types(graph):
