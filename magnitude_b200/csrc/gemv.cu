@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
                         for (int spin = 1; !mbar_try_wait(ebar, (uses - 1) & 1); ++spin) {
                             if (*fail_flag) ok = false;
                             if ((spin & 63) == 0) {
+                                if (t0 == 0) pdl_wait();       // (the consumers stand there until the launch before has ended)
                                 const uint64_t now = globaltimer_ns();
                                 if (t0 == 0) t0 = now;
                                 else if (now - t0 > kWaitLimitNs) {

@@ -2,6 +2,9 @@
 stays usable.  The wait is made to run out on the host's terms (a peer that never posts: the second
 "rank" is a context that simply does not call), with the wait limit set to 50 ms; nothing faults,
 traps or hangs.  One GPU: the two contexts live on the same device and only one of them launches."""
+import ctypes
+import time
+
 import numpy as np
 import pytest
 
@@ -49,6 +52,73 @@ def test_peer_exchange_times_out_and_the_context_survives(orc):
         a.set_option(B.OPT_WAIT_LIMIT_MS, 2000)
         a.close()
         b.close()
+
+
+def _sharded(be, qt, n, k, rank, m):
+    """Rank `rank` of two's half of a row-parallel product: weight and activations."""
+    rng = np.random.default_rng(10 * rank + qt)
+    w = be.upload(qt, gq.synth_weights(qt, n, k, 3 + rank), n, k)
+    return w, torch.from_numpy(rng.standard_normal((m, k), dtype=np.float32)).cuda().to(torch.bfloat16)
+
+
+def _words(cu, base):
+    """A device buffer's 64-bit words: (address, words)."""
+    start, size = ctypes.c_uint64(), ctypes.c_size_t()
+    assert cu.cuMemGetAddressRange_v2(ctypes.byref(start), ctypes.byref(size), ctypes.c_uint64(base)) == 0
+    out = np.zeros(size.value // 8, np.uint64)
+    assert cu.cuMemcpyDtoH_v2(out.ctypes.data_as(ctypes.c_void_p), start, ctypes.c_size_t(size.value)) == 0
+    return start.value, out
+
+
+def test_waiting_for_the_launch_before_has_no_limit(orc):
+    """A launch that starts early stands idle until the one before has ended, however long that takes: here its two waits for a
+    peer, each within the limit, together beyond it.  The peer's shares are copied into the buffer by the host."""
+    n, k, m = 4, 1024, 1
+    cu = ctypes.CDLL("libcuda.so.1")
+    a, b, c = mb.Backend(0), mb.Backend(0), mb.Backend(0)
+    try:
+        bufs = [a.peer_buffer(), b.peer_buffer()]
+        plans, outs, own = [], [], []
+        for r, be in enumerate((a, b)):
+            jobs = [_sharded(be, mb.TYPE_Q4_K, n, k, r + 2 * i, m) for i in range(2)]
+            own.append([be.project(w, x) for w, x in jobs])
+            be.sync()
+            outs.append([torch.zeros((m, n), device="cuda") for _ in range(2)])
+            plans.append(be.plan([([w], x, [o]) for (w, x), o in zip(jobs, outs[r])], sum_ranks=[True, True]))
+            be.peer_attach_buffers(r, 2, bufs)
+        big, xb = _sharded(c, mb.TYPE_Q4_K, 8192, 8192, 5, m)      # more than a ring holds, so that its producers wait
+        want, got = c.project(big, xb), torch.zeros((m, 8192), device="cuda")
+        c.sync()
+        # rank 1 alone: its shares of exchanges 1 and 2 land in rank 0's buffer, its own wait runs out
+        a.set_option(B.OPT_WAIT_LIMIT_MS, 50)
+        plans[1].run()
+        with pytest.raises(mb.B200QError):
+            b.sync()
+        base, words = _words(cu, bufs[0])
+        assert cu.cuMemsetD8_v2(ctypes.c_uint64(base), ctypes.c_ubyte(0), ctypes.c_size_t(8 * len(words))) == 0
+        a.set_option(B.OPT_WAIT_LIMIT_MS, 400)
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        plans[0].run(stream=stream)
+        c.project(big, xb, out=got, stream=stream)
+        for exchange in (1, 2):
+            time.sleep(0.25)
+            shares = np.flatnonzero(words >> np.uint64(32) == exchange)
+            assert len(shares) == m * n
+            for i in shares:
+                word = words[i:i + 1]
+                assert cu.cuMemcpyHtoD_v2(ctypes.c_uint64(base + 8 * int(i)), word.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(8)) == 0
+        a.sync(stream)
+        c.sync(stream)
+        assert torch.equal(got, want)
+        for o, y0, y1 in zip(outs[0], *own):
+            assert torch.equal(o, y0 + y1)
+        a.peer_detach()
+        b.peer_detach()
+    finally:
+        a.set_option(B.OPT_WAIT_LIMIT_MS, 2000)
+        for be in (a, b, c):
+            be.close()
 
 
 def test_option_ranges(backend):
