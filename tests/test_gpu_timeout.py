@@ -61,6 +61,54 @@ def _sharded(be, qt, n, k, rank, m):
     return w, torch.from_numpy(rng.standard_normal((m, k), dtype=np.float32)).cuda().to(torch.bfloat16)
 
 
+@pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q6_K])
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("waits", [False, True])
+def test_plan_sums_of_two_ranks_one_after_the_other(qt, m, waits):
+    """Both ranks of a plan that sums inside its launch, on one GPU and one at a time.  Rank 1 posts its shares and its waits for
+    rank 0 run out: Timeout.  Rank 0 then finds rank 1's shares in its buffer and ends with the sums, in rank order.  After the
+    failure rank 1's plan, alone in the world, gives its own products again, run after run: a plan whose jobs wait finds its
+    completion counter at zero."""
+    n, n2, k = 200, 3000, 1024
+    ranks = [mb.Backend(0), mb.Backend(0)]
+    try:
+        bufs = [be.peer_buffer() for be in ranks]
+        plans, outs, own = [], [], []
+        for r, be in enumerate(ranks):
+            w, x = _sharded(be, qt, n, k, r, m)
+            w2, x2 = _sharded(be, qt, n2, k, r + 2, m)
+            own.append([be.project(w, x), be.project(w2, x2)])
+            be.sync()
+            outs.append([torch.zeros((m, n), device="cuda"), torch.zeros((m, n2), device="cuda")])
+            plans.append(be.plan([([w], x, outs[r][:1]), ([w2], x2, outs[r][1:])], waits=[False, waits], sum_ranks=[True, True]))
+            be.peer_attach_buffers(r, 2, bufs)
+        ranks[0].set_option(B.OPT_WAIT_LIMIT_MS, 50)
+        plans[1].run()
+        with pytest.raises(mb.B200QError) as e:
+            ranks[1].sync()
+        assert e.value.status == B.ERR_TIMEOUT
+        # (where jobs wait, the blocks that gave up first leave later jobs out: their shares may be missing)
+        if not waits:
+            plans[0].run()
+            ranks[0].sync()
+            for got, a, b in zip(outs[0], *own):
+                assert torch.equal(got, a + b)
+        for r, be in enumerate(ranks):
+            be.peer_detach()
+        for r in (1, 0):
+            for _ in range(3):
+                for o in outs[r]:
+                    o.zero_()
+                plans[r].run()
+                ranks[r].sync()
+                for got, want in zip(outs[r], own[r]):
+                    assert torch.equal(got, want)
+    finally:
+        ranks[0].set_option(B.OPT_WAIT_LIMIT_MS, 2000)
+        for be in ranks:
+            be.close()
+
+
 def _words(cu, base):
     """A device buffer's 64-bit words: (address, words)."""
     start, size = ctypes.c_uint64(), ctypes.c_size_t()
