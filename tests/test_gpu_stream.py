@@ -102,7 +102,8 @@ def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
 
 @pytest.mark.parametrize("m", [1, 2])
 def test_plans_of_small_products_share_the_grid(backend, orc, m):
-    """Products of few rows run on halves and quarters of the grid, beside a large one and a SWIGLU job; three runs alike."""
+    """Products of few rows run on halves and quarters of the grid, beside a large one and a SWIGLU job; three runs alike.
+    (Which part a job gets: test_stream_rules.py.)"""
     shapes = [(mb.TYPE_Q4_K, 512, 1024), (mb.TYPE_Q4_K, 1000, 4096), (mb.TYPE_Q6_K, 37, 512), (mb.TYPE_Q8_0, 4096, 4096), (mb.TYPE_Q4_K, 14336, 4096)]
     shapes = (shapes * 5)[:23]
     jobs, outs, want = [], [], []
@@ -113,17 +114,20 @@ def test_plans_of_small_products_share_the_grid(backend, orc, m):
         jobs.append(([w], x, [y]))
         outs.append(y)
         want.append(backend.project(w, x))
-    g, u = jobs[0][0][0], jobs[5][0][0]
+    g, u = jobs[0][0][0], backend.upload(mb.TYPE_Q4_K, _weights(orc, mb.TYPE_Q4_K, 512, 1024, 99), 512, 1024)
     act = torch.zeros((m, 512), device="cuda")
+    gate, up = want[0].double(), backend.project(u, jobs[0][1]).double()
     for extra in (False, True):
         plan = backend.plan(jobs + ([([g, u], jobs[0][1], [act])] if extra else []), **({"swiglu": [False] * len(jobs) + [True]} if extra else {}))
         for _ in range(3):
-            for y in outs:
+            for y in outs + [act]:
                 y.zero_()
             plan.run()
             backend.sync()
             for a, b in zip(outs, want):
                 assert torch.equal(a, b)
+            if extra:       # the quick exponential: a few units in the last place, and a division and a product
+                assert torch.allclose(act.double(), gate / (1 + torch.exp(-gate)) * up, rtol=2e-6, atol=1e-12)
 
 
 @pytest.mark.parametrize("qt", [mb.TYPE_Q4_K, mb.TYPE_Q4_0, mb.TYPE_MXFP4])
