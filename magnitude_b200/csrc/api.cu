@@ -116,7 +116,7 @@ struct b200q_ctx {
     uint64_t tp_timeout_ms = 60000;   // host deadline of b200q_tp_init
     bool peer_stale = false;          // a peer exchange timed out: the ranks' call counters no longer agree
     bool peer_ipc = true;             // peer buffers were mapped through CUDA IPC (else given as pointers)
-    int skinny_min_m = 3;             // smallest M that takes the skinny route (smaller batches: the dp4a kernel)
+    int skinny_min_m = 3;             // smallest M that takes the skinny route (smaller batches: the streaming kernel)
     int mid_max_m = 48;               // largest M that runs on the small-batch kernels (17 and more rows)
     int gemm_bn = 0, gemm_debug = 0, gemm_pair = 0, gemm_ksplit = 1, gemm_dense = -1;
     // tunables (environment overrides for experiments)

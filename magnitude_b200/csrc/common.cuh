@@ -76,11 +76,6 @@ __host__ __device__ inline int64_t chunk_row_bytes(int qt, int64_t c, int64_t ns
     const int64_t sb1 = (c + 1) * kChunkRecs < nsb ? (c + 1) * kChunkRecs : nsb;
     return range_bytes(qt, c * kChunkRecs, sb1, nsb);
 }
-// rows of row group g that exist in an N-row tensor (the rest of the group is zero padding)
-__host__ __device__ inline int group_rows(int64_t g, int64_t N) {
-    const int64_t left = N - g * kRowGroup;
-    return left < kRowGroup ? (int)left : kRowGroup;
-}
 // rows a tensor of N rows occupies in device memory
 __host__ __device__ inline int64_t padded_rows(int64_t N) { return (N + kRowGroup - 1) / kRowGroup * kRowGroup; }
 // byte offset of tile (row group g, chunk c) from the start of the tensor

@@ -274,8 +274,9 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
     const int turn = p.turn;
 
     // =========================================================================================
-    // Producer warps: warp i copies slots i, i + 4, ... of all jobs, lane j of it tile j.  (A slot's wait, address
-    // arithmetic and copies are a chain of 700 to 1300 cycles, as long as HBM takes for one slot, so four warps share them.)
+    // Producer warps: warp i of the `turn` at work copies slots i, i + turn, ... of all jobs, lane j of it tile j.  (A slot's
+    // wait, address arithmetic and copies are a chain of 700 to 1300 cycles, as long as HBM takes for one slot, so up to four
+    // warps share them.)
     // =========================================================================================
     if (warp >= kWarps) {
         setmaxnreg_dec<kProducerRegs>();

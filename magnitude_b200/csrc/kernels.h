@@ -198,9 +198,9 @@ constexpr size_t kPeerSlotBytes = size_t(kPeerSlotFloats) * 8;
 constexpr size_t kPeerRegionSlots = size_t(2) * kPeerMaxWorld * kPeerSlotBytes;      // 2 MB
 constexpr size_t kPeerEpochOff = 0;                    // [kPeerBlocks] u32
 constexpr size_t kPeerSlotOff = 4096;
-constexpr size_t kPeerFusedEpochOff = kPeerSlotOff + kPeerRegionSlots;               // [2 teams][kPeerCtas] u32
-constexpr size_t kPeerFusedSlotOff = kPeerFusedEpochOff + 4096;                      // [2 teams][2 sets][ranks][elements]
-constexpr size_t kPeerBufferBytes = kPeerFusedSlotOff + 2 * kPeerRegionSlots;
+constexpr size_t kPeerFusedEpochOff = kPeerSlotOff + kPeerRegionSlots;               // [kPeerCtas] u32
+constexpr size_t kPeerFusedSlotOff = kPeerFusedEpochOff + 4096;                      // [2 sets][ranks][elements]
+constexpr size_t kPeerBufferBytes = kPeerFusedSlotOff + kPeerRegionSlots;
 struct PeerLaunch {
     float *y;                       // in place: partial sums in, sums over ranks out
     int count;

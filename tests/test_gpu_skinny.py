@@ -83,7 +83,7 @@ def test_skinny_q8_0_ragged_k(backend, orc):
 
 @pytest.mark.parametrize("qt", TYPES)
 def test_skinny_small_m_when_selected(backend, orc, qt):
-    # M = 2 normally takes the dp4a kernel; the context option moves it to this route (and back)
+    # M = 2 normally takes the streaming kernel; the context option moves it to this route (and back)
     n, k = 150, 3072
     packed = _weights(orc, qt, n, k, seed=5)
     w = backend.upload(qt, packed, n, k)
