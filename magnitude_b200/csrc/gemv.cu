@@ -150,8 +150,8 @@ struct Place {
 };
 
 // A consumer warp's part of a section: records wr and wr + 4 of the team's slots of quads q0..q1-1, the row sums into
-// the partial sums.  False if a wait ran out.
-template <int QT, int MT>
+// the partial sums.  False if a wait ran out.  HALF: no quad has more than two tiles, so no lane's second row exists.
+template <int QT, int MT, bool HALF>
 __device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLane &xl) {
     // The lane's two rows of a quad: row g / 2 of tiles (g & 1) and (g & 1) + 2, g = lane / 4.  Neighbouring lane
     // groups read different tiles, whose places in the slot are offset so that their 16-byte loads meet no bank twice.
@@ -190,16 +190,16 @@ __device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLan
             if (rec + 4 * k < t.nsb) {
                 WRec<QT> r0, r1;
                 r0.load(a + 4 * k * rec_bytes(QT), d + 8 * k, c4);
-                r1.load(a + 4 * k * rec_bytes(QT) + step, d + 8 * k + step, c4);
+                if (!HALF) r1.load(a + 4 * k * rec_bytes(QT) + step, d + 8 * k + step, c4);
                 if (k == 1 || rec + 4 >= t.nsb) give_back();       // everything is in registers
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     RecSums<QT> sums;
                     XScales<QT> xs;
-                    sums.run(r0, r1, xl, rec + 4 * k, m * t.img_bytes, c4);
+                    sums.template run<HALF>(r0, r1, xl, rec + 4 * k, m * t.img_bytes, c4);
                     xs.load(xl, rec + 4 * k, m * t.img_bytes, c4);
                     acc[0][m] += sums.finish(0, r0.s, xs, c4);
-                    acc[1][m] += sums.finish(1, r1.s, xs, c4);
+                    if (!HALF) acc[1][m] += sums.finish(1, r1.s, xs, c4);
                 }
             }
         }
@@ -218,9 +218,10 @@ __device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLan
         const uint32_t cell = cell0 + (q - t.q0) * quad_cells + 16 * c;
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
-            float v = (h ? acc[1][m] : acc[0][m]) + __shfl_xor_sync(0xFFFFFFFFu, h ? acc[0][m] : acc[1][m], 1);
+            const float mine = h && !HALF ? acc[1][m] : acc[0][m], other = h || HALF ? acc[0][m] : acc[1][m];
+            float v = mine + __shfl_xor_sync(0xFFFFFFFFu, other, 1);
             v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-            if (c4 < 2) sts32f(cell + m * 16 * row_cells, v);
+            if (c4 < (HALF ? 1 : 2)) sts32f(cell + m * 16 * row_cells, v);
         }
     }
     return true;
@@ -228,10 +229,11 @@ __device__ __forceinline__ bool section_dot(const Walk &t, Place &at, const XLan
 
 // VAR: which optional code the instantiation carries.  Bit 0: the fused epilogues (SWIGLU, ACCUM, norm on
 // the load) for launches that hold such jobs; bit 1: the rank-sum exchange, for launches of attached
-// tensor-parallel ranks.
+// tensor-parallel ranks; bit 2: launches that give no CTA more than two row groups (8 rows) of a job, where half of each MMA's
+// rows are not there: their unpacking and scaling is left out (see stream_launch_one).
 template <int MT, int VAR>
 __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_constant__ StreamParams p) {
-    constexpr bool FUSED = (VAR & 1) != 0, PEER = (VAR & 2) != 0;
+    constexpr bool FUSED = (VAR & 1) != 0, PEER = (VAR & 2) != 0, HALF = (VAR & 4) != 0;
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -603,12 +605,12 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
             t.partial = smem_u32(partial);
             t.fail = fail_flag;
             bool ok;
-            if (qt == QT_Q4_K) ok = section_dot<QT_Q4_K, MT>(t, at, xl);
-            else if (qt == QT_Q6_K) ok = section_dot<QT_Q6_K, MT>(t, at, xl);
-            else if (qt == QT_Q8_0) ok = section_dot<QT_Q8_0, MT>(t, at, xl);
-            else if (qt == QT_Q5_K) ok = section_dot<QT_Q5_K, MT>(t, at, xl);
-            else if (qt == QT_Q4_0) ok = section_dot<QT_Q4_0, MT>(t, at, xl);
-            else ok = section_dot<QT_MXFP4, MT>(t, at, xl);
+            if (qt == QT_Q4_K) ok = section_dot<QT_Q4_K, MT, HALF>(t, at, xl);
+            else if (qt == QT_Q6_K) ok = section_dot<QT_Q6_K, MT, HALF>(t, at, xl);
+            else if (qt == QT_Q8_0) ok = section_dot<QT_Q8_0, MT, HALF>(t, at, xl);
+            else if (qt == QT_Q5_K) ok = section_dot<QT_Q5_K, MT, HALF>(t, at, xl);
+            else if (qt == QT_Q4_0) ok = section_dot<QT_Q4_0, MT, HALF>(t, at, xl);
+            else ok = section_dot<QT_MXFP4, MT, HALF>(t, at, xl);
             if (!ok && lane == 0) {
                 atomicMax(p.status, DEV_ERR_PIPE_TIMEOUT);
                 *fail_flag = 1;
@@ -870,7 +872,12 @@ cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
     p.peer_rank = a.peer_rank;
     p.peer_world = a.peer_world;
     for (int r = 0; r < kPeerMaxWorld; ++r) p.peer_base[r] = a.peer_base[r];
-    bool fused = false, sums = false;
+    // Up to two row groups a CTA (1184 rows on 148 SMs): the form without second rows.  A kernel of its own: beside the other path in
+    // one kernel it cost large launches registers (dependent layers 376 -> 386 us).  Calls of one row, us: full quads / halves (the
+    // dp4a kernel, which worked by rows of one tile): Q4_K 512 x 14336 7.0 / 6.2 (6.6), Q5_K 512 x 28672 13.4 / 10.8 (10.6), Q6_K
+    // 512 x 14336 8.5 / 7.3 (7.5), 1024 x 4096 4.7 / 4.2 (5.7); of two rows, Q6_K 512 x 14336 12.1 / 10.6 (11.7).  Only for plain
+    // launches of the route's own sizes: fused and rank-sum ones are whole layers.
+    bool fused = false, sums = false, half = true;
     for (int i = 0; i < a.njobs; ++i) {
         const StreamJob &J = a.jobs_host[i];
         switch (J.qt) {
@@ -880,6 +887,7 @@ cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
         if (J.flags & STREAM_JOB_WAITS) p.has_dep = 1;
         fused = fused || (J.flags & (STREAM_JOB_SWIGLU | STREAM_JOB_ACCUM)) != 0 || J.gamma != nullptr;
         sums = sums || (J.flags & STREAM_JOB_SUM_RANKS) != 0;
+        half = half && J.share + (J.share_rest > 0) <= QG / 2;
     }
     const int grid = a.grid;
     if (p.has_dep && grid > a.sm_count) return cudaErrorInvalidValue;   // the counter wait needs every CTA resident
@@ -894,7 +902,9 @@ cudaError_t stream_launch_one(const StreamLaunch &a, cudaStream_t st) {
     }
     const bool peer = sums && p.peer_world > 1;
     if (peer) return fused ? launch_m<3>(a, p, grid, st) : launch_m<2>(a, p, grid, st);
-    return fused ? launch_m<1>(a, p, grid, st) : launch_m<0>(a, p, grid, st);
+    if (fused) return launch_m<1>(a, p, grid, st);
+    if (half && a.M <= 2) return a.M == 1 ? launch_t<1, 4>(a, p, grid, st) : launch_t<2, 4>(a, p, grid, st);
+    return launch_m<0>(a, p, grid, st);
 }
 
 }  // namespace

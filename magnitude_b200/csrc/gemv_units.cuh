@@ -289,6 +289,7 @@ template <int QT> struct XScales {
 // The integer sums of one record of sixteen weight rows (r0, r1: the lane's two) against one activation row.
 template <int QT> struct RecSums {
     int d[kSets<QT>][4];
+    template <bool HALF>          // there is no r1
     __device__ __forceinline__ void run(const WRec<QT> &r0, const WRec<QT> &r1, const XLane &xl, int rec, uint32_t row_off, int c) {
         // (the zero area is shared by all rows: only real addresses move)
         const uint32_t b0 = xl.base[0] + (xl.step[0] ? rec * xl.step[0] + row_off : 0u);
@@ -298,9 +299,9 @@ template <int QT> struct RecSums {
             const uint4 b = lds128(((l & 1) ? b1 : b0) + bload_off<QT>(l));
             const int s = kSets<QT> == 4 ? l : l >> 1;
             const bool first = kSets<QT> == 4 || (l & 1) == 0;
-            uint32_t w0[4], w1[4];
+            uint32_t w0[4], w1[4] = {0, 0, 0, 0};
             r0.words(l, c, w0);
-            r1.words(l, c, w1);
+            if (!HALF) r1.words(l, c, w1);
             imma<QT == QT_Q8_0>(d[s], w0[0], w1[0], w0[1], w1[1], b.x, b.y, first);
             imma<QT == QT_Q8_0>(d[s], w0[2], w1[2], w0[3], w1[3], b.z, b.w, false);
         }

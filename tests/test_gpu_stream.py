@@ -24,8 +24,9 @@ def _acts(m, k, seed):
 
 
 @pytest.mark.parametrize("qt", TYPES)
-@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (1, 2367, 256 * 9), (2, 17, 256 * 11), (1, 700, 256 * 20), (2, 4700, 256 * 7), (1, 13, 256 * 33)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (1, 2367, 256 * 9), (2, 17, 256 * 11), (1, 700, 256 * 20), (2, 4700, 256 * 7), (1, 13, 256 * 33), (2, 1184, 2304), (1, 1185, 2304)])
 def test_rows_and_chunks_of_every_length(backend, orc, qt, m, n, k):
+    """(Up to 1184 rows, two row groups a block, run on the form without second rows.)"""
     p = _weights(orc, qt, n, k, n + k)
     x = _acts(m, k, 3)
     y = backend.project(backend.upload(qt, p, n, k), x)
