@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
         for (int jb = 0; jb < p.njobs; ++jb)
             if (jobs_s[jb].gamma && !jobs_s[jb].xq && tid * 32 < jobs_s[jb].K) asm volatile("prefetch.global.L2 [%0];" ::"l"(jobs_s[jb].gamma + tid * 32));
     pdl_wait();   // the previous kernel's writes (activations, images) are visible from here
-    if (p.x_bufs == 2 && tid == 0) fetch_image(next_job(0), 0);
+    if (tid == 0) fetch_image(next_job(0), 0);
 #pragma unroll 1
     for (int jb = next_job(0); jb < p.njobs; jb = next_job(jb + 1), ++own) {
         const StreamJob &J = jobs_s[jb];
@@ -517,14 +517,13 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
         const uint32_t img_bytes = (uint32_t)nsb * ximg_rec_bytes(qt);
 
         // ---- activation image ----------------------------------------------------------------
-        // All warps have left the job before this one (its last barrier), so with one area it is free now and with
-        // two the other one is: the next job's image can travel while this job runs, sent for by the team whose turn is last.
+        // All warps have left the job before this one (its last barrier), so with two areas the other one is free: the next
+        // job's image can travel while this job runs, sent for by the team whose turn is last.  With one area it is sent for
+        // before this job's last final pass.
         const int area = p.x_bufs == 2 ? own & 1 : 0;
         uint8_t *ximg = ximg0 + area * p.x_bytes;
         if (p.x_bufs == 2) {
             if (tid == kTeamWarps * 32 * (first_slot == 0 ? turn - 1 : first_slot - 1)) fetch_image(next_job(jb + 1), area ^ 1);
-        } else if (tid == 0) {
-            fetch_image(jb, 0);
         }
         if (J.xq) {
             // every thread waits for the image itself, no barrier
@@ -630,6 +629,9 @@ __global__ void __launch_bounds__(kThreads, 1) stream_kernel(const __grid_consta
                 return;
             }
             ++section_no;
+            // with one area: nobody reads this job's image any more, so the next one's travels during the final pass (plans of
+            // Q8_0 6144 x 4096, whose 35 KB slots leave room for one: 6.1 us a product when it was sent for at the job's start, 5.3 now)
+            if (p.x_bufs == 1 && q1 == nquads && tid == kConsumers - 32) fetch_image(next_job(jb + 1), 0);
 
             // ---- final pass: every row's partial sums in order, epilogue, store ------------------------
             if (xsum && q0 == 0) {

@@ -63,7 +63,8 @@ def test_blocks_of_extreme_size(backend, orc, qt, peak, weight, m):
 def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
     """From all of the shared memory down to what is refused, in steps smaller than a slot and then smaller than a copy of the
     partial sums: every number of slots and teams down to one, and one copy of the sums.  Two to three row quads a block, a
-    final pass after each; calls, plans of independent jobs and of jobs that wait."""
+    final pass after each; calls, plans of independent jobs and one with a job that waits, whose
+    activation is converted in the launch between two prepared ones."""
     n, k = 3000, 256 * 65
     p, p2 = _weights(orc, qt, n, k, 1), _weights(orc, qt, 300, 2304, 2)
     x, x2 = _acts(m, k, 5), _acts(m, 2304, 6)
@@ -76,7 +77,7 @@ def test_results_do_not_depend_on_the_ring(backend, orc, qt, m):
         out = [torch.zeros((m, n), device="cuda") for _ in range(3)] + [torch.zeros((m, 300), device="cuda") for _ in range(2)]
         try:
             out.append(be.project(w, x))
-            for o, waits in ((out[0:2] + out[3:4], [False, True, True]), ([out[2], torch.zeros_like(out[2]), out[4]], None)):
+            for o, waits in ((out[0:2] + out[3:4], [False, True, False]), ([out[2], torch.zeros_like(out[2]), out[4]], None)):
                 plan = be.plan([([w], x, o[:1]), ([w2], x2, o[2:]), ([w], x, o[1:2])], waits=waits)
                 for _ in range(2):
                     plan.run()
