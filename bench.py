@@ -45,7 +45,7 @@ FALLBACK_TFLOPS = 1400.0
 # 4-layer launch and is proportional to the layers a launch streams, so it is kept as a ratio to
 # the algorithmic bytes; the two launches of a prefill product (fp16 copies, then the GEMM on them: 123.7 + 177.7 MB) are
 # one whole product whatever the number of copies.
-NCU_DECODE_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.014
+NCU_DECODE_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.015
 NCU_PREFILL_TRAFFIC_BYTES_PER_PRODUCT = 301.4e6
 
 
@@ -470,7 +470,7 @@ def run_b200(args):
         be.sync(stream)
         ms_dep = e0.elapsed_time(e1) / reps
         dependent = {"ms_per_step": ms_dep, "value": LAYERS * (2 * algorithmic_bytes(INTER, HIDDEN) + algorithmic_bytes(HIDDEN, INTER)) / (ms_dep * 1e-3) / 1e9,
-                     "unit": UNIT, "note": "same step, every down projection flagged as reading what gate/up wrote (one consumer team, grid counter between jobs)"}
+                     "unit": UNIT, "note": "same step, every down projection flagged as reading what gate/up wrote (the CTAs meet at a grid counter between jobs)"}
         dep_plan.close()
         # The MLP block as a model runs it: h = silu(gate x) * (up x) in the gate/up job's epilogue, down
         # reads h and adds into the residual stream x, the next layer's gate/up reads that stream.

@@ -314,7 +314,8 @@ typedef struct b200q_plan b200q_plan;
 
 enum {
     /* the job's activation is written by earlier jobs of the same plan (e.g. the down projection
-     * reading what gate/up produced): all CTAs finish those jobs before this one converts x */
+     * reading what gate/up produced): all CTAs finish those jobs before this one converts x.  A launch with
+     * such a job needs a block on every SM at the same time: order two such plans of one device with events */
     B200Q_JOB_WAITS_FOR_EARLIER = 1,
     /* row-parallel projection under tensor parallelism: the job's outputs are partial sums, and the
      * launch itself adds them up over the ranks attached with b200q_peer_attach (peer-memory stores

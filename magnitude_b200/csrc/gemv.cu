@@ -14,7 +14,7 @@
 //   * up to four teams of four consumer warps take the slots in turn; in a slot each warp owns two
 //     records of all sixteen rows and multiplies each with eight integer mma.m16n8k32
 //     (gemv_units.cuh).  What bounds the kernel is instructions: 240 per 2304 bytes of Q4_K with all
-//     bookkeeping, 60 % of the schedulers' slots at 5.9 TB/s; dp4a, at half rate, took 250 slots for the
+//     bookkeeping, 58 % of the schedulers' slots at 5.2 TB/s; dp4a, at half rate, took 250 slots for the
 //     products alone.  A record per warp and two teams (331 instructions) reached 4.6 TB/s, the dp4a
 //     kernel before 4.2 (ten independent 25600 x 5120 Q4_K products in a plan; 6.2 of Q8_0, 4.6 of Q6_K).
 //   * per job each CTA owns a contiguous range of 4-row groups; a row's partial sums go to shared
@@ -22,7 +22,8 @@
 //     the partition or the ring and are bit-reproducible.
 //   * the activation is converted once per CTA and job into a 16-bit fixed-point image in shared
 //     memory; plans of several independent jobs have a small launch convert all their activations and
-//     the CTA fetches each image with one bulk copy, one job ahead where two images fit.
+//     the CTA fetches each image with one bulk copy, one job ahead where two images fit, else during
+//     the final pass of the job before.
 //   * a job may declare that it reads what earlier jobs of the same launch wrote; the CTAs then
 //     meet at a counter in global memory before converting that job's activation.
 //   * every wait (mbarrier, counter) is bounded; on expiry the waiter raises the status word and

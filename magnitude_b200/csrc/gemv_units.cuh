@@ -44,7 +44,7 @@ __host__ __device__ constexpr int ximg_rec_bytes(int qt) { return qt == QT_Q6_K 
 // be multiplied per weight, and lane group c (= lane & 3) holds (hi, lo) of sub-block c of every set.  What a
 // weight costs is its unpacking (two logic operations per eight weights of Q4_K); dp4a, at half rate and four
 // weights per instruction and plane, used to cost four more.  (Sums from such accumulators through a biased fp32
-// number instead of an int-to-float conversion: 53 against 51 cycles of an SM per record, dropped.)
+// number instead of an int-to-float conversion were a little slower.)
 //
 // Shared memory order of K is free: A takes whatever 16 bytes lane group c loads, B the activation bytes of the
 // same positions.  B load l (of four, two MMAs each) of lane (n = lane >> 2, kc = lane & 3) reads 16 bytes of
