@@ -144,13 +144,13 @@ def test_waiting_for_the_launch_before_has_no_limit(orc):
             b.sync()
         base, words = _words(cu, bufs[0])
         assert cu.cuMemsetD8_v2(ctypes.c_uint64(base), ctypes.c_ubyte(0), ctypes.c_size_t(8 * len(words))) == 0
-        a.set_option(B.OPT_WAIT_LIMIT_MS, 400)
+        a.set_option(B.OPT_WAIT_LIMIT_MS, 1000)
         stream = torch.cuda.Stream()
         torch.cuda.synchronize()
         plans[0].run(stream=stream)
         c.project(big, xb, out=got, stream=stream)
         for exchange in (1, 2):
-            time.sleep(0.25)
+            time.sleep(0.6)
             shares = np.flatnonzero(words >> np.uint64(32) == exchange)
             assert len(shares) == m * n
             for i in shares:
